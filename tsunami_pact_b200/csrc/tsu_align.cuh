@@ -61,17 +61,24 @@ __device__ __forceinline__ void group_sync(int gid) {
   }
 }
 
+}  // namespace tsu
+
+#include "tsu_packed.cuh"
+
+namespace tsu {
+
 template <int GW>
 constexpr int cta_threads() {
   return GW <= 4 ? 128 : 32 * GW;
 }
 template <int kMode, int GW>
 constexpr int cta_min_blocks() {
-  return kMode == kModeShared ? (GW == 1 ? 7 : (GW <= 4 ? 6 : (GW == 8 ? 3 : 1))) : (GW <= 4 ? 4 : (GW == 8 ? 2 : 1));
+  return kMode == kModeShared ? (GW == 1 ? 6 : (GW <= 4 ? 6 : (GW == 8 ? 3 : 1))) : (GW <= 4 ? 4 : (GW == 8 ? 2 : 1));
 }
 
-template <bool kCigar, int kMode, int GW, int kModel = kModelAffine>
-__global__ void __launch_bounds__(cta_threads<GW>(), (cta_min_blocks<kMode, GW>())) align_kernel(AlignArgs a) {
+// The body of align_kernel for the global ring and for low-memory CIGARs.
+template <bool kCigar, int kMode, int GW, int kModel>
+__device__ __forceinline__ void align_ring(const AlignArgs& a, unsigned char* smem_raw) {
   static_assert(GW == 1 || GW == 2 || GW == 4 || GW == 8 || GW == 16 || GW == 32, "warps per pair");
   constexpr bool kDual = (kModel & 7) == kModelDual;
   constexpr bool kLin = (kModel & 7) == kModelLinear;
@@ -97,11 +104,6 @@ __global__ void __launch_bounds__(cta_threads<GW>(), (cta_min_blocks<kMode, GW>(
   constexpr bool kStage = kMode == kModeGlobal && GW < 32;
   using S = typename std::conditional<kMode == kModeShared, SharedSeq,
                                       typename std::conditional<kStage, AnySeq, GlobalSeq>::type>::type;
-#ifdef TSU_WARP_EMU
-  unsigned char* smem_raw = emu::dyn_smem();  // CPU warp emulation of the tests
-#else
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-#endif
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int GT = 32 * GW;  // threads per group
   const int tid = threadIdx.x;
@@ -816,6 +818,19 @@ __global__ void __launch_bounds__(cta_threads<GW>(), (cta_min_blocks<kMode, GW>(
     }
     group_sync<GW>(gid);  // the group's shared memory is free for the next pair
   }
+}
+
+template <bool kCigar, int kMode, int GW, int kModel = kModelAffine>
+__global__ void __launch_bounds__(cta_threads<GW>(), (cta_min_blocks<kMode, GW>())) align_kernel(AlignArgs a) {
+#ifdef TSU_WARP_EMU
+  unsigned char* smem_raw = emu::dyn_smem();  // CPU warp emulation of the tests
+#else
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+#endif
+  if constexpr (kMode == kModeShared && !(kModel & kLowMemFlag))
+    align_packed<kCigar, GW, kModel>(a, smem_raw);
+  else
+    align_ring<kCigar, kMode, GW, kModel>(a, smem_raw);
 }
 
 }  // namespace tsu

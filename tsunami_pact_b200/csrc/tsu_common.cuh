@@ -176,16 +176,33 @@ __host__ __device__ inline int64_t ckpt_bytes_for(const Pen& p, int ring_w, int 
 // Warp partials per warp and step parity: 7 (one piece) or 11 values.
 __host__ __device__ inline int partial_words(const Pen& p) { return p.dual() ? 16 : 8; }
 
-// Shared memory per group of gw warps, in bytes: slot limits (lo, hi, alo
-// per slot), warp partials [2][gw][partial_words] (gw > 1), 4 broadcast
-// words, then in shared mode an int16 ring of slots * ring_w and seq_cap
-// sequence words; in global mode with seq_cap > 0, at the next 16-byte
-// boundary, 16 reserved bytes and seq_cap sequence words.
+// The shared-ring kernel (tsu_packed.cuh): longest side its 16-bit offsets
+// hold (2 h + 32768 plus one 16-base window past the end stays below 65536),
+// deepest ring its 64-bit record of the last scores covers, 32-bit words per
+// ring row (ring_w halfwords and 4 on each side) and bytes before the ring
+// (4 broadcast words, 2 gw partials, 16 bytes of row offsets per M slot and
+// per I / D slot pair).
+constexpr int kPackedMaxLen = 16352;
+constexpr int kPackedMaxDepth = 64;
+__host__ __device__ inline int packed_row_words(int ring_w) { return (ring_w + 8) / 2; }
+__host__ __device__ inline int packed_head_bytes(const Pen& p, int gw) {
+  return ((16 + 8 * gw + 15) & ~15) + 16 * (p.rm + p.re + p.re2);
+}
+
+// Shared memory per group of gw warps, in bytes.  Global mode and the
+// low-memory kernels: slot limits (lo, hi, alo per slot), warp partials
+// [2][gw][partial_words] (gw > 1), 4 broadcast words, then in shared mode an
+// int16 ring of slots * ring_w and seq_cap sequence words; in global mode with
+// seq_cap > 0, at the next 16-byte boundary, 16 reserved bytes and seq_cap
+// sequence words.  Shared mode takes the larger of that and of the packed
+// kernel's head, slots + 1 rows and sequence words.
 __host__ __device__ inline int group_smem_bytes(const Pen& p, int ring_w, int mode, int seq_cap, int gw) {
   const int ns = p.slots();
   int b = 3 * ns * 4 + (gw > 1 ? 2 * partial_words(p) * gw * 4 : 0) + 16;
   if (mode == kModeShared) {
     b += ((ns * ring_w * 2 + 15) & ~15) + seq_cap * 4;
+    const int packed = packed_head_bytes(p, gw) + (ns + 1) * packed_row_words(ring_w) * 4 + seq_cap * 4;
+    if (packed > b) b = packed;
   } else if (seq_cap > 0) {
     b = ((b + 15) & ~15) + 16 + seq_cap * 4;
   }

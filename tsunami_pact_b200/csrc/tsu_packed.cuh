@@ -1,0 +1,731 @@
+// tsu_packed.cuh -- the shared-ring align kernel: two diagonals per thread.
+//
+// The wavefront ring of the last max(x, o+e)+1 scores is 16-bit in shared
+// memory, and one thread computes two neighbouring diagonals (one 32-bit
+// word) at a time with per-halfword add-max / add-min instructions.  What
+// bounds it is the integer ALU pipe (half an instruction per cycle and
+// scheduler; ncu: 75 % busy in the one-diagonal form), so the layout is
+// chosen to spend few ALU instructions per cell:
+//   * an offset h is held as 2 h + kZero (kZero = 32768): an absent cell is
+//     any halfword with bit 15 clear, and bit 0 is free.  A candidate enters a
+//     maximum with bit 0 set when it wins ties, so one add-max both takes the
+//     maximum and records which side won; I, D and M of two cells take nine
+//     such instructions with all their source bits;
+//   * absent cells stay below kZero: M rows store absent as 0, I climbs by 2
+//     per diagonal it moves, at most 2 ring_w < kZero;
+//   * every row has the same diagonal-to-position map (position = k - kbase)
+//     and is all absent before its first write, so no read needs a range
+//     test; a source row that does not exist at this score is a permanent
+//     row of absent cells;
+//   * the range of diagonals at score s follows from the penalties alone
+//     (one more on each side per gap extension), clipped to [-m, n], so a step
+//     has no reductions: its end test is one read of M on diagonal n - m;
+//   * an M offset beyond the matrix edge is clamped to the edge instead of
+//     dropped.  A clamped cell stands for a position that is reachable at no
+//     higher cost, from which the alignment cannot end earlier than it does
+//     through the cell that reached the edge, so neither the score nor the
+//     cells on the backtrace's path change;
+//   * with CIGARs a cell's history is its source bits alone (4 bits; 8 with
+//     two gap pieces), not its offset: the backtrace follows the bits from the
+//     end to score 0, and the matches between the edits are then found
+//     again from the front, 512 bases per warp comparison.
+// Measured on one B200 against the one-diagonal form (the same ring, limits
+// per row kept by warp reductions, 4-byte history words; align pass, scores +
+// CIGARs): 200,000 x 1 kbp at 5 % 31.9 -> 16.6 ms (scores only 24.0 -> 11.9),
+// 1,000 x 10 kbp at 15 % on 16 warps 112 -> 50.5 ms, 20,000 x 1 kbp dual
+// gap-affine on 8 warps 42.5 -> 15.4 ms.  A cell pair takes 75 warp
+// instructions scored (90 with history) and a step 145, against 175 per 32
+// cells before; issue slots are 86 % and the ALU pipe 68 % busy.
+// Limits: sides of at most kPackedMaxLen bases, ACGT only, at most 64 score
+// steps of ring depth; other pairs go to the global ring (tsu_align.cuh).
+#pragma once
+
+#include <type_traits>
+
+#include "tsu_common.cuh"
+#include "tsu_extend.cuh"
+
+namespace tsu {
+
+constexpr uint32_t kZero = 32768u;  // halfword of offset 0 (a multiple of 32: the low 5 bits of a halfword are
+                                    // twice the base's place in its 16-base word)
+
+// ---- halfword pairs ------------------------------------------------------
+#ifdef TSU_WARP_EMU
+template <class F>
+inline uint32_t h2_each(uint32_t a, uint32_t b, uint32_t c, F f) {
+  const uint16_t lo = f((uint16_t)a, (uint16_t)b, (uint16_t)c);
+  const uint16_t hi = f((uint16_t)(a >> 16), (uint16_t)(b >> 16), (uint16_t)(c >> 16));
+  return (uint32_t)lo | ((uint32_t)hi << 16);
+}
+inline uint32_t h2_addmax(uint32_t a, uint32_t b, uint32_t c) {
+  return h2_each(a, b, c, [](uint16_t x, uint16_t y, uint16_t z) { return std::max<uint16_t>((uint16_t)(x + y), z); });
+}
+inline uint32_t h2_addmin(uint32_t a, uint32_t b, uint32_t c) {
+  return h2_each(a, b, c, [](uint16_t x, uint16_t y, uint16_t z) { return std::min<uint16_t>((uint16_t)(x + y), z); });
+}
+inline uint32_t h2_max(uint32_t a, uint32_t b) { return h2_addmax(a, 0, b); }
+inline uint32_t h2_min(uint32_t a, uint32_t b) { return h2_addmin(a, 0, b); }
+inline uint32_t h2_next(uint32_t a, uint32_t b) { return (a >> 16) | (b << 16); }
+inline uint32_t h2_signmask(uint32_t a) { return ((a & 0x8000u) ? 0xffffu : 0u) | ((a & 0x80000000u) ? 0xffff0000u : 0u); }
+inline int h2_tz(uint32_t d) { return d ? __builtin_ctz(d) : 32; }
+inline uint32_t h2_sum(uint32_t a, uint32_t acc) { return acc + (a & 0xffffu) + (a >> 16); }
+#else
+// max(a + b, c), min(a + b, c) per halfword, the sum modulo 2^16
+__device__ __forceinline__ uint32_t h2_addmax(uint32_t a, uint32_t b, uint32_t c) { return __viaddmax_u16x2(a, b, c); }
+__device__ __forceinline__ uint32_t h2_addmin(uint32_t a, uint32_t b, uint32_t c) { return __viaddmin_u16x2(a, b, c); }
+__device__ __forceinline__ uint32_t h2_max(uint32_t a, uint32_t b) { return __vmaxu2(a, b); }
+__device__ __forceinline__ uint32_t h2_min(uint32_t a, uint32_t b) { return __vminu2(a, b); }
+// (high half of a, low half of b)
+__device__ __forceinline__ uint32_t h2_next(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x5432); }
+// 0xffff in each half whose bit 15 is set (prmt replicates the sign of bytes 1 and 3)
+__device__ __forceinline__ uint32_t h2_signmask(uint32_t a) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %1, 0xbb99;" : "=r"(r) : "r"(a));
+  return r;
+}
+// trailing zero bits, 32 for 0
+__device__ __forceinline__ int h2_tz(uint32_t d) { return __clz((int)__brev(d)); }
+// acc + both halves (below 2^15 each)
+__device__ __forceinline__ uint32_t h2_sum(uint32_t a, uint32_t acc) {
+  return (uint32_t)__dp2a_lo((int)a, 0x0101, (int)acc);
+}
+#endif
+__device__ __forceinline__ uint32_t h2_dup(uint32_t v) { return (v & 0xffffu) * 0x10001u; }
+
+// ---- shared memory by byte address --------------------------------------------
+// One address register per group, taken once: accesses are a register and a
+// constant.  (Through pointers the base address of the block's shared memory
+// was formed again at every step: 13 of its 200 instructions.)
+#ifdef TSU_WARP_EMU
+using smem_t = unsigned char*;
+inline smem_t smem_addr(unsigned char* p) { return p; }
+template <int kOff = 0>
+inline uint32_t lds32(smem_t a) {
+  uint32_t v;
+  std::memcpy(&v, a + kOff, 4);
+  return v;
+}
+inline uint32_t lds16(smem_t a) {
+  uint16_t v;
+  std::memcpy(&v, a, 2);
+  return v;
+}
+inline void lds128(smem_t a, int& x, int& y, int& z, int& w) {
+  int v[4];
+  std::memcpy(v, a, 16);
+  x = v[0], y = v[1], z = v[2], w = v[3];
+}
+inline void sts32(smem_t a, uint32_t v) { std::memcpy(a, &v, 4); }
+inline void sts16(smem_t a, uint32_t v) {
+  const uint16_t h = (uint16_t)v;
+  std::memcpy(a, &h, 2);
+}
+inline void sts128(smem_t a, int x, int y, int z, int w) {
+  const int v[4] = {x, y, z, w};
+  std::memcpy(a, v, 16);
+}
+#else
+using smem_t = uint32_t;
+__device__ __forceinline__ smem_t smem_addr(unsigned char* p) {
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("" : "+r"(a));  // opaque: kept in a register
+  return a;
+}
+template <int kOff = 0>
+__device__ __forceinline__ uint32_t lds32(smem_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(kOff));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds16(smem_t a) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void lds128(smem_t a, int& x, int& y, int& z, int& w) {
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(a));
+}
+__device__ __forceinline__ void sts32(smem_t a, uint32_t v) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void sts16(smem_t a, uint32_t v) {
+  asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((uint16_t)v) : "memory");
+}
+__device__ __forceinline__ void sts128(smem_t a, int x, int y, int z, int w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+#endif
+
+// 16 bases from position pos of the packed words at address w.
+__device__ __forceinline__ uint32_t lds_win16(smem_t w, int pos) {
+  const smem_t a = w + ((pos >> 4) << 2);
+  return __funnelshift_r(lds32(a), lds32<4>(a), (uint32_t)pos << 1);
+}
+// lcp16 (tsu_extend.cuh) over words in shared memory.
+__device__ __forceinline__ int lds_lcp(smem_t pw, int v, smem_t tw, int h, int rem) {
+  int l = 0;
+  while (l < rem) {
+    const uint32_t d = lds_win16(pw, v + l) ^ lds_win16(tw, h + l);
+    if (d) {
+      l += h2_tz(d) >> 1;
+      break;
+    }
+    l += 16;
+  }
+  return l < rem ? l : rem;
+}
+
+// Bytes of history per pair of diagonals.
+template <bool kDual>
+constexpr int hist_pair_bytes() {
+  return kDual ? 2 : 1;
+}
+
+// Longest common prefix of pattern[v..] and text[h..], at most rem, by a
+// whole warp: 512 bases per comparison.
+__device__ __forceinline__ int warp_lcp(smem_t pw, int v, smem_t tw, int h, int rem, int lane) {
+  int l = 0;
+  while (l < rem) {
+    const int at = l + 16 * lane;
+    int lx = 0;  // lanes past the end stop the run at their start, which min() below cuts to rem
+    if (at < rem) lx = h2_tz(lds_win16(pw, v + at) ^ lds_win16(tw, h + at)) >> 1;
+    const unsigned stop = __ballot_sync(0xffffffffu, lx < 16);
+    if (stop) {
+      const int src = __ffs((int)stop) - 1;
+      return min(l + 16 * src + __shfl_sync(0xffffffffu, lx, src), rem);
+    }
+    l += 512;
+  }
+  return rem;
+}
+
+// The CIGAR of a finished pair, by one warp.  First the walk: from the end
+// (s_end, k_fin) along the source bits to score 0, 32 scores of history in
+// registers at a time (lane l holds score top - l: 16 diagonals around the
+// path; 8 with two gap pieces), each edit or gap written as one entry
+// (length << 4 | op) downwards from out + cap.  Then the replay from the
+// front: matches found again between the entries, runs written upwards from
+// out.  Of e entries at most 2 e + 1 runs are written, 2 j + 1 of them before
+// entry j is read, so with cap >= 2 e + 2 they share the space.  Returns the
+// number of runs, or -1 on an inconsistency.
+template <int kModel>
+__device__ __forceinline__ int packed_cigar(const uint32_t* hist, int64_t hist_chunks,
+                                            const int2* table, int s_end, int k_fin, int m, int n,
+                                            const Pen& pen, int kbase, int lo0, int hi0, smem_t pw,
+                                            smem_t tw, uint32_t* out, int cap, int lane) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr bool kDual = kModel == kModelDual, kLin = kModel == kModelLinear;
+  constexpr int kCS = kDual ? 1 : 2;  // log2 of pairs of diagonals per 32-bit chunk
+  int s = s_end, k = k_fin;
+  int state = 0;  // 0: M; 1, 2: inside an I, D of the first gap piece; 3, 4: of the second
+  int top = -1, c0 = 0;
+  uint32_t d0 = 0, d1 = 0;
+  int ne = 0;           // entries
+  uint32_t gap = 0;     // the open gap's entry
+  while (s > 0) {
+    const int pos = k - kbase;
+    const int ch = pos >> (kCS + 1);
+    if (s > top || s <= top - 32 || ch < c0 || ch > c0 + 1) {
+      top = s;
+      c0 = (pos - (1 << kCS)) >> (kCS + 1);
+      d0 = d1 = 0;
+      if (s - lane > 0) {
+        const int2 te = table[s - lane];
+        const int64_t i = (int64_t)te.y + c0 - te.x;
+        if (i >= 0 && i < hist_chunks) d0 = hist[i];
+        if (i + 1 >= 0 && i + 1 < hist_chunks) d1 = hist[i + 1];
+      }
+    }
+    const uint32_t word = __shfl_sync(FULL, ch == c0 ? d0 : d1, top - s);
+    uint32_t ins, ext;
+    if constexpr (kDual) {
+      const uint32_t b = word >> ((pos & 3) * 8);
+      int comp = state;
+      if (comp == 0) comp = (b & 1u) ? 0 : (b & 2u) ? 4 : (b & 4u) ? 2 : (b & 8u) ? 3 : 1;
+      if (comp == 0) {
+        if (lane == 0 && ne < cap) out[cap - 1 - ne] = (1u << 4) | kOpX;
+        ++ne;
+        s -= pen.x;
+        continue;
+      }
+      ins = comp & 1;
+      ext = (b >> (3 + comp)) & 1u;
+      s -= ext ? (comp <= 2 ? pen.ge : pen.ge2) : (comp <= 2 ? pen.go : pen.go2);
+      state = ext ? comp : 0;
+    } else {
+      const uint32_t b = word >> ((pos & 7) * 4);
+      if (state == 0) {
+        if (b & 1u) {
+          if (lane == 0 && ne < cap) out[cap - 1 - ne] = (1u << 4) | kOpX;
+          ++ne;
+          s -= pen.x;
+          continue;
+        }
+        state = (b & 2u) ? 2 : 1;
+      }
+      ins = state & 1;
+      ext = kLin ? 0u : (b >> (1 + state)) & 1u;
+      s -= ext ? pen.ge : pen.go;
+      if (!ext) state = 0;
+    }
+    gap += 1u << 4;
+    k += ins ? -1 : 1;
+    if (!ext) {
+      if (lane == 0 && ne < cap) out[cap - 1 - ne] = gap | (ins ? kOpI : kOpD);
+      ++ne;
+      gap = 0;
+    }
+  }
+  if (s < 0 || gap || state || k < lo0 || k > hi0 || 2 * ne + 2 > cap) return -1;
+  __syncwarp();
+  // ---- replay
+  int v = k < 0 ? -k : 0, h = k > 0 ? k : 0;  // the free leading gap
+  int nr = 0;
+  uint32_t cur = 0;  // the open run
+  auto put = [&](uint32_t op, int len) {
+    if (len <= 0) return;
+    if (cur && (cur & 15u) == op) {
+      cur += (uint32_t)len << 4;
+      return;
+    }
+    if (cur) {
+      if (lane == 0) out[nr] = cur;
+      ++nr;
+    }
+    cur = ((uint32_t)len << 4) | op;
+  };
+  put(kOpD, v);
+  put(kOpI, h);
+  uint32_t ent = 0;
+  for (int j = 0;; ++j) {
+    const int rem = min(m - v, n - h);
+    if (rem < 0) return -1;
+    const int l = warp_lcp(pw, v, tw, h, rem, lane);
+    put(kOpM, l);
+    v += l;
+    h += l;
+    if (j == ne) break;
+    if ((j & 31) == 0) {
+      __syncwarp();
+      ent = j + lane < ne ? out[cap - ne + j + lane] : 0u;
+      __syncwarp();
+    }
+    const uint32_t e = __shfl_sync(FULL, ent, j & 31);
+    const int len = (int)(e >> 4);
+    const uint32_t op = e & 15u;
+    put(op, len);
+    if (op != kOpI) v += len;
+    if (op != kOpD) h += len;
+  }
+  if (h - v != k_fin || h != min(n, m + k_fin)) return -1;
+  put(kOpD, m - v);
+  put(kOpI, n - h);
+  if (cur) {
+    if (lane == 0) out[nr] = cur;
+    ++nr;
+  }
+  return nr;
+}
+
+// The body of align_kernel for the shared ring (see the head of this file).
+template <bool kCigar, int GW, int kModel>
+__device__ __forceinline__ void align_packed(const AlignArgs& a, unsigned char* smem_raw) {
+  constexpr bool kDual = kModel == kModelDual;
+  constexpr bool kLin = kModel == kModelLinear;
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int GT = 32 * GW;
+  constexpr int kHB = hist_pair_bytes<kDual>();
+  constexpr int kCS = kDual ? 1 : 2;  // log2 of diagonal pairs per 32-bit history chunk
+  constexpr uint32_t kOne2 = 0x00010001u, kClean = 0xfffefffeu;
+  const int tid = threadIdx.x;
+  const int gid = tid / GT;
+  const int gt = tid - gid * GT;
+  const int lane = tid & 31;
+  const int wig = gt >> 5;
+  const int gpb = blockDim.x / GT;
+  const int64_t ggroup = (int64_t)blockIdx.x * gpb + gid;
+  const int W = a.ring_w;
+  const int RB = packed_row_words(W) * 4;  // bytes per row
+  const int rm = a.pen.rm, re = a.pen.re, re2 = a.pen.re2;
+  const int rows = a.pen.slots() + 1;  // and the row of absent cells
+  // 4 broadcast words, 2 GW partials of the free-end test, the row tables,
+  // the ring, the sequences
+  const smem_t bc = smem_addr(smem_raw) + (size_t)gid * group_smem_bytes(a.pen, W, kModeShared, a.seq_cap, GW);
+  const smem_t part = bc + 16;
+  const smem_t tab_m = bc + packed_head_bytes(Pen(), GW), tab_g = tab_m + 16 * rm, tab_g2 = tab_g + 16 * re;
+  const smem_t ring = bc + packed_head_bytes(a.pen, GW);
+  const smem_t ring0 = ring + 8;  // position 0 of row 0
+  const smem_t pws = ring + rows * RB;
+  {
+    // Row tables: the byte offsets of the rows a score writes and reads, by
+    // its place in the ring: M {out, s-x, s-o-e, s-o2-e2}, I and D {out I, out
+    // D, I and D at s-e}, I2 and D2 likewise.
+    auto back = [](int slot, int by, int depth) -> int { return slot < by ? slot - by + depth : slot - by; };
+    for (int j = gt; j < rm; j += GT)
+      sts128(tab_m + 16 * j, j * RB, back(j, a.pen.x, rm) * RB, back(j, a.pen.go, rm) * RB,
+             kDual ? back(j, a.pen.go2, rm) * RB : 0);
+    for (int j = gt; j < re; j += GT) {
+      const int q = rm + back(j, a.pen.ge, re);
+      sts128(tab_g + 16 * j, (rm + j) * RB, (rm + re + j) * RB, q * RB, (q + re) * RB);
+    }
+    for (int j = gt; j < re2; j += GT) {
+      const int g0 = rm + 2 * re, q = g0 + back(j, a.pen.ge2, re2);
+      sts128(tab_g2 + 16 * j, (g0 + j) * RB, (g0 + re2 + j) * RB, q * RB, (q + re2) * RB);
+    }
+  }
+  uint32_t* const hist = kCigar ? a.hist + ggroup * a.hist_cap : nullptr;
+  const int hist_cap = (int)a.hist_cap;  // below 2^31 (tsu_plan.h)
+  int2* const table = kCigar ? a.table + ggroup * (int64_t)a.table_cap : nullptr;
+
+  for (;;) {
+    unsigned qi;
+    if constexpr (GW == 1) {
+      unsigned q = 0;
+      if (lane == 0) q = atomicAdd(a.queue, 1u);
+      qi = __shfl_sync(FULL, q, 0);
+    } else {
+      if (gt == 0) sts32(bc, atomicAdd(a.queue, 1u));
+      group_sync<GW>(gid);
+      qi = lds32(bc);
+    }
+    if ((int64_t)qi >= a.n_order) break;
+    const int64_t pair = a.order ? a.order[qi] : (int64_t)qi;
+    const int m = a.seq.pat_len[pair];
+    const int n = a.seq.txt_len[pair];
+    const bool bytemode = a.pk.nonacgt[pair] | a.pk.nonacgt[a.seq.n + pair];
+    const int pwn = 2 * (int)packed_words(m);  // uint32 words
+    const int twn = 2 * (int)packed_words(n);
+    const int k_end = n - m;
+    int32_t st = kPairOk;
+    if (bytemode || m > kPackedMaxLen || n > kPackedMaxLen || pwn + twn > a.seq_cap) st = kPairScratch;
+    int s_end = -1, k_fin = k_end;
+    int s = 0;
+    int hbase = 0;  // history chunks in use
+    unsigned long long n_cells = 0;
+    uint32_t n_steps = 0, n_ext2 = 0;  // n_ext2: twice the bases matched by this thread's extend steps
+    // diagonals of score 0 (free beginnings), and the ring's window
+    const int lo0 = -min(a.ef_pb, m), hi0 = min(a.ef_tb, n);
+    int kbase = -m;
+    if (m + n + 2 > W) {
+      // the window's middle on the middle of the beginning, inside [-m, n]
+      kbase = min(max((lo0 + hi0 - W) >> 1, -m), n + 1 - W);
+    }
+    if (lo0 < kbase || hi0 - kbase >= W) st = kPairScratch;
+
+    if (st == kPairOk) {
+      const uint32_t* gpw = reinterpret_cast<const uint32_t*>(a.pk.words + a.pk.woff[pair]);
+      const uint32_t* gtw = reinterpret_cast<const uint32_t*>(a.pk.words + a.pk.woff[a.seq.n + pair]);
+      const smem_t tws = pws + 4 * pwn;
+      for (int i = gt; i < pwn; i += GT) sts32(pws + 4 * i, __ldg(gpw + i));
+      for (int i = gt; i < twn; i += GT) sts32(tws + 4 * i, __ldg(gtw + i));
+      // every row all absent, the words on both sides of it included
+      for (int i = 16 * gt; i < rows * RB; i += 16 * GT) sts128(ring + i, 0, 0, 0, 0);
+      group_sync<GW>(gid);
+      const int k_hi = k_end + a.ef_pe;  // highest diagonal that may end with pattern characters left
+      const bool free_te = a.ef_te > 0;
+      const int n_te = n - a.ef_te;
+      const bool ends_free = a.ef_pe > 0 || free_te;
+      // whether M at text offset om on diagonal k (om <= min(n, m + k)) ends the alignment
+      auto ends_at = [&](int om, int k) -> bool {
+        return (om >= n && k <= k_hi) || (free_te && om - k >= m && om >= n_te);
+      };
+      // ---- score 0
+      int fk = INT_MAX;
+      {
+        for (int k = lo0 + gt; k <= hi0; k += GT) {
+          const int p0 = k > 0 ? k : 0;
+          const int om = p0 + lds_lcp(pws, p0 - k, tws, p0, min(m - (p0 - k), n - p0));
+          sts16(ring0 + 2 * (k - kbase), 2 * (uint32_t)om + kZero);
+          if (ends_free && fk == INT_MAX && ends_at(om, k)) fk = k;
+        }
+        n_cells = (unsigned)(hi0 - lo0 + 1);
+      }
+      // the cell on diagonal n - m (the row of absent cells' first one when
+      // the window does not hold it)
+      const int pend = k_end - kbase;
+      const bool end_in = pend >= 0 && pend < W;
+      const smem_t end_cell = ring0 + (end_in ? 2 * pend : 0);
+      const uint32_t end_val = end_in ? 2 * (uint32_t)n + kZero : 0x10000u;
+      // After a step: has the alignment ended?  (One barrier, which also
+      // separates the step's writes from the next one's reads.)
+      int flip = 0;  // the free-end partials are double-buffered by step computed
+      auto ended = [&](int fkt, int row_m, bool free_ends) {
+        if (free_ends) {
+          fkt = __reduce_min_sync(FULL, fkt);
+          if constexpr (GW > 1) {
+            flip ^= 4 * GW;
+            const smem_t pp = part + flip;
+            if (lane == 0) sts32(pp + 4 * wig, (uint32_t)fkt);
+            group_sync<GW>(gid);
+            fkt = __reduce_min_sync(FULL, lane < GW ? (int)lds32(pp + 4 * lane) : INT_MAX);
+          } else {
+            __syncwarp();
+          }
+          if (fkt != INT_MAX) {
+            s_end = s;
+            k_fin = fkt;
+          }
+        } else {
+          group_sync<GW>(gid);
+          if (lds16(end_cell + row_m) >= end_val) s_end = s;
+        }
+      };
+      ended(fk, 0, ends_free);
+
+      const int64_t bound = score_bound(m, n, a.pen);
+      // scores this launch can compute: past s_max the end would have been
+      // found (an inconsistency), past the step table the pair is handed back
+      const int s_max = (int)(bound < INT_MAX - 1 ? bound : INT_MAX - 1);
+      const int s_lim = kCigar ? min(s_max, a.table_cap - 1) : s_max;
+      // diagonals each side can gain before the range leaves the ring's window
+      const int grow_lim = min(kbase > -m ? lo0 - kbase : INT_MAX, kbase + W <= n ? kbase + W - 1 - hi0 : INT_MAX);
+      constexpr uint32_t kZero2 = kZero * 0x10001u;
+      const uint32_t m2 = h2_dup(2 * (uint32_t)m);
+      // 2 k + kZero of the diagonals at word w: kw0 + 4 w in each half; the
+      // same of diagonal n - m; all below 2^16, so plain adds carry nothing
+      const uint32_t kw0 = (uint32_t)((int)kZero + 2 * kbase) + ((uint32_t)((int)kZero + 2 * kbase + 2) << 16);
+      const uint32_t kend2 = h2_dup((uint32_t)((int)kZero + 2 * k_end));
+      smem_t tm = tab_m, tg = tab_g, tg2 = tab_g2;  // the score's rows
+      int grow = 0, grow_at = a.pen.go;                       // diagonals gained on each side, next score that gains one
+      int grow2 = 0, grow2_at = kDual ? a.pen.go2 : INT_MAX;  // the second gap piece
+      // the score's diagonals, words, history chunks
+      int lo = max(lo0, -m), hi = min(hi0, n);
+      int wlo = (lo - kbase) >> 1, whi = (hi - kbase) >> 1;
+      int hc0 = wlo >> kCS, chunks = (whi >> kCS) - hc0 + 1;
+      // which of the last 64 scores have an M (an I or D) wavefront; once
+      // every score in reach has all of them it stays so (full)
+      unsigned long long has_m = 1, has_g = 0, has_g2 = 0;
+      bool full = false;
+      const int none_row = (rows - 1) * RB;
+      auto steps = [&](auto ends_tag) {
+        constexpr bool kEnds = decltype(ends_tag)::value;
+        while (s_end < 0) {
+          ++s;
+          tm = tm + 16 == tab_g ? tab_m : tm + 16;
+          int w_m, r_mx, r_mo, r_mo2, w_i = 0, w_d = 0, r_ie = 0, r_de = 0, w_i2 = 0, w_d2 = 0, r_ie2 = 0, r_de2 = 0;
+          lds128(tm, w_m, r_mx, r_mo, r_mo2);
+          if constexpr (!kLin) {
+            tg = tg + 16 == tab_g2 ? tab_g : tg + 16;
+            lds128(tg, w_i, w_d, r_ie, r_de);
+          }
+          if constexpr (kDual) {
+            tg2 = tg2 + 16 == tab_g2 + 16 * re2 ? tab_g2 : tg2 + 16;
+            lds128(tg2, w_i2, w_d2, r_ie2, r_de2);
+          }
+          bool wider = false;
+          if (s >= grow_at) {
+            ++grow;
+            grow_at += a.pen.ge;
+            wider = true;
+          }
+          if constexpr (kDual) {
+            if (s >= grow2_at) {
+              ++grow2;
+              grow2_at += a.pen.ge2;
+              wider = true;
+            }
+          }
+          if (wider) {
+            const int g = kDual ? max(grow, grow2) : grow;
+            if (g > grow_lim) {
+              st = kPairScratch;  // wider than the ring's window
+              break;
+            }
+            lo = max(lo0 - g, -m);
+            hi = min(hi0 + g, n);
+            wlo = (lo - kbase) >> 1;
+            whi = (hi - kbase) >> 1;
+            hc0 = wlo >> kCS;
+            chunks = (whi >> kCS) - hc0 + 1;
+          }
+          if (s > s_lim) {
+            st = s > s_max ? kPairInternal : kPairScratch;
+            break;
+          }
+          if (!full) {
+            // a wavefront that does not exist is read as the row of absent cells
+            const bool px = (has_m >> (a.pen.x - 1)) & 1, po = (has_m >> (a.pen.go - 1)) & 1;
+            const bool pe = !kLin && ((has_g >> (a.pen.ge - 1)) & 1);
+            const bool po2 = kDual && ((has_m >> (a.pen.go2 - 1)) & 1);
+            const bool pe2 = kDual && ((has_g2 >> (a.pen.ge2 - 1)) & 1);
+            const bool pm = px | po | pe | po2 | pe2;
+            has_m = (has_m << 1) | (pm ? 1u : 0u);
+            if constexpr (!kLin) has_g = (has_g << 1) | ((po | pe) ? 1u : 0u);
+            if constexpr (kDual) has_g2 = (has_g2 << 1) | ((po2 | pe2) ? 1u : 0u);
+            if (!pm) {  // null step (wfa_gpu.cu:417-422); no row of it is read
+              --n_steps;
+              continue;
+            }
+            const unsigned long long dm = (1ull << (rm - 1)) - 1, dg = (1ull << a.pen.ge) - 1,
+                                     dg2 = kDual ? (1ull << a.pen.ge2) - 1 : 0;
+            full = (has_m & dm) == dm && (kLin || (has_g & dg) == dg) && (!kDual || (has_g2 & dg2) == dg2);
+            if (!px) r_mx = none_row;
+            if (!po) r_mo = none_row;
+            if constexpr (!kLin) {
+              if (!pe) r_ie = r_de = none_row;
+            }
+            if constexpr (kDual) {
+              if (!po2) r_mo2 = none_row;
+              if (!pe2) r_ie2 = r_de2 = none_row;
+            }
+          }
+          uint8_t* hrow = nullptr;
+          if constexpr (kCigar) {
+            if (hbase + chunks > hist_cap) {
+              st = kPairScratch;
+              break;
+            }
+            if (gt == 0) table[s] = make_int2(hc0, hbase);
+            hrow = reinterpret_cast<uint8_t*>(hist + (hbase - hc0));
+            hbase += chunks;
+          }
+          fk = INT_MAX;
+          // Every lane runs every iteration: lanes past the last word compute
+          // it again and store the same values to the same places.
+          for (int w0 = wlo + 32 * wig; w0 <= whi; w0 += GT) {
+            const int w = min(w0 + lane, whi);
+            const smem_t at = ring0 + 4 * w;
+            const uint32_t k2 = kw0 + (uint32_t)w * 0x00040004u;
+            const uint32_t ob = lds32(at + r_mo);
+            const uint32_t mo_l = h2_next(lds32<-4>(at + r_mo), ob);  // M[s-o-e] on k-1
+            const uint32_t mo_r = h2_next(ob, lds32<4>(at + r_mo));   // on k+1
+            const uint32_t mx = lds32(at + r_mx);
+            // I is kept as 2 (h - 1) + kZero, so that M[k-1] is its own
+            // insertion candidate; bit 0 of ins, del: extension; of t: deletion
+            // over insertion; of p: mismatch over both (ties go that way)
+            uint32_t ins = 0, del = 0, t, bits2 = 0;
+            if constexpr (!kLin) {
+              ins = h2_addmax(h2_next(lds32<-4>(at + r_ie), lds32(at + r_ie)), 3 * kOne2, mo_l);
+              del = h2_addmax(h2_next(lds32(at + r_de), lds32<4>(at + r_de)), kOne2, mo_r);
+              const uint32_t insc = ins & kClean;
+              sts32(at + w_i, insc);
+              sts32(at + w_d, del & kClean);
+              if constexpr (!kDual) {
+                t = h2_addmax(insc, 2 * kOne2, del | kOne2);
+              } else {
+                const uint32_t o2 = lds32(at + r_mo2);
+                const uint32_t mo2_l = h2_next(lds32<-4>(at + r_mo2), o2), mo2_r = h2_next(o2, lds32<4>(at + r_mo2));
+                const uint32_t ins2 = h2_addmax(h2_next(lds32<-4>(at + r_ie2), lds32(at + r_ie2)), 3 * kOne2, mo2_l);
+                const uint32_t del2 = h2_addmax(h2_next(lds32(at + r_de2), lds32<4>(at + r_de2)), kOne2, mo2_r);
+                sts32(at + w_i2, ins2 & kClean);
+                sts32(at + w_d2, del2 & kClean);
+                const uint32_t t1 = h2_max(insc, ins2 | kOne2);                      // I2 over I1
+                const uint32_t t2 = h2_addmax(t1 & kClean, 2 * kOne2, del | kOne2);  // D1 over both
+                t = h2_max(t2 & kClean, del2 | kOne2);                               // D2 over all
+                // bits 1..7 of the cell's byte (bit 0: mismatch, from p)
+                if constexpr (kCigar)
+                  bits2 = ((t & kOne2) << 1) | ((t2 & kOne2) << 2) | ((t1 & kOne2) << 3) | ((ins & kOne2) << 4) |
+                          ((del & kOne2) << 5) | ((ins2 & kOne2) << 6) | ((del2 & kOne2) << 7);
+              }
+            } else {
+              t = h2_addmax(mo_l, 2 * kOne2, mo_r | kOne2);
+            }
+            const uint32_t p = h2_addmax(mx, 3 * kOne2, t & kClean);
+            // extend both M cells: clamp into [first, last] offset of the
+            // diagonal (absent cells compare some window of it), compare 16
+            // bases at the halfword's place, add twice the matches
+            const uint32_t up = h2_min(k2, kend2) + m2;  // min(n, m + k)
+            const uint32_t c = h2_min(h2_max(p & kClean, h2_max(k2, kZero2)), up);
+            const uint32_t vv = c - k2 + kZero2;
+            constexpr int kZeroByte = (int)(kZero >> 5) * 4;  // byte offset of halfword kZero's base word
+            const smem_t h0 = tws + (((c & 0xffffu) >> 5) << 2), h1 = tws + ((c >> 21) << 2);
+            const smem_t v0 = pws + (((vv & 0xffffu) >> 5) << 2), v1 = pws + ((vv >> 21) << 2);
+            const uint32_t x0 = __funnelshift_r(lds32<-kZeroByte>(v0), lds32<4 - kZeroByte>(v0), vv) ^
+                                __funnelshift_r(lds32<-kZeroByte>(h0), lds32<4 - kZeroByte>(h0), c);
+            const uint32_t x1 = __funnelshift_r(lds32<-kZeroByte>(v1), lds32<4 - kZeroByte>(v1), vv >> 16) ^
+                                __funnelshift_r(lds32<-kZeroByte>(h1), lds32<4 - kZeroByte>(h1), c >> 16);
+            const uint32_t valid = h2_signmask(p);
+            uint32_t z = (uint32_t)(h2_tz(x0) + (h2_tz(x1) << 16)) & 0x003e003eu & valid;
+            if (z & 0x00200020u) {  // a whole window matched: go on in that half
+#pragma unroll 1
+              for (int half = 0; half < 32; half += 16) {
+                if ((z >> half) & 0x20u) {
+                  const int h = (int)(((c >> half) & 0xffffu) - kZero) >> 1, v = (int)(((vv >> half) & 0xffffu) - kZero) >> 1;
+                  const int rem = min(m - v, n - h) - 16;
+                  if (rem > 0) z += (uint32_t)(2 * lds_lcp(pws, v + 16, tws, h + 16, rem)) << half;
+                }
+              }
+            }
+            const uint32_t om = h2_addmin(c, z, up) & valid;
+            if (w0 + lane <= whi) n_ext2 = h2_sum(om - (c & valid), n_ext2);
+            sts32(at + w_m, om);
+            if constexpr (kEnds) {
+              const int k = kbase + 2 * w;
+              if ((valid & 1u) && k >= lo && ends_at((int)((om & 0xffffu) - kZero) >> 1, k)) fk = min(fk, k);
+              if ((valid >> 31) && k < hi && ends_at((int)((om >> 16) - kZero) >> 1, k + 1)) fk = min(fk, k + 1);
+            }
+            if constexpr (kCigar) {
+              if constexpr (kDual) {
+                const uint32_t f = (p & kOne2) | bits2;
+                reinterpret_cast<uint16_t*>(hrow)[w] = (uint16_t)(f | (f >> 8));
+              } else if constexpr (kLin) {
+                const uint32_t f = (p & kOne2) | ((t & kOne2) << 1);
+                hrow[w] = (uint8_t)(f | (f >> 12));
+              } else {
+                const uint32_t f1 = (p & kOne2) | ((t << 1) & (2 * kOne2));
+                const uint32_t f2 = (ins & kOne2) | ((del << 1) & (2 * kOne2));
+                const uint32_t f = f1 | (f2 << 2);
+                hrow[w] = (uint8_t)(f | (f >> 12));
+              }
+            }
+          }
+          n_cells += (unsigned)(hi - lo + 1);
+          ended(fk, w_m, kEnds);
+        }
+      };
+      if (ends_free)
+        steps(std::true_type{});
+      else
+        steps(std::false_type{});
+      n_steps += (uint32_t)s + (st == kPairOk ? 1u : 0u);
+
+      if (st == kPairOk) {
+        if (gt == 0) a.score[pair] = s_end * a.g;
+        if constexpr (kCigar) {
+          if (wig == 0) {
+            // reserve the run bound 2*s/min_pen + 4 in the arena, then walk
+            const int64_t bound = 2 * (int64_t)(s_end / a.pen.min_pen()) + 4;  // + a free gap at each end
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(a.arena_cursor, (unsigned long long)bound);
+            at = __shfl_sync(FULL, at, 0);
+            int len = 0;
+            if ((int64_t)at + bound > a.arena_cap) {
+              st = kPairArena;
+            } else {
+              __syncwarp();
+              len = packed_cigar<kModel>(hist, hbase, table, s_end, k_fin, m, n, a.pen, kbase, lo0, hi0, pws, tws,
+                                         a.arena + at, (int)bound, lane);
+              if (len < 0) {
+                st = kPairInternal;
+                len = 0;
+              }
+            }
+            if (lane == 0) {
+              a.cig_pos[pair] = (int64_t)at;
+              a.cig_len[pair] = len;
+            }
+          }
+        }
+      }
+    }
+    if (a.work) {
+      const unsigned we = __reduce_add_sync(FULL, n_ext2 >> 1);
+      if (lane == 0 && we) atomicAdd(a.work + 2, (unsigned long long)we);
+    }
+    if (gt == 0) {
+      a.status[pair] = st;
+      if (st == kPairScratch || st == kPairArena) {
+        const unsigned r = atomicAdd(a.retry_count, 1u);
+        a.retry[r] = (int32_t)pair;
+      }
+      if (a.work) {
+        atomicAdd(a.work, n_cells);
+        atomicAdd(a.work + 1, (unsigned long long)n_steps);
+      }
+    }
+    group_sync<GW>(gid);  // the group's shared memory is free for the next pair
+  }
+}
+
+}  // namespace tsu

@@ -41,7 +41,10 @@ struct PassGeom {
 constexpr int kSharedW1 = 384;         // shared-mode ring width for one warp per pair (diagonals)
 constexpr int kSharedSeqWords1 = 544;  // staging area for one warp per pair (uint32 words)
 constexpr int kSharedSeqWordsN = 4096; // staging area for a group of warps
-constexpr int kSharedMaxLen = 32000;   // int16 ring limit
+constexpr int kSharedMaxLen = 32000;   // int16 ring limit of the low-memory kernels
+// A launch of the packed kernel takes pairs up to the end of their length
+// band; the few beyond kPackedMaxLen are handed back one by one.
+constexpr int kPackedPlanLen = 16383;
 // widest int16 ring: a negative (invalid) I value grows by one per diagonal
 // of the ring's width and must stay negative (the kernel's store clamp)
 constexpr int kSharedMaxW = 16368;
@@ -66,7 +69,7 @@ inline int shared_ring_width(const Pen& pen, int gw, int seq_cap, int smem_optin
   const int gpc = cta_threads_for(gw) / (32 * gw);
   const int per_group = per_cta / gpc;
   const int fixed = group_smem_bytes(pen, 0, kModeShared, seq_cap, gw) + 16;
-  const int w = std::min((per_group - fixed) / (2 * ns), kSharedMaxW);
+  const int w = std::min((per_group - fixed) / (2 * (ns + 1)), kSharedMaxW);
   return std::max(0, w & ~15);
 }
 
@@ -78,7 +81,7 @@ inline int shared_cap(const Pen& pen, int gw, int seq_cap, int smem_optin) {
   if (gw != 1) return shared_ring_width(pen, gw, seq_cap, smem_optin);
   const int gpc = cta_threads_for(1) / 32;
   if (gpc * group_smem_bytes(pen, kSharedW1, kModeShared, seq_cap, 1) <= smem_optin) return kSharedW1;
-  const int w = (smem_optin / gpc - group_smem_bytes(pen, 0, kModeShared, seq_cap, 1) - 16) / (2 * pen.slots());
+  const int w = (smem_optin / gpc - group_smem_bytes(pen, 0, kModeShared, seq_cap, 1) - 16) / (2 * (pen.slots() + 1));
   return std::max(0, w & ~15);
 }
 
@@ -99,7 +102,8 @@ inline PassGeom plan_geometry(const Pen& pen, int32_t max_m, int32_t max_n, int 
   p.gw = gw;
   p.cta_threads = cta_threads_for(gw);
   p.groups_per_cta = p.cta_threads / (32 * gw);
-  p.mode = (mode == kModeShared && maxlen <= kSharedMaxLen) ? kModeShared : kModeGlobal;
+  const bool fits = lowmem ? maxlen <= kSharedMaxLen : (maxlen <= kPackedPlanLen && pen.rm <= kPackedMaxDepth);
+  p.mode = (mode == kModeShared && fits) ? kModeShared : kModeGlobal;
   if (p.mode == kModeShared) {
     const int64_t seqw = 2 * packed_words(max_m) + 2 * packed_words(max_n);
     p.seq_cap = (int)std::min<int64_t>(seqw, gw == 1 ? kSharedSeqWords1 : kSharedSeqWordsN);
@@ -124,7 +128,11 @@ inline PassGeom plan_geometry(const Pen& pen, int32_t max_m, int32_t max_n, int 
   p.table_cap = want_cigar ? (int)std::min<int64_t>(s_hint + 1, INT32_MAX / 2) : 0;
   if (want_cigar) {
     const int64_t sq = s_hint * s_hint / ge + 2 * s_hint + 64;
-    p.hist_cap = std::min<int64_t>(std::min<int64_t>(sq, (s_hint + 1) * width_hint), INT32_MAX - 64);
+    int64_t cells = std::min<int64_t>(sq, (s_hint + 1) * width_hint);
+    // the packed kernel keeps 4 bits per cell (8 with two gap pieces), each
+    // score's row rounded out to whole words at both ends
+    if (p.mode == kModeShared && !lowmem) cells = std::min<int64_t>(cells / (pen.dual() ? 4 : 8) + 3 * (s_hint + 1) + 64, INT32_MAX - 65536);
+    p.hist_cap = std::min<int64_t>(cells, INT32_MAX - 64);
   }
   p.ring_ints = p.mode == kModeShared ? 0 : (int64_t)ns * p.ring_w;
   if (lowmem) {
@@ -156,7 +164,7 @@ inline PassGeom plan_geometry(const Pen& pen, int32_t max_m, int32_t max_n, int 
 inline PassChoice next_pass(PassChoice prev, const Pen& pen, int32_t max_m, int32_t max_n, int smem_optin,
                             int global_gw = 16) {
   const int64_t need_w = (int64_t)max_m + max_n + 3;
-  if (prev.mode == kModeShared && std::max(max_m, max_n) <= kSharedMaxLen) {
+  if (prev.mode == kModeShared && std::max(max_m, max_n) <= kPackedMaxLen && pen.rm <= kPackedMaxDepth) {
     const int64_t seqw =
         std::min<int64_t>(2 * packed_words(max_m) + 2 * packed_words(max_n), kSharedSeqWordsN);
     static const int kGW[] = {2, 4, 8, 16};
@@ -181,7 +189,7 @@ inline PassChoice fit_start(PassChoice pc, const Pen& pen, int32_t max_m, int32_
   const int64_t w =
       std::min<int64_t>((int64_t)max_m + max_n + 3, 2 * hint_score(pen, maxlen, hint) / pen.min_ge() + 3);
   if (pc.mode != kModeShared) return {kModeGlobal, w > 16384 ? 32 : pc.gw};
-  if (maxlen > kSharedMaxLen) return {kModeGlobal, w > 16384 ? 32 : std::max(8, pc.gw)};
+  if (maxlen > kPackedMaxLen || pen.rm > kPackedMaxDepth) return {kModeGlobal, w > 16384 ? 32 : std::max(8, pc.gw)};
   const int64_t seqw = 2 * packed_words(max_m) + 2 * packed_words(max_n);
   static const int kGW[] = {1, 2, 4, 8, 16};
   for (int gw : kGW) {
@@ -211,7 +219,7 @@ inline int length_band(int32_t L) {
 // compiled one), adjusted for lengths beyond the int16 shared ring.
 inline PassChoice band_start_in(const PassChoice* table, int band, int32_t maxlen) {
   PassChoice r = table[band < 0 ? 0 : (band >= kBands ? kBands - 1 : band)];
-  if (r.mode == kModeShared && maxlen > kSharedMaxLen) r = {kModeGlobal, r.gw >= 8 ? r.gw : 8};
+  if (r.mode == kModeShared && maxlen > kPackedPlanLen) r = {kModeGlobal, r.gw >= 8 ? r.gw : 8};
   return r;
 }
 inline const PassChoice* band_start_table(bool dual = false) {
@@ -233,7 +241,7 @@ inline double next_hint(double hint, bool grow) { return grow ? std::min(hint * 
 inline int64_t arena_runs(const Pen& pen, int64_t n, int32_t max_m, int32_t max_n, double hint) {
   const int64_t maxlen = std::max(max_m, max_n);
   const int64_t per_pair = 2 * hint_score(pen, maxlen, hint) / pen.min_pen() + 1;
-  return std::max<int64_t>(n * std::min<int64_t>(per_pair, (int64_t)max_m + max_n + 1), 1024);
+  return std::max<int64_t>(n * (std::min<int64_t>(per_pair, (int64_t)max_m + max_n + 1) + 3), 1024);
 }
 
 }  // namespace tsu
