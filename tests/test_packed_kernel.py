@@ -41,10 +41,10 @@ def test_null_steps_and_deep_rings(emu, oracle, pen):  # noqa: F811
 
 
 def test_longest_sides(emu, oracle):  # noqa: F811
-    """Sides of 16,352 (the longest) and 16,353 bases (handed back), with runs of matches over many 512-base comparisons."""
+    """Sides of 16,351 (the longest) and 16,352 bases (handed back), with runs of matches over many 512-base comparisons."""
     rng = random.Random(8)
     pairs = []
-    for n in (16352, 16353):
+    for n in (16351, 16352):
         p = _rand(rng, n)
         t = list(p)
         t[5] = "ACGT"[("ACGT".index(t[5]) + 1) % 4]

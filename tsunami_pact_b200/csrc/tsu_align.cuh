@@ -56,6 +56,7 @@ __device__ __forceinline__ void group_sync(int gid) {
 #ifdef TSU_WARP_EMU
     emu::named_bar(1 + gid, 32 * GW);
 #else
+    __syncwarp();  // bar.sync counts warps: every lane must arrive with its warp
     asm volatile("bar.sync %0, %1;" ::"r"(1 + gid), "r"(32 * GW) : "memory");
 #endif
   }
@@ -820,17 +821,35 @@ __device__ __forceinline__ void align_ring(const AlignArgs& a, unsigned char* sm
   }
 }
 
+// Bounded launches run two words at a time (packed_words_step, U = 2): 128
+// registers, 16 warps per SM.
+template <int kMode, int GW, int kModel>
+constexpr int kernel_min_blocks() {
+  return (kModel & kBoundFlag) ? (GW <= 4 ? 4 : (GW == 8 ? 2 : 1)) : cta_min_blocks<kMode, GW>();
+}
+
 template <bool kCigar, int kMode, int GW, int kModel = kModelAffine>
-__global__ void __launch_bounds__(cta_threads<GW>(), (cta_min_blocks<kMode, GW>())) align_kernel(AlignArgs a) {
+__global__ void __launch_bounds__(cta_threads<GW>(), (kernel_min_blocks<kMode, GW, kModel>())) align_kernel(AlignArgs a) {
 #ifdef TSU_WARP_EMU
   unsigned char* smem_raw = emu::dyn_smem();  // CPU warp emulation of the tests
 #else
   extern __shared__ __align__(16) unsigned char smem_raw[];
 #endif
   if constexpr (kMode == kModeShared && !(kModel & kLowMemFlag))
-    align_packed<kCigar, GW, kModel>(a, smem_raw);
+    align_packed<kCigar, GW, kModel & 7, (kModel & kBoundFlag) != 0>(a, smem_raw);
   else
     align_ring<kCigar, kMode, GW, kModel>(a, smem_raw);
+}
+
+constexpr int kProbeThreads = 128;
+template <int kModel>
+__global__ void __launch_bounds__(kProbeThreads, 5) probe_kernel(ProbeArgs a) {
+#ifdef TSU_WARP_EMU
+  unsigned char* smem_raw = emu::dyn_smem();
+#else
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+#endif
+  probe_packed<kModel>(a, smem_raw);
 }
 
 }  // namespace tsu

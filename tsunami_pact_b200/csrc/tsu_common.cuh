@@ -31,6 +31,9 @@ enum : int { kModelAffine = 0, kModelDual = 1, kModelLinear = 2 };
 // added to a model: the low-memory (checkpointed history) variant of its
 // CIGAR kernels
 enum : int { kLowMemFlag = 8 };
+// added to a model: the shared-ring kernels of pairs with score bounds
+// (AlignArgs::bound)
+enum : int { kBoundFlag = 16 };
 
 struct SeqView {
   int64_t n;  // pairs
@@ -128,6 +131,8 @@ inline Pen reduce_linear(int mismatch, int ext, int* g) {
   return p;
 }
 
+constexpr int32_t kNoBound = 0x7f7f7f7f;  // a pair without a score bound (bytes 0x7f: set by memset)
+
 struct AlignArgs {
   SeqView seq;
   PackView pk;
@@ -164,7 +169,47 @@ struct AlignArgs {
   uint8_t* ckpt;
   int64_t ckpt_stride;
   int32_t ckpt_bytes, ckpt_cap, ckpt_k;
+  // upper bounds of the pairs' scores in score units ([n], kNoBound: none;
+  // nullptr: none of them): the shared-ring kernel computes only diagonals
+  // that a path within the bound can use (end-to-end pairs only)
+  const int32_t* bound;
+  int group_bytes;  // bounded launches: shared memory per group
 };
+
+// The bound probe (tsu_packed.cuh).
+constexpr int kProbeW = 128;
+struct ProbeArgs {
+  SeqView seq;
+  PackView pk;
+  const int32_t* order;
+  int64_t n_order;
+  Pen pen;
+  int seq_cap;       // shared-memory sequence words (uint32) per warp
+  int32_t* bound;    // [n]
+  unsigned int* queue;
+};
+
+// Diagonals [lo, hi] that an end-to-end path of cost at most ub can visit,
+// and two more on each side: at score s up to g(s) from 0 (gap openings and
+// extensions) and up to (ub - s) / e from n - m; the two lines cross at lo and
+// hi.
+__host__ __device__ inline void bound_reach(const Pen& p, int m, int n, int ub, int* lo, int* hi) {
+  const int64_t e = p.min_ge();
+  auto side = [&](int64_t k_end) -> int64_t {  // furthest diagonal towards k_end's positive side
+    int64_t best = k_end > 0 ? k_end : 0;
+    auto piece = [&](int64_t go, int64_t ge) {
+      const int64_t s = ((k_end - 1) * ge * e + (int64_t)ub * ge + go * e) / (ge + e);
+      const int64_t v = s >= go ? 1 + (s - go) / ge : 0;
+      if (v > best) best = v;
+    };
+    piece(p.go, p.ge);
+    if (p.dual()) piece(p.go2, p.ge2);
+    return best + 2;
+  };
+  const int64_t h = side(n - m), l = side(m - n);
+  *hi = (int)(h < n ? h : n);
+  *lo = (int)(l < m ? -l : -m);
+}
 
 // Bytes of one low-memory checkpoint: limits (3 ints per slot), then the
 // ring's values (ring_w per slot) in the ring's element type.
@@ -177,16 +222,27 @@ __host__ __device__ inline int64_t ckpt_bytes_for(const Pen& p, int ring_w, int 
 __host__ __device__ inline int partial_words(const Pen& p) { return p.dual() ? 16 : 8; }
 
 // The shared-ring kernel (tsu_packed.cuh): longest side its 16-bit offsets
-// hold (2 h + 32768 plus one 16-base window past the end stays below 65536),
+// hold (tsu_packed.cuh),
 // deepest ring its 64-bit record of the last scores covers, 32-bit words per
 // ring row (ring_w halfwords and 4 on each side) and bytes before the ring
 // (4 broadcast words, 2 gw partials, 16 bytes of row offsets per M slot and
 // per I / D slot pair).
-constexpr int kPackedMaxLen = 16352;
+constexpr int kPackedPlainLen = 16351;  // launches without score bounds
+constexpr int kPackedMaxLen = 20463;    // launches with them, and the probe
+constexpr int kPackedMaxW = 12288;  // diagonals per ring row (absent I cells climb 2 per diagonal, below offset 0)
 constexpr int kPackedMaxDepth = 64;
-__host__ __device__ inline int packed_row_words(int ring_w) { return (ring_w + 8) / 2; }
+__host__ __device__ constexpr int packed_row_words(int ring_w) { return (ring_w + 8) / 2; }
 __host__ __device__ inline int packed_head_bytes(const Pen& p, int gw) {
   return ((16 + 8 * gw + 15) & ~15) + 16 * (p.rm + p.re + p.re2);
+}
+
+// Ring width of a window of d diagonals (one more where its first is odd);
+// rows are whole 16-byte pieces.
+__host__ __device__ inline int packed_width(int d) { return d < 16 ? 16 : (d + 1 + 15) & ~15; }
+// Shared memory a bounded pair needs: d diagonals, words 32-bit words of
+// sequence, gw warps.
+__host__ __device__ inline int bounded_bytes(const Pen& p, int d, int words, int gw) {
+  return (packed_head_bytes(p, gw) + (p.slots() + 1) * packed_row_words(packed_width(d)) * 4 + words * 4 + 15) & ~15;
 }
 
 // Shared memory per group of gw warps, in bytes.  Global mode and the
@@ -207,6 +263,11 @@ __host__ __device__ inline int group_smem_bytes(const Pen& p, int ring_w, int mo
     b = ((b + 15) & ~15) + 16 + seq_cap * 4;
   }
   return (b + 15) & ~15;
+}
+
+// Shared memory per warp of the bound probe.
+__host__ __device__ inline int probe_smem_bytes(const Pen& p, int seq_cap) {
+  return 16 * (p.rm + p.re + p.re2) + (p.slots() + 1) * packed_row_words(kProbeW) * 4 + ((seq_cap * 4 + 15) & ~15);
 }
 
 // Packed 64-bit words allocated per sequence of len bases: ceil(len / 32)

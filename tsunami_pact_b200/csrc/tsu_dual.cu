@@ -6,13 +6,21 @@
 namespace tsu {
 
 cudaError_t align_occupancy_dual(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ,
-                                 bool lowmem) {
-  return launch_detail::occupancy<kModelDual>(cigar, mode, gw, threads, smem, optin, occ, lowmem);
+                                 bool lowmem, bool bounded) {
+  return launch_detail::occupancy<kModelDual>(cigar, mode, gw, threads, smem, optin, occ, lowmem, bounded);
 }
 
 void launch_align_dual(bool cigar, int mode, int gw, int blocks, int threads, size_t smem, cudaStream_t st,
-                       const AlignArgs& a, bool lowmem) {
-  launch_detail::launch<kModelDual>(cigar, mode, gw, blocks, threads, smem, st, a, lowmem);
+                       const AlignArgs& a, bool lowmem, bool bounded) {
+  launch_detail::launch<kModelDual>(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded);
+}
+
+cudaError_t probe_occupancy_dual(int threads, size_t smem, int optin, int* occ) {
+  return launch_detail::probe_occupancy<kModelDual>(threads, smem, optin, occ);
+}
+
+void launch_probe_dual(int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {
+  launch_detail::probe<kModelDual>(blocks, threads, smem, st, a);
 }
 
 }  // namespace tsu

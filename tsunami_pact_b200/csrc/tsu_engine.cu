@@ -43,6 +43,13 @@ struct HostBuf {
   size_t cap = 0;
 };
 
+// Launches of a call before the retry ladders: length bands, then classes of
+// pairs with a score bound and the bands of pairs whose bound did not help,
+// the latter twice (pairs bounded at once, pairs bounded after a first pass).
+constexpr int kRunSlots = tsu::kBands + 2 * (tsu::kBoundClasses + tsu::kBands);
+// Streams beside the context's own for the launches of bounded classes.
+constexpr int kSideStreams = 3;
+
 struct Pass {
   tsu::PassGeom g;
   int64_t groups = 0;  // pairs in flight (groups of g.gw warps)
@@ -76,11 +83,14 @@ struct tsu_ctx {
   DevBuf b_rwords, b_rnonacgt, b_segs, b_bout;            // bidirectional mode: reversed words, segments, cuts
   DevBuf b_bsegs, b_boff, b_blen, b_bruns, b_bfirst;      // bidirectional CIGARs: base cases, their runs
   DevBuf b_pre;                                           // bidirectional CIGARs: the whole-pair launch's results
+  DevBuf b_bound;                                         // score bounds of the pairs (bound probe)
   bool one_warp = false;  // TSU_ONE_WARP of the current call
   bool bidir = false;     // TSU_BIDIRECTIONAL of the current call
   cudaEvent_t pev[2] = {};  // per-pass timing
   std::string passlog;      // passes of the last align call (tsu_pass_log)
   cudaStream_t h2d_stream = nullptr, d2h_stream = nullptr;  // chunk pipeline copy streams
+  cudaStream_t side[kSideStreams] = {};  // classes of bounded pairs, side by side
+  cudaEvent_t fork_ev = nullptr;
   cudaEvent_t fence_ev[2] = {};  // orders frees after the copy streams' queued work
   cudaMemPool_t pool = nullptr;  // the device's buffer pool
   bool exact_grow = false;       // grow buffers to the asked size only
@@ -94,6 +104,7 @@ struct tsu_ctx {
   HostBuf h_list;     // int32 pass order / retry list
   HostBuf h_status;   // int32 pair statuses (tsu_align_batch)
   HostBuf h_bidir;    // bidirectional mode: segments down, cuts and run counts up
+  HostBuf h_bound;    // score bounds of the pairs
   std::vector<void*> h_retired;  // outgrown page-locked buffers, freed at destroy
   // events of the host-buffer pipeline (tsu_align_batch): 8 chunks at most
   cudaEvent_t cev_up[8] = {}, cev_done[8] = {}, cev_down[8] = {}, cev_t[2] = {};
@@ -108,7 +119,7 @@ struct tsu_ctx {
   bool capturing = false;
   cudaGraphExec_t gexec = nullptr;
   int64_t graph_launches = 0;
-  cudaEvent_t bev[2 * tsu::kBands] = {};  // first pass of each band: start, end
+  cudaEvent_t bev[2 * kRunSlots] = {};  // first pass of each band or class: start, end
   cudaEvent_t wait_ev = nullptr;  // blocking-sync event of those waits
   size_t need_bytes = 0;         // budget the last TSU_ENOMEM step needed
   size_t peak_held = 0;          // most bytes held during the current call (tsu_timing.device_bytes)
@@ -122,7 +133,7 @@ struct tsu_ctx {
     return {&b_pat,  &b_txt,    &b_poff,     &b_toff,  &b_plen,  &b_tlen,   &b_words_cnt, &b_woff, &b_words,
             &b_nonacgt, &b_score, &b_status, &b_cpos, &b_clen, &b_clen64, &b_coff,      &b_out,  &b_order,
             &b_retry, &b_counters, &b_scratch, &b_arena, &b_scan_tmp, &b_out2, &b_rwords, &b_rnonacgt,
-            &b_segs,  &b_bout, &b_bsegs, &b_boff, &b_blen, &b_bruns, &b_bfirst, &b_pre};
+            &b_segs,  &b_bout, &b_bsegs, &b_boff, &b_blen, &b_bruns, &b_bfirst, &b_pre, &b_bound};
   }
   size_t held() const {
     size_t s = 0;
@@ -294,24 +305,50 @@ struct BatchInfo {
 // lowmem: the checkpointed-history variant (CIGAR passes of a low-memory
 // context).
 cudaError_t align_occupancy(const tsu_ctx* ctx, bool cigar, int mode, int gw, int threads, size_t smem, int optin,
-                            int* occ, bool lowmem) {
+                            int* occ, bool lowmem, bool bounded) {
   switch (ctx->rp.model()) {
-    case tsu::kModelDual: return tsu::align_occupancy_dual(cigar, mode, gw, threads, smem, optin, occ, lowmem);
-    case tsu::kModelLinear: return tsu::align_occupancy_linear(cigar, mode, gw, threads, smem, optin, occ, lowmem);
+    case tsu::kModelDual: return tsu::align_occupancy_dual(cigar, mode, gw, threads, smem, optin, occ, lowmem, bounded);
+    case tsu::kModelLinear: return tsu::align_occupancy_linear(cigar, mode, gw, threads, smem, optin, occ, lowmem, bounded);
     default:
-      return tsu::launch_detail::occupancy<tsu::kModelAffine>(cigar, mode, gw, threads, smem, optin, occ, lowmem);
+      return tsu::launch_detail::occupancy<tsu::kModelAffine>(cigar, mode, gw, threads, smem, optin, occ, lowmem, bounded);
   }
 }
 
 void launch_align(const tsu_ctx* ctx, bool cigar, int mode, int gw, int blocks, int threads, size_t smem,
                   cudaStream_t st, const tsu::AlignArgs& a) {
-  const bool lowmem = cigar && a.ckpt_k > 0;
+  const bool lowmem = cigar && a.ckpt_k > 0, bounded = a.bound != nullptr;
   switch (ctx->rp.model()) {
-    case tsu::kModelDual: tsu::launch_align_dual(cigar, mode, gw, blocks, threads, smem, st, a, lowmem); break;
-    case tsu::kModelLinear: tsu::launch_align_linear(cigar, mode, gw, blocks, threads, smem, st, a, lowmem); break;
+    case tsu::kModelDual: tsu::launch_align_dual(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded); break;
+    case tsu::kModelLinear: tsu::launch_align_linear(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded); break;
     default:
-      tsu::launch_detail::launch<tsu::kModelAffine>(cigar, mode, gw, blocks, threads, smem, st, a, lowmem);
+      tsu::launch_detail::launch<tsu::kModelAffine>(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded);
       break;
+  }
+}
+
+// Launch shape of the bound probe (tsu_packed.cuh) over n pairs.
+int plan_probe(tsu_ctx* ctx, int seq_cap, int64_t n, int* blocks, size_t* smem) {
+  const int wpb = tsu::kProbeThreads / 32;
+  *smem = (size_t)wpb * tsu::probe_smem_bytes(ctx->rp, seq_cap);
+  int occ = 0;
+  cudaError_t e = cudaSuccess;
+  switch (ctx->rp.model()) {
+    case tsu::kModelDual: e = tsu::probe_occupancy_dual(tsu::kProbeThreads, *smem, ctx->smem_optin, &occ); break;
+    case tsu::kModelLinear: e = tsu::probe_occupancy_linear(tsu::kProbeThreads, *smem, ctx->smem_optin, &occ); break;
+    default:
+      e = tsu::launch_detail::probe_occupancy<tsu::kModelAffine>(tsu::kProbeThreads, *smem, ctx->smem_optin, &occ);
+      break;
+  }
+  if (e != cudaSuccess) return set_err(ctx, TSU_EDEVICE, "probe occupancy query failed (%d)", (int)e);
+  *blocks = (int)std::min<int64_t>((int64_t)ctx->sms * occ, (n + wpb - 1) / wpb);  // 0: does not fit
+  return TSU_OK;
+}
+
+void launch_probe(const tsu_ctx* ctx, int blocks, size_t smem, cudaStream_t st, const tsu::ProbeArgs& a) {
+  switch (ctx->rp.model()) {
+    case tsu::kModelDual: tsu::launch_probe_dual(blocks, tsu::kProbeThreads, smem, st, a); break;
+    case tsu::kModelLinear: tsu::launch_probe_linear(blocks, tsu::kProbeThreads, smem, st, a); break;
+    default: tsu::launch_detail::probe<tsu::kModelAffine>(blocks, tsu::kProbeThreads, smem, st, a); break;
   }
 }
 
@@ -321,20 +358,16 @@ size_t group_scratch_bytes(const tsu::PassGeom& g) {
                   64);
 }
 
-// Configure a pass of configuration pc over pairs of at most bi's lengths:
-// geometry, then as many groups as fit the SMs, the pairs and `avail` bytes
-// of scratch.
-int plan_pass_within(tsu_ctx* ctx, const BatchInfo& bi, int64_t n_pairs, tsu::PassChoice pc, double hint,
-                     bool want_cigar, size_t avail, Pass* out) {
+// The launch of geometry g: as many groups as fit the SMs, the pairs and
+// `avail` bytes of scratch.
+int plan_groups(tsu_ctx* ctx, const tsu::PassGeom& g, int64_t n_pairs, bool want_cigar, size_t avail, Pass* out) {
   Pass p;
-  const tsu::PassGeom g = tsu::plan_geometry(ctx->rp, bi.max_m, bi.max_n, pc.mode, pc.gw, hint, want_cigar,
-                                             ctx->smem_optin, want_cigar ? ctx->low_mem : 0);
   p.g = g;
   const int gpc = g.groups_per_cta;
   int occ = 0;
   cudaError_t e =
       align_occupancy(ctx, want_cigar, g.mode, g.gw, g.cta_threads, (size_t)gpc * g.group_smem, ctx->smem_optin, &occ,
-                      g.ckpt_k > 0);
+                      g.ckpt_k > 0, g.bounded);
   if (e != cudaSuccess || occ < 1) return set_err(ctx, TSU_EDEVICE, "occupancy query failed (%d)", (int)e);
   int64_t warps = (int64_t)ctx->sms * occ * gpc;  // groups
   const size_t per_warp = group_scratch_bytes(g);
@@ -360,6 +393,14 @@ int plan_pass_within(tsu_ctx* ctx, const BatchInfo& bi, int64_t n_pairs, tsu::Pa
   p.smem_bytes = (size_t)gpb * g.group_smem;
   *out = p;
   return TSU_OK;
+}
+
+// A pass of configuration pc over pairs of at most bi's lengths.
+int plan_pass_within(tsu_ctx* ctx, const BatchInfo& bi, int64_t n_pairs, tsu::PassChoice pc, double hint,
+                     bool want_cigar, size_t avail, Pass* out) {
+  const tsu::PassGeom g = tsu::plan_geometry(ctx->rp, bi.max_m, bi.max_n, pc.mode, pc.gw, hint, want_cigar,
+                                             ctx->smem_optin, want_cigar ? ctx->low_mem : 0);
+  return plan_groups(ctx, g, n_pairs, want_cigar, avail, out);
 }
 
 // plan_pass_within with the budget left beside the context's other buffers
@@ -410,6 +451,19 @@ void split_bands(int64_t n, const int32_t* h_plen, const int32_t* h_tlen, BandSp
   }
   for (int64_t i = 0; i < n; ++i) by_len[(size_t)start[cls(i)]++] = (int32_t)i;
   for (int32_t i : by_len) out->bands[(size_t)tsu::length_band(std::max(h_plen[i], h_tlen[i]))].push_back(i);
+}
+
+// The bands without the pairs that wait for a score bound.
+void drop_probed(int64_t n, const int32_t* h_plen, const int32_t* h_tlen, const std::vector<int32_t>& probed,
+                 BandSplit* split) {
+  std::vector<bool> out((size_t)n, false);
+  for (int32_t i : probed) out[(size_t)i] = true;
+  if (split->uniform)  // one length class: the bands were not filled
+    for (int64_t i = 0; i < n; ++i)
+      split->bands[(size_t)tsu::length_band(std::max(h_plen[i], h_tlen[i]))].push_back((int32_t)i);
+  split->uniform = false;
+  for (std::vector<int32_t>& b : split->bands)
+    b.erase(std::remove_if(b.begin(), b.end(), [&](int32_t i) { return out[(size_t)i]; }), b.end());
 }
 
 // Record an event on the stream; inside a stream capture as an event node
@@ -474,9 +528,9 @@ size_t scratch_bytes(const Pass& ps, bool cigar) {
   return std::max<size_t>(b, 256);
 }
 
-void carve_scratch(tsu_ctx* ctx, const Pass& ps, bool cigar, tsu::AlignArgs* a) {
+void carve_scratch(tsu_ctx* ctx, const Pass& ps, bool cigar, tsu::AlignArgs* a, size_t at = 0) {
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  char* p = P<char>(ctx->b_scratch);
+  char* p = P<char>(ctx->b_scratch) + at;
   const size_t groups = (size_t)ps.groups;
   a->hist = nullptr;
   a->table = nullptr;
@@ -1165,12 +1219,46 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   const tsu::PackView pk{P<uint64_t>(ctx->b_words), P<int64_t>(ctx->b_woff), P<uint8_t>(ctx->b_nonacgt)};
   if ((rc = grow(ctx, ctx->b_cpos, sizeof(int64_t) * n))) return rc;
   if ((rc = grow(ctx, ctx->b_clen, sizeof(int32_t) * n))) return rc;
-  if ((rc = grow(ctx, ctx->b_retry, sizeof(int32_t) * n))) return rc;
-  if ((rc = grow(ctx, ctx->b_order, sizeof(int32_t) * n))) return rc;
-  // counters: +16 arena cursor, +24 work (cells, steps, extension bases), +64 + 8b queue head
+  // pass orders and retry lists: the first passes', then those of pairs that
+  // got a bound after outgrowing theirs
+  if ((rc = grow(ctx, ctx->b_retry, sizeof(int32_t) * 2 * n))) return rc;
+  if ((rc = grow(ctx, ctx->b_order, sizeof(int32_t) * 2 * n))) return rc;
+  // counters: +8 the bound probe's queue head, +16 arena cursor, +24 work (cells, steps, extension bases), +64 + 8b queue head
   // and retry count of band slot b
-  constexpr size_t kCounterBytes = 64 + 8 * tsu::kBands;
+  constexpr size_t kCounterBytes = 64 + 8 * kRunSlots;
+  constexpr size_t kProbeQueue = 8;  // the bound probe's queue head
   if ((rc = grow(ctx, ctx->b_counters, kCounterBytes))) return rc;
+  // Pairs with a bound probe (tsu::wants_bound; end to end, history of every
+  // score): they wait for their bounds, the others start at once.
+  const bool can_bound = !ctx->one_warp && h_plen && ctx->rp.rm <= tsu::kPackedMaxDepth && !(want_cigar && ctx->low_mem) &&
+                         !(ctx->ends_free[0] | ctx->ends_free[1] | ctx->ends_free[2] | ctx->ends_free[3]);
+  std::vector<int32_t> probed;
+  if (can_bound) {
+    for (int64_t i = 0; i < n; ++i)
+      if (tsu::wants_bound(ctx->rp, h_plen[i], h_tlen[i])) probed.push_back((int32_t)i);
+    if ((int64_t)probed.size() <= ctx->sms)
+      probed.erase(std::remove_if(probed.begin(), probed.end(),
+                                  [&](int32_t i) { return std::max(h_plen[i], h_tlen[i]) < tsu::kBoundFewLen; }),
+                   probed.end());
+    if ((rc = grow(ctx, ctx->b_bound, sizeof(int32_t) * n))) return rc;
+    if ((rc = host_grow(ctx, ctx->h_bound, sizeof(int32_t) * (size_t)n))) return rc;
+    std::stable_sort(probed.begin(), probed.end(), [&](int32_t u, int32_t v) {
+      return (int64_t)h_plen[u] + h_tlen[u] > (int64_t)h_plen[v] + h_tlen[v];
+    });
+  }
+  struct ProbePlan {
+    int seq = 0, blocks = 0;
+    size_t smem = 0;
+  };
+  auto probe_plan = [&](const std::vector<int32_t>& list, ProbePlan* p) -> int {
+    for (int32_t i : list)
+      p->seq = std::max(p->seq, (int)(2 * tsu::packed_words(h_plen[i]) + 2 * tsu::packed_words(h_tlen[i])));
+    return list.empty() ? TSU_OK : plan_probe(ctx, p->seq, (int64_t)list.size(), &p->blocks, &p->smem);
+  };
+  ProbePlan probe;
+  if ((rc = probe_plan(probed, &probe))) return rc;
+  if (!probe.blocks) probed.clear();  // rings too deep for the probe's blocks
+  const int64_t n_probed = (int64_t)probed.size();
   const int min_pen = ctx->rp.min_pen();
   int64_t arena_cap = 0;
   if (want_cigar) {
@@ -1209,9 +1297,11 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     tsu::PassChoice pc;
     double hint = 0;
     Pass ps;
+    bool rebound = false;  // the pairs that outgrew it have run again with bounds
   };
   BandSplit split;
   if (!ctx->one_warp && h_plen) split_bands(n, h_plen, h_tlen, &split);
+  if (n_probed) drop_probed(n, h_plen, h_tlen, probed, &split);
   const bool all_pairs = ctx->one_warp || !h_plen || split.uniform;  // one band of every pair, input order
   std::vector<BandRun> runs;
   std::vector<int32_t> order_all;
@@ -1252,6 +1342,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       r.hint = ctx->err_hint;
       if (ctx->fit_start && !ctx->one_warp)
         r.pc = tsu::fit_start(r.pc, ctx->rp, r.bi.max_m, r.bi.max_n, r.hint, ctx->smem_optin);
+      if (!ctx->one_warp) r.pc = tsu::fill_warps(r.pc, r.n, ctx->sms);
       if ((rc = plan_pass_within(ctx, r.bi, r.n, r.pc, r.hint, want_cigar, avail, &r.ps))) return rc;
       need = std::max(need, scratch_bytes(r.ps, want_cigar));
     }
@@ -1260,6 +1351,8 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       if ((rc = grow(ctx, ctx->b_scratch, need))) return rc;
     }
   }
+  const int64_t probe_off = (int64_t)order_all.size();  // the probed pairs' slice of the order
+  order_all.insert(order_all.end(), probed.begin(), probed.end());
   if (!order_all.empty()) {
     if ((rc = host_grow(ctx, ctx->h_list, sizeof(int32_t) * order_all.size()))) return rc;
     memcpy(ctx->h_list.p, order_all.data(), sizeof(int32_t) * order_all.size());
@@ -1293,7 +1386,135 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     a.ef_pe = ctx->ends_free[1];
     a.ef_tb = ctx->ends_free[2];
     a.ef_te = ctx->ends_free[3];
+    a.bound = ps.g.bounded ? P<int32_t>(ctx->b_bound) : nullptr;
+    a.group_bytes = ps.g.group_smem;
     return a;
+  };
+  // The bound probe over `count` pairs of the order from `off` on, their bounds
+  // to ctx->h_bound.
+  auto queue_probe = [&](const ProbePlan& p, int64_t off, int64_t count) -> int {
+    CU(cudaMemsetAsync(ctx->b_bound.p, 0x7f, sizeof(int32_t) * n, st));  // kNoBound
+    tsu::ProbeArgs b{};
+    b.seq = sv;
+    b.pk = pk;
+    b.order = P<int32_t>(ctx->b_order) + off;
+    b.n_order = count;
+    b.pen = ctx->rp;
+    b.seq_cap = p.seq;
+    b.bound = P<int32_t>(ctx->b_bound);
+    b.queue = reinterpret_cast<unsigned int*>(d_cnt + kProbeQueue);
+    launch_probe(ctx, p.blocks, p.smem, st, b);
+    CU(cudaGetLastError());
+    CU(cudaMemcpyAsync(ctx->h_bound.p, ctx->b_bound.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
+    return TSU_OK;
+  };
+  // The probed pairs, their bounds in ctx->h_bound: classes by the width their
+  // bounds need, each one launch on the shared ring planned from the bounds;
+  // pairs without a bound, or too wide for a block's ring, by length band as
+  // the others.  Appends to runs and reads the counters back.
+  auto bounded_runs = [&](const std::vector<int32_t>& list, int64_t off) -> int {
+    const int32_t* ub = static_cast<const int32_t*>(ctx->h_bound.p);
+    struct Class {
+      std::vector<int32_t> pairs;
+      BatchInfo bi;
+      int bytes = 0;  // of shared memory, at 16 warps per pair
+      int32_t ub = 0;
+      int64_t hist = 0;
+    };
+    std::vector<Class> cls((size_t)tsu::kBoundClasses + tsu::kBands);
+    const size_t wide = (size_t)tsu::kBoundClasses;
+    for (int32_t i : list) {
+      const int32_t m = h_plen[i], t = h_tlen[i], u = ub[i];
+      size_t c = wide + (size_t)tsu::length_band(std::max(m, t));
+      tsu::BoundNeed need;
+      int bytes = 0;
+      if (u != tsu::kNoBound) {
+        need = tsu::bound_need(ctx->rp, m, t, u);
+        bytes = tsu::bounded_bytes(ctx->rp, need.width, need.words, 16);
+        int per_sm = 0;
+        if (tsu::packed_width(need.width) <= tsu::kPackedMaxW &&
+            tsu::bounded_warps(bytes, INT32_MAX, ctx->sms, ctx->smem_optin, &per_sm))
+          c = (size_t)tsu::bound_class(per_sm);
+      }
+      Class& k = cls[c];
+      k.pairs.push_back(i);
+      k.bi.max_m = std::max(k.bi.max_m, m);
+      k.bi.max_n = std::max(k.bi.max_n, t);
+      k.bytes = std::max(k.bytes, bytes);
+      k.ub = std::max(k.ub, u);
+      k.hist = std::max(k.hist, need.hist);
+    }
+    const size_t first = runs.size();
+    std::vector<int32_t> order;
+    const size_t fixed = ctx->held() - ctx->b_scratch.cap + out_reserve();
+    const size_t avail = ctx->budget > fixed ? ctx->budget - fixed : 0;
+    size_t need_bytes = 0, each = 0;
+    int rc2;
+    for (int j = 0; j < tsu::kBoundClasses + tsu::kBands; ++j) {
+      // unbounded bands first (longest first), then the widest class first
+      const int c = j < tsu::kBands ? tsu::kBoundClasses + tsu::kBands - 1 - j : j - tsu::kBands;
+      Class& k = cls[(size_t)c];
+      if (k.pairs.empty()) continue;
+      BandRun r;
+      r.slot = (int)runs.size();
+      r.off = off + (int64_t)order.size();
+      r.n = (int64_t)k.pairs.size();
+      r.bi = k.bi;
+      r.bi.n = r.n;
+      r.hint = ctx->err_hint;
+      int gw = 0;
+      if (c < tsu::kBoundClasses)
+        gw = tsu::bounded_warps(k.bytes, r.n, ctx->sms, ctx->smem_optin);
+      if (gw) {
+        r.pc = tsu::PassChoice{tsu::kModeShared, gw};
+        const tsu::PassGeom g = tsu::plan_bounded(k.bytes, k.ub, k.hist, gw, want_cigar);
+        if ((rc2 = plan_groups(ctx, g, r.n, want_cigar, avail, &r.ps))) return rc2;
+      } else {
+        r.band = c < tsu::kBoundClasses ? tsu::kBands - 1 : c - tsu::kBoundClasses;
+        r.pc = tsu::band_start_in(ctx->band_start, r.band, std::max(k.bi.max_m, k.bi.max_n));
+        if (ctx->fit_start) r.pc = tsu::fit_start(r.pc, ctx->rp, k.bi.max_m, k.bi.max_n, r.hint, ctx->smem_optin);
+        if ((rc2 = plan_pass_within(ctx, r.bi, r.n, r.pc, r.hint, want_cigar, avail, &r.ps))) return rc2;
+      }
+      need_bytes = std::max(need_bytes, scratch_bytes(r.ps, want_cigar));
+      each += scratch_bytes(r.ps, want_cigar);
+      order.insert(order.end(), k.pairs.begin(), k.pairs.end());
+      runs.push_back(r);
+    }
+    // The launches run side by side, each in its own part of the scratch, so
+    // that one class's last pairs and the next one's first share the SMs; one
+    // after the other when the budget does not hold them all at once.
+    const bool side = runs.size() - first > 1 && each <= avail;
+    if (side) need_bytes = each;
+    if (need_bytes > ctx->b_scratch.cap) {
+      release(ctx, ctx->b_scratch);
+      if ((rc2 = grow(ctx, ctx->b_scratch, need_bytes))) return rc2;
+    }
+    if ((rc2 = host_grow(ctx, ctx->h_list, sizeof(int32_t) * order.size()))) return rc2;
+    memcpy(ctx->h_list.p, order.data(), sizeof(int32_t) * order.size());
+    CU(cudaMemcpyAsync(P<int32_t>(ctx->b_order) + off, ctx->h_list.p, sizeof(int32_t) * order.size(),
+                       cudaMemcpyHostToDevice, st));
+    if (side) CU(cudaEventRecord(ctx->fork_ev, st));
+    size_t at = 0;
+    for (size_t j = first; j < runs.size(); ++j) {
+      const BandRun& r = runs[j];
+      tsu::AlignArgs a = align_args(r.ps, P<int32_t>(ctx->b_order) + r.off, r.n, r.slot, P<int32_t>(ctx->b_retry) + r.off);
+      const size_t lane = (j - first) % (kSideStreams + 1);
+      cudaStream_t cs = side && lane ? ctx->side[lane - 1] : st;
+      if (side) {
+        carve_scratch(ctx, r.ps, want_cigar, &a, at);
+        at += scratch_bytes(r.ps, want_cigar);
+        if (cs != st) CU(cudaStreamWaitEvent(cs, ctx->fork_ev, 0));
+      }
+      CU(cudaEventRecord(ctx->bev[2 * r.slot], cs));
+      launch_align(ctx, want_cigar, r.ps.g.mode, r.ps.g.gw, r.ps.blocks, r.ps.threads, r.ps.smem_bytes, cs, a);
+      CU(cudaGetLastError());
+      CU(cudaEventRecord(ctx->bev[2 * r.slot + 1], cs));
+      if (cs != st) CU(cudaStreamWaitEvent(st, ctx->bev[2 * r.slot + 1], 0));
+      ctx->timing.kernel_launches++;
+    }
+    CU(cudaMemcpyAsync(h_cnt, d_cnt, kCounterBytes, cudaMemcpyDeviceToHost, st));
+    CU(wait_stream(ctx, st));
+    return TSU_OK;
   };
   std::string passlog;  // mode, warps per pair x groups : pairs @ time, per pass (for error messages)
   auto log_pass = [&](const Pass& ps, int64_t pairs) {
@@ -1318,6 +1539,9 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
                          cudaMemcpyHostToDevice, st));
     CU(cudaMemsetAsync(d_cnt, 0, kCounterBytes, st));
     CU(record(ctx, ctx->ev[4], st));
+    if (n_probed) {
+      if (const int prc = queue_probe(probe, probe_off, n_probed)) return prc;
+    }
     for (const BandRun& r : runs) {
       const tsu::AlignArgs a = align_args(r.ps, all_pairs ? nullptr : P<int32_t>(ctx->b_order) + r.off, r.n, r.slot,
                                           P<int32_t>(ctx->b_retry) + r.off);
@@ -1330,11 +1554,57 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     return TSU_OK;
   });
   if (rc) return rc;
-  ctx->timing.kernel_launches += 3 + (int64_t)runs.size();
+  ctx->timing.kernel_launches += 3 + (int64_t)runs.size() + (n_probed ? 1 : 0);
   CU(wait_stream(ctx, st));
+  if (n_probed) {
+    if ((rc = bounded_runs(probed, probe_off))) return rc;
+  }
+  // Pairs that outgrew an unbounded shared ring get a bound, and a second
+  // start with it: 20,000 pairs of 800 - 1,000 bp at 10 % took 13.2 ms through
+  // the ladder.  (Few of them: the ladder's 16 warps are as good.)
+  if (can_bound) {
+    std::vector<int32_t> again;
+    const size_t first_runs = runs.size();
+    for (size_t j = 0; j < first_runs; ++j) {
+      BandRun& r = runs[j];
+      const unsigned int c = *reinterpret_cast<const unsigned int*>(h_cnt + 64 + 8 * r.slot + 4);
+      if (!c || r.ps.g.bounded || r.ps.g.mode != tsu::kModeShared) continue;
+      if ((rc = host_grow(ctx, ctx->h_list, sizeof(int32_t) * c))) return rc;
+      CU(cudaMemcpyAsync(ctx->h_list.p, P<int32_t>(ctx->b_retry) + r.off, sizeof(int32_t) * c, cudaMemcpyDeviceToHost, st));
+      CU(wait_stream(ctx, st));
+      const int32_t* l = static_cast<const int32_t*>(ctx->h_list.p);
+      const size_t before = again.size();
+      for (unsigned int i = 0; i < c; ++i)
+        if (std::max(h_plen[l[i]], h_tlen[l[i]]) <= tsu::kPackedMaxLen && std::min(h_plen[l[i]], h_tlen[l[i]]) > 0)
+          again.push_back(l[i]);
+      if (again.size() - before == c && c > (unsigned)ctx->sms)
+        r.rebound = true;  // all of them
+      else
+        again.resize(before);
+    }
+    ProbePlan p;
+    if ((rc = probe_plan(again, &p))) return rc;
+    if (p.blocks) {
+      std::stable_sort(again.begin(), again.end(), [&](int32_t u, int32_t v) {
+        return (int64_t)h_plen[u] + h_tlen[u] > (int64_t)h_plen[v] + h_tlen[v];
+      });
+      if ((rc = host_grow(ctx, ctx->h_list, sizeof(int32_t) * again.size()))) return rc;
+      memcpy(ctx->h_list.p, again.data(), sizeof(int32_t) * again.size());
+      CU(cudaMemcpyAsync(P<int32_t>(ctx->b_order) + n, ctx->h_list.p, sizeof(int32_t) * again.size(),
+                         cudaMemcpyHostToDevice, st));
+      CU(cudaMemsetAsync(d_cnt + kProbeQueue, 0, 8, st));
+      if ((rc = queue_probe(p, n, (int64_t)again.size()))) return rc;
+      ctx->timing.kernel_launches++;
+      ctx->timing.retried_pairs += (int64_t)again.size();
+      CU(wait_stream(ctx, st));
+      if ((rc = bounded_runs(again, n))) return rc;
+    } else {
+      for (BandRun& r : runs) r.rebound = false;
+    }
+  }
   std::vector<unsigned int> first_retry(runs.size());
   for (const BandRun& r : runs) {
-    first_retry[(size_t)r.slot] = *reinterpret_cast<const unsigned int*>(h_cnt + 64 + 8 * r.slot + 4);
+    first_retry[(size_t)r.slot] = r.rebound ? 0u : *reinterpret_cast<const unsigned int*>(h_cnt + 64 + 8 * r.slot + 4);
     log_pass(r.ps, r.n);
     char t[48];
     snprintf(t, sizeof t, "@%.1fms", ev_ms(ctx->bev[2 * r.slot], ctx->bev[2 * r.slot + 1]));
@@ -1621,7 +1891,7 @@ int predict_bytes(tsu_ctx* ctx, const BatchShape& sh, uint32_t flags, double hin
       len_sum += (int64_t)pl[i] + tl[i];
     }
     size_t f = 2 * r(16 * (size_t)nc) + r(8 * (size_t)ci.total_words) + r(2 * (size_t)nc) + r(8 * (size_t)nc) +
-               3 * r(4 * (size_t)nc) + r(64);
+               2 * r(4 * (size_t)nc) + 2 * r(8 * (size_t)nc) + r(64 + 8 * kRunSlots);
     size_t tmp = scan_tmp(2 * nc);
     if (want_cigar) {
       const int64_t arena = std::max<int64_t>(tsu::arena_runs(ctx->rp, nc, ci.max_m, ci.max_n, hint), 1024);
@@ -1757,6 +2027,8 @@ int create(const Spec& spec, const tsu_config* cfg, bool single_stream, tsu_ctx*
     cudaStreamCreateWithFlags(&ctx->h2d_stream, cudaStreamNonBlocking);
     cudaStreamCreateWithFlags(&ctx->d2h_stream, cudaStreamNonBlocking);
   }
+  for (auto& sd : ctx->side) cudaStreamCreateWithFlags(&sd, cudaStreamNonBlocking);
+  cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming);
   ctx->pool = device_pool(ctx->device);
   for (auto& ev : ctx->bev) cudaEventCreate(&ev);
   {
@@ -1764,7 +2036,7 @@ int create(const Spec& spec, const tsu_config* cfg, bool single_stream, tsu_ctx*
     const char* gv = getenv("TSU_GRAPH");
     ctx->use_graph = !(gv && gv[0] == '0');
   }
-  if (!ctx->pool || host_grow(ctx, ctx->h_scalars, 256) != TSU_OK) {
+  if (!ctx->pool || host_grow(ctx, ctx->h_scalars, 512) != TSU_OK) {
     tsu_destroy(ctx);
     return TSU_EDEVICE;
   }
@@ -1883,11 +2155,14 @@ int tsu_destroy(tsu_ctx* ctx) {
   if (ctx->wait_ev) cudaEventDestroy(ctx->wait_ev);
   for (auto& ev : ctx->bev) cudaEventDestroy(ev);
   if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
-  for (HostBuf* hb : {&ctx->h_scalars, &ctx->h_list, &ctx->h_status, &ctx->h_bidir})
+  for (HostBuf* hb : {&ctx->h_scalars, &ctx->h_list, &ctx->h_status, &ctx->h_bidir, &ctx->h_bound})
     if (hb->p) cudaFreeHost(hb->p);
   for (void* p : ctx->h_retired) cudaFreeHost(p);
   if (ctx->h2d_stream && ctx->h2d_stream != ctx->stream) cudaStreamDestroy(ctx->h2d_stream);
   if (ctx->d2h_stream && ctx->d2h_stream != ctx->stream) cudaStreamDestroy(ctx->d2h_stream);
+  for (auto& sd : ctx->side)
+    if (sd) cudaStreamDestroy(sd);
+  if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
   return TSU_OK;

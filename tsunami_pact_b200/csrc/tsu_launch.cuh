@@ -20,17 +20,36 @@ namespace tsu {
 // The dual gap-affine kernels (tsu_dual.cu) and the gap-linear ones
 // (tsu_linear.cu).
 // lowmem: the low-memory variant of the CIGAR kernel (cigar is then
-// ignored).
+// ignored); bounded: the shared-ring variant of pairs with score bounds.
 cudaError_t align_occupancy_dual(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ,
-                                 bool lowmem);
+                                 bool lowmem, bool bounded);
 void launch_align_dual(bool cigar, int mode, int gw, int blocks, int threads, size_t smem, cudaStream_t st,
-                       const AlignArgs& a, bool lowmem);
+                       const AlignArgs& a, bool lowmem, bool bounded);
 cudaError_t align_occupancy_linear(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ,
-                                   bool lowmem);
+                                   bool lowmem, bool bounded);
 void launch_align_linear(bool cigar, int mode, int gw, int blocks, int threads, size_t smem, cudaStream_t st,
-                         const AlignArgs& a, bool lowmem);
+                         const AlignArgs& a, bool lowmem, bool bounded);
+
+// The bound probe of each model (probe_kernel).
+cudaError_t probe_occupancy_dual(int threads, size_t smem, int optin, int* occ);
+void launch_probe_dual(int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a);
+cudaError_t probe_occupancy_linear(int threads, size_t smem, int optin, int* occ);
+void launch_probe_linear(int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a);
 
 namespace launch_detail {
+
+template <int kModel>
+cudaError_t probe_occupancy(int threads, size_t smem, int optin, int* occ) {
+  const cudaError_t e =
+      cudaFuncSetAttribute(probe_kernel<kModel>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+  if (e != cudaSuccess) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, probe_kernel<kModel>, threads, smem);
+}
+
+template <int kModel>
+void probe(int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {
+  probe_kernel<kModel><<<blocks, threads, smem, st>>>(a);
+}
 
 template <bool kCigar, int kMode, int GW, int kModel>
 cudaError_t occ_one(int threads, size_t smem, int optin, int* occ) {
@@ -56,13 +75,19 @@ cudaError_t occ_gw(int gw, int threads, size_t smem, int optin, int* occ) {
     case 4: return occ_one<kCigar, kMode, 4, kModel>(threads, smem, optin, occ);
     case 8: return occ_one<kCigar, kMode, 8, kModel>(threads, smem, optin, occ);
     case 16: return occ_one<kCigar, kMode, 16, kModel>(threads, smem, optin, occ);
-    case 32: return occ_one<kCigar, kMode, 32, kModel>(threads, smem, optin, occ);
+    case 32:
+      if constexpr (!(kModel & kBoundFlag)) return occ_one<kCigar, kMode, 32, kModel>(threads, smem, optin, occ);
+      return cudaErrorInvalidValue;
     default: return cudaErrorInvalidValue;
   }
 }
 
 template <int kModel>
-cudaError_t occupancy(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ, bool lowmem) {
+cudaError_t occupancy(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ, bool lowmem,
+                      bool bounded) {
+  if (bounded)
+    return cigar ? occ_gw<true, kModeShared, kModel | kBoundFlag>(gw, threads, smem, optin, occ)
+                 : occ_gw<false, kModeShared, kModel | kBoundFlag>(gw, threads, smem, optin, occ);
   if (lowmem)
     return mode == kModeShared ? occ_gw<true, kModeShared, kModel | kLowMemFlag>(gw, threads, smem, optin, occ)
                                : occ_gw<true, kModeGlobal, kModel | kLowMemFlag>(gw, threads, smem, optin, occ);
@@ -81,15 +106,22 @@ void launch_gw(int gw, int blocks, int threads, size_t smem, cudaStream_t st, co
     case 4: align_kernel<kCigar, kMode, 4, kModel><<<blocks, threads, smem, st>>>(a); break;
     case 8: align_kernel<kCigar, kMode, 8, kModel><<<blocks, threads, smem, st>>>(a); break;
     case 16: align_kernel<kCigar, kMode, 16, kModel><<<blocks, threads, smem, st>>>(a); break;
-    case 32: align_kernel<kCigar, kMode, 32, kModel><<<blocks, threads, smem, st>>>(a); break;
+    case 32:
+      if constexpr (!(kModel & kBoundFlag)) align_kernel<kCigar, kMode, 32, kModel><<<blocks, threads, smem, st>>>(a);
+      break;
     default: break;
   }
 }
 
 template <int kModel>
 void launch(bool cigar, int mode, int gw, int blocks, int threads, size_t smem, cudaStream_t st, const AlignArgs& a,
-            bool lowmem) {
-  if (lowmem) {
+            bool lowmem, bool bounded) {
+  if (bounded) {
+    if (cigar)
+      launch_gw<true, kModeShared, kModel | kBoundFlag>(gw, blocks, threads, smem, st, a);
+    else
+      launch_gw<false, kModeShared, kModel | kBoundFlag>(gw, blocks, threads, smem, st, a);
+  } else if (lowmem) {
     if (mode == kModeShared)
       launch_gw<true, kModeShared, kModel | kLowMemFlag>(gw, blocks, threads, smem, st, a);
     else

@@ -7,13 +7,21 @@
 namespace tsu {
 
 cudaError_t align_occupancy_linear(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ,
-                                   bool lowmem) {
-  return launch_detail::occupancy<kModelLinear>(cigar, mode, gw, threads, smem, optin, occ, lowmem);
+                                   bool lowmem, bool bounded) {
+  return launch_detail::occupancy<kModelLinear>(cigar, mode, gw, threads, smem, optin, occ, lowmem, bounded);
 }
 
 void launch_align_linear(bool cigar, int mode, int gw, int blocks, int threads, size_t smem, cudaStream_t st,
-                         const AlignArgs& a, bool lowmem) {
-  launch_detail::launch<kModelLinear>(cigar, mode, gw, blocks, threads, smem, st, a, lowmem);
+                         const AlignArgs& a, bool lowmem, bool bounded) {
+  launch_detail::launch<kModelLinear>(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded);
+}
+
+cudaError_t probe_occupancy_linear(int threads, size_t smem, int optin, int* occ) {
+  return launch_detail::probe_occupancy<kModelLinear>(threads, smem, optin, occ);
+}
+
+void launch_probe_linear(int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {
+  launch_detail::probe<kModelLinear>(blocks, threads, smem, st, a);
 }
 
 }  // namespace tsu

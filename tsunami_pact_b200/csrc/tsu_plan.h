@@ -36,6 +36,7 @@ struct PassGeom {
   int ckpt_k = 0;          // low-memory mode: checkpoint interval (0: off)
   int ckpt_cap = 0;        // checkpoints per group
   int64_t ckpt_bytes = 0;  // bytes per checkpoint
+  bool bounded = false;    // pairs with score bounds (plan_bounded)
 };
 
 constexpr int kSharedW1 = 384;         // shared-mode ring width for one warp per pair (diagonals)
@@ -43,11 +44,11 @@ constexpr int kSharedSeqWords1 = 544;  // staging area for one warp per pair (ui
 constexpr int kSharedSeqWordsN = 4096; // staging area for a group of warps
 constexpr int kSharedMaxLen = 32000;   // int16 ring limit of the low-memory kernels
 // A launch of the packed kernel takes pairs up to the end of their length
-// band; the few beyond kPackedMaxLen are handed back one by one.
-constexpr int kPackedPlanLen = 16383;
-// widest int16 ring: a negative (invalid) I value grows by one per diagonal
-// of the ring's width and must stay negative (the kernel's store clamp)
-constexpr int kSharedMaxW = 16368;
+// band; the few beyond kPackedPlainLen are handed back one by one.
+constexpr int kPackedBandLen = 16383;
+// widest shared ring (kPackedMaxW; the low-memory kernels' int16 ring holds
+// 16,368: a negative I value grows by one per diagonal and must stay negative)
+constexpr int kSharedMaxW = kPackedMaxW;
 constexpr int kSmemPerSM = 228 * 1024; // B200 shared memory per SM (bytes)
 
 // Reduced-unit score expected at edit rate `hint` for a pair of length L.
@@ -102,7 +103,7 @@ inline PassGeom plan_geometry(const Pen& pen, int32_t max_m, int32_t max_n, int 
   p.gw = gw;
   p.cta_threads = cta_threads_for(gw);
   p.groups_per_cta = p.cta_threads / (32 * gw);
-  const bool fits = lowmem ? maxlen <= kSharedMaxLen : (maxlen <= kPackedPlanLen && pen.rm <= kPackedMaxDepth);
+  const bool fits = lowmem ? maxlen <= kSharedMaxLen : (maxlen <= kPackedBandLen && pen.rm <= kPackedMaxDepth);
   p.mode = (mode == kModeShared && fits) ? kModeShared : kModeGlobal;
   if (p.mode == kModeShared) {
     const int64_t seqw = 2 * packed_words(max_m) + 2 * packed_words(max_n);
@@ -164,7 +165,7 @@ inline PassGeom plan_geometry(const Pen& pen, int32_t max_m, int32_t max_n, int 
 inline PassChoice next_pass(PassChoice prev, const Pen& pen, int32_t max_m, int32_t max_n, int smem_optin,
                             int global_gw = 16) {
   const int64_t need_w = (int64_t)max_m + max_n + 3;
-  if (prev.mode == kModeShared && std::max(max_m, max_n) <= kPackedMaxLen && pen.rm <= kPackedMaxDepth) {
+  if (prev.mode == kModeShared && std::max(max_m, max_n) <= kPackedPlainLen && pen.rm <= kPackedMaxDepth) {
     const int64_t seqw =
         std::min<int64_t>(2 * packed_words(max_m) + 2 * packed_words(max_n), kSharedSeqWordsN);
     static const int kGW[] = {2, 4, 8, 16};
@@ -189,7 +190,7 @@ inline PassChoice fit_start(PassChoice pc, const Pen& pen, int32_t max_m, int32_
   const int64_t w =
       std::min<int64_t>((int64_t)max_m + max_n + 3, 2 * hint_score(pen, maxlen, hint) / pen.min_ge() + 3);
   if (pc.mode != kModeShared) return {kModeGlobal, w > 16384 ? 32 : pc.gw};
-  if (maxlen > kPackedMaxLen || pen.rm > kPackedMaxDepth) return {kModeGlobal, w > 16384 ? 32 : std::max(8, pc.gw)};
+  if (maxlen > kPackedPlainLen || pen.rm > kPackedMaxDepth) return {kModeGlobal, w > 16384 ? 32 : std::max(8, pc.gw)};
   const int64_t seqw = 2 * packed_words(max_m) + 2 * packed_words(max_n);
   static const int kGW[] = {1, 2, 4, 8, 16};
   for (int gw : kGW) {
@@ -219,7 +220,7 @@ inline int length_band(int32_t L) {
 // compiled one), adjusted for lengths beyond the int16 shared ring.
 inline PassChoice band_start_in(const PassChoice* table, int band, int32_t maxlen) {
   PassChoice r = table[band < 0 ? 0 : (band >= kBands ? kBands - 1 : band)];
-  if (r.mode == kModeShared && maxlen > kPackedPlanLen) r = {kModeGlobal, r.gw >= 8 ? r.gw : 8};
+  if (r.mode == kModeShared && maxlen > kPackedBandLen) r = {kModeGlobal, r.gw >= 8 ? r.gw : 8};
   return r;
 }
 inline const PassChoice* band_start_table(bool dual = false) {
@@ -242,6 +243,111 @@ inline int64_t arena_runs(const Pen& pen, int64_t n, int32_t max_m, int32_t max_
   const int64_t maxlen = std::max(max_m, max_n);
   const int64_t per_pair = 2 * hint_score(pen, maxlen, hint) / pen.min_pen() + 1;
   return std::max<int64_t>(n * (std::min<int64_t>(per_pair, (int64_t)max_m + max_n + 1) + 3), 1024);
+}
+
+// ---- passes of pairs whose score bound is known ----------------------------
+
+// Whether a pair of a large batch is worth a bound probe: its full wavefronts
+// are expected to reach 420 diagonals at 4 % edits (gap-affine 4/6/2: from
+// 1.3 kbp), or one warp's unbounded ring takes over 14 KB (two gap pieces,
+// deep penalties), so that an SM holds few of them.  Below that a pair fits
+// one warp's ring without a bound and the probe, two words per lane and score,
+// costs about what it saves.
+constexpr int kBoundMinWidth = 420;
+constexpr int kBoundMinRing = 14 << 10;
+inline bool wants_bound(const Pen& pen, int32_t m, int32_t n) {
+  const int64_t L = std::max(m, n);
+  if (L > kPackedMaxLen || std::min(m, n) <= 0) return false;
+  const int64_t ring = (int64_t)(pen.slots() + 1) * 2 * std::min<int64_t>((int64_t)m + n + 3, kSharedW1);
+  return 2 * hint_score(pen, L, 0.04) / pen.min_ge() >= kBoundMinWidth || ring > kBoundMinRing;
+}
+// With no more such pairs than SMs each has an SM to itself, and a probe (0.35
+// us per score on one warp) adds what the narrower search saves (148 x 8 kbp
+// at 10 %: 3.1 ms either way; one 8 kbp pair at 1 %: 0.56 ms without, 0.60
+// with): only pairs that may not fit the widest shared ring at all are probed.
+constexpr int kBoundFewLen = 8192;
+
+// What a pair of score bound ub needs: diagonals of the ring's window,
+// 32-bit sequence words, and 32-bit history words (each side of the band grows
+// to its crossing and shrinks again, one diagonal per gap extension; three
+// words of rounding per score).
+struct BoundNeed {
+  int width = 0, words = 0;
+  int64_t hist = 0;
+};
+inline BoundNeed bound_need(const Pen& pen, int32_t m, int32_t n, int32_t ub) {
+  BoundNeed b;
+  int lo, hi;
+  bound_reach(pen, m, n, ub, &lo, &hi);
+  b.width = hi - lo + 1;
+  b.words = (int)(2 * packed_words(m) + 2 * packed_words(n));
+  const int64_t h = hi, l = -(int64_t)lo, e = pen.min_ge();
+  const int64_t cells = std::min<int64_t>(e * (h * h + l * l) + (int64_t)ub + 1, (int64_t)(b.width + 1) * ((int64_t)ub + 1));
+  b.hist = cells / (pen.dual() ? 4 : 8) + 3 * ((int64_t)ub + 1) + 64;
+  return b;
+}
+
+// Geometry of a launch of bounded pairs: bytes of shared memory per group
+// (bounded_bytes of the pair that needs most at these warps), history and
+// step table as their bounds say.
+inline PassGeom plan_bounded(int bytes, int32_t max_ub, int64_t hist, int gw, bool want_cigar) {
+  PassGeom p;
+  p.mode = kModeShared;
+  p.bounded = true;
+  p.gw = gw;
+  p.cta_threads = cta_threads_for(gw);
+  p.groups_per_cta = p.cta_threads / (32 * gw);
+  p.min_blocks = min_blocks_for(kModeShared, gw);
+  p.group_smem = bytes;
+  if (want_cigar) {
+    p.table_cap = max_ub + 2;
+    p.hist_cap = std::min<int64_t>(hist, INT32_MAX - 65536);
+  }
+  return p;
+}
+
+// Classes of bounded pairs, one launch each: by how many of their kind an SM's
+// shared memory holds (1, 2-3, 4-7, ... 64 and more: class 0 to 6).  Pairs of
+// one class run at its widest member's ring, which costs none of them a place
+// beyond the class; classes by width alone cut 10 kbp pairs at 4,096 diagonals
+// and ran the last 13 of 309 as a wave of their own.
+constexpr int kBoundClasses = 7;
+inline int bound_class(int pairs_per_sm) {
+  int c = 0;
+  while (c < kBoundClasses - 1 && pairs_per_sm >= 2 << c) ++c;
+  return c;
+}
+
+// Warps per pair of a bounded launch of n pairs: the fewest that keep 16 warps
+// on an SM with the pairs its shared memory holds (a step costs every warp of
+// a group the same bookkeeping, so fewer warps do less work: 4,000 x 2 kbp at
+// 5 % took 1.7 ms on 2 warps, 2.3 on 4, 2.7 on 8), and as many as fill 8 per
+// SM when there are few pairs (148 x 1 kbp: 0.21 ms on 1 warp, 0.15 on 4 to
+// 16; 600: 0.19 on 2, 0.26 on 4).  0: the ring does not fit a block.
+inline int bounded_warps(int bytes, int64_t n, int sms, int smem_optin, int* pairs_per_sm = nullptr) {
+  int best = 0;
+  for (int gw = 1; gw <= 16; gw *= 2) {
+    const int gpc = cta_threads_for(gw) / (32 * gw);
+    const int64_t block = (int64_t)gpc * bytes;
+    if (block > smem_optin) continue;
+    const int64_t pairs = kSmemPerSM / (block + 1024) * gpc;
+    best = gw;
+    if (pairs_per_sm) *pairs_per_sm = (int)pairs;
+    if (pairs * gw >= 16 && n * gw * 2 > (int64_t)sms * 8) break;
+  }
+  return best;
+}
+
+// Warps per pair of an unbounded shared-ring launch of n pairs: 16 when each
+// pair can have an SM to itself (one pair of 1 kbp: 0.21 ms on 1 warp, 0.14 on
+// 16; 148 of 8 kbp at 10 %: 3.1 ms, and 5.4 from 8 warps, whose ring they
+// outgrow), else those of the rung, doubled while the launch leaves an SM
+// fewer than 8 warps (600 pairs of 1 kbp: 0.22 ms on 1, 0.19 on 2, 0.26 on 4).
+inline PassChoice fill_warps(PassChoice pc, int64_t n, int sms) {
+  if (pc.mode != kModeShared) return pc;
+  if (n <= sms) pc.gw = std::max(pc.gw, 16);
+  while (pc.gw < 16 && n * pc.gw * 2 <= (int64_t)sms * 8) pc.gw *= 2;
+  return pc;
 }
 
 }  // namespace tsu
