@@ -2,8 +2,9 @@
 // from its bounds, through the CPU warp emulator (test infrastructure;
 // compiled by tests/test_bound_probe.py with AddressSanitizer).
 //
-// Input (stdin):  x o e o2 e2 cigar gw loose N, then N records "m n\n<pattern>\n<text>\n"
-//   (o2 < 0: one gap piece; o < 0: gap-linear); loose: added to each bound
+// Input (stdin):  x o e o2 e2 cigar gw loose wide N, then N records "m n\n<pattern>\n<text>\n"
+//   (o2 < 0: one gap piece; o < 0: gap-linear); loose: added to each bound;
+//   wide: 0, or the wide probe and kernel with ring cells of 2 or 4 bytes
 // Output: per pair "bound<TAB>score<TAB>ops" (score -1: no bound, not aligned).
 #include "warp_emu.h"
 // clang-format off
@@ -30,10 +31,18 @@ static void align(int gw, int threads, size_t smem, const tsu::AlignArgs& a) {
   }
 }
 
+template <int kM>
+static void align_wide(bool cigar, int cell, size_t smem, const tsu::AlignArgs& a) {
+  if (cell == 2)
+    emu::launch(1, 512, smem, [&] { cigar ? tsu::wide_kernel<true, kM, uint16_t>(a) : tsu::wide_kernel<false, kM, uint16_t>(a); });
+  else
+    emu::launch(1, 512, smem, [&] { cigar ? tsu::wide_kernel<true, kM, uint32_t>(a) : tsu::wide_kernel<false, kM, uint32_t>(a); });
+}
+
 int main() {
-  int X, O, E, O2, E2, cigar, gw, loose;
+  int X, O, E, O2, E2, cigar, gw, loose, wide;
   int64_t N;
-  if (!(std::cin >> X >> O >> E >> O2 >> E2 >> cigar >> gw >> loose >> N)) return 2;
+  if (!(std::cin >> X >> O >> E >> O2 >> E2 >> cigar >> gw >> loose >> wide >> N)) return 2;
   std::vector<std::string> pats(N), txts(N);
   for (int64_t i = 0; i < N; ++i) {
     int m, n;
@@ -79,9 +88,15 @@ int main() {
   for (int64_t i = 0; i < N; ++i) bound[i] = tsu::kNoBound;
   tsu::ProbeArgs b{sv, pk, order, N, rp, seq_cap, bound, queue};
   const int threads = 64;
-  const size_t psmem = 2 * (size_t)tsu::probe_smem_bytes(rp, seq_cap);
+  const size_t psmem = 2 * (size_t)(wide ? tsu::wide_probe_smem_bytes(rp) : tsu::probe_smem_bytes(rp, seq_cap));
   emu::launch(1, threads, psmem, [&] {
-    if (rp.linear())
+    if (wide && rp.linear())
+      tsu::wide_probe_kernel<tsu::kModelLinear>(b);
+    else if (wide && rp.dual())
+      tsu::wide_probe_kernel<tsu::kModelDual>(b);
+    else if (wide)
+      tsu::wide_probe_kernel<tsu::kModelAffine>(b);
+    else if (rp.linear())
       tsu::probe_kernel<tsu::kModelLinear>(b);
     else if (rp.dual())
       tsu::probe_kernel<tsu::kModelDual>(b);
@@ -89,18 +104,20 @@ int main() {
       tsu::probe_kernel<tsu::kModelAffine>(b);
   });
   std::vector<int32_t> found(bound, bound + N), todo;
-  int bytes = 0;
+  int bytes = 0, width = 0;
   int32_t ub = 0;
   int64_t hist = 0, runs = 0;
   for (int64_t i = 0; i < N; ++i) {
     if (bound[i] == tsu::kNoBound) continue;
     bound[i] += loose;
     const tsu::BoundNeed need = tsu::bound_need(rp, pl[i], tl[i], bound[i]);
+    width = std::max(width, need.width);
     bytes = std::max(bytes, tsu::bounded_bytes(rp, need.width, need.words, gw)), ub = std::max(ub, bound[i]), hist = std::max(hist, need.hist);
     runs += 2 * (int64_t)bound[i] / rp.min_pen() + 4;
     todo.push_back((int32_t)i);
   }
-  const tsu::PassGeom geo = tsu::plan_bounded(bytes, ub, hist, gw, cigar != 0);
+  tsu::PassGeom geo = wide ? tsu::plan_wide(rp, wide == 2 ? 0 : tsu::kWide16MaxLen + 1, width, ub, hist, cigar != 0)
+                           : tsu::plan_bounded(bytes, ub, hist, gw, cigar != 0);
   const int groups = geo.groups_per_cta;
   int32_t *score = block<int32_t>(N), *status = block<int32_t>(N), *clen = block<int32_t>(N), *retry = block<int32_t>(N);
   int64_t* cpos = block<int64_t>(N);
@@ -116,8 +133,15 @@ int main() {
   a.arena = block<uint32_t>(runs), a.arena_cursor = cnt, a.arena_cap = runs;
   a.cig_pos = cpos, a.cig_len = clen, a.queue = queue, a.retry = retry, a.retry_count = queue + 1, a.work = cnt + 1;
   a.bound = bound;
+  a.wide_cell = geo.wide_cell, a.ring_global = block<int32_t>(geo.ring_ints), a.ring_stride = geo.ring_ints;
   const size_t smem = (size_t)groups * geo.group_smem;
-  if (rp.linear())
+  if (wide && rp.linear())
+    align_wide<tsu::kModelLinear>(cigar, wide, smem, a);
+  else if (wide && rp.dual())
+    align_wide<tsu::kModelDual>(cigar, wide, smem, a);
+  else if (wide)
+    align_wide<tsu::kModelAffine>(cigar, wide, smem, a);
+  else if (rp.linear())
     cigar ? align<tsu::kModelLinear, true>(gw, geo.cta_threads, smem, a) : align<tsu::kModelLinear, false>(gw, geo.cta_threads, smem, a);
   else if (rp.dual())
     cigar ? align<tsu::kModelDual, true>(gw, geo.cta_threads, smem, a) : align<tsu::kModelDual, false>(gw, geo.cta_threads, smem, a);

@@ -27,9 +27,9 @@ def emu_bound():
     return EXE
 
 
-def _run(exe, pairs, pen, cigar=True, gw=1, loose=0):
+def _run(exe, pairs, pen, cigar=True, gw=1, loose=0, wide=0):
     o2, e2 = (pen[3], pen[4]) if len(pen) == 5 else (-1, 0)
-    hdr = f"{pen[0]} {pen[1]} {pen[2]} {o2} {e2} {int(cigar)} {gw} {loose} {len(pairs)}\n"
+    hdr = f"{pen[0]} {pen[1]} {pen[2]} {o2} {e2} {int(cigar)} {gw} {loose} {wide} {len(pairs)}\n"
     body = b"".join(f"{len(p)} {len(t)}\n".encode() + p + b"\n" + t + b"\n" for p, t in pairs)
     env = dict(os.environ, ASAN_OPTIONS="detect_leaks=0:abort_on_error=1", UBSAN_OPTIONS="halt_on_error=1")
     r = subprocess.run([exe], input=hdr.encode() + body, capture_output=True, env=env, timeout=600)
@@ -54,15 +54,44 @@ def _pairs(rng):
 
 
 @pytest.mark.parametrize("pen", [(4, 6, 2), (5, 11, 3), (4, 6, 2, 24, 1), (1, -1, 1), (3, -1, 1)])
-@pytest.mark.parametrize("gw,loose,cigar", [(1, 0, True), (1, 7, True), (4, 0, True), (1, 0, False)])
-def test_bounded_equals_oracle(emu_bound, oracle, pen, gw, loose, cigar):
+@pytest.mark.parametrize("gw,loose,cigar,wide", [(1, 0, True, 0), (1, 7, True, 0), (4, 0, True, 0), (1, 0, False, 0),
+                                                 (16, 0, True, 2), (16, 3, True, 4)])
+def test_bounded_equals_oracle(emu_bound, oracle, pen, gw, loose, cigar, wide):
+    """wide: the kernels of sides beyond the 16-bit ring (tsu_wide.cuh)."""
     pairs = _pairs(random.Random(sum(pen) + gw + loose))
-    for (p, t), (ub, s, ops) in zip(pairs, _run(emu_bound, pairs, pen, cigar, gw, loose)):
+    if wide:
+        pairs = pairs[:2] + pairs[5:]
+    for (p, t), (ub, s, ops) in zip(pairs, _run(emu_bound, pairs, pen, cigar, gw, loose, wide)):
         if b"N" in p:
             assert ub == "none"
             continue
         es, eops = _align(oracle, p, t, pen)
         assert ub == "none" or (int(ub) >= es and int(s) == es and ops == (eops if cigar else "")), (p, t, pen, ub, s, es)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("low_memory", [False, True])
+def test_long_pairs_gpu(oracle, low_memory):
+    """Pairs past the 16-bit shared ring: 20-34 kbp, a text of more than
+    65,532 bases, a band wider than a block's ring, a pair with bytes outside
+    ACGT; with and without low-memory mode (whose short pairs get bounds too)."""
+    import tsunami_pact_b200 as T
+
+    rng = np.random.default_rng(8)
+    lens = np.array([20464, 30000, 34000, 66000, 66000, 20400, 21000, 300, 255], np.int32)
+    rates = np.array([0.02, 0.1, 0.15, 0.01, 0.004, 0.3, 0.02, 0.1, 0.1])
+    pbuf, poff, plen, tbuf, toff, tlen = T.gen_batch(9, lens, rates)
+    pats = [bytes(pbuf[poff[i]:poff[i] + plen[i]]) for i in range(len(lens))]
+    txts = [bytes(tbuf[toff[i]:toff[i] + tlen[i]]) for i in range(len(lens))]
+    pats[1], txts[4] = pats[1][700:], txts[4][: 66000 - 300]
+    pats[6] = pats[6][:5000] + b"N" + pats[6][5001:]
+    osc, oops = oracle.align_batch(pats, txts, 4, 6, 2)
+    with T.Aligner(4, 6, 2) as al:
+        if low_memory:
+            al.set_low_memory(-1)
+        scores, ops = al.align(pats, txts)
+        assert list(scores) == list(osc) and ops == oops
+        assert list(al.align(pats, txts, cigar=False)[0]) == list(osc)
 
 
 @pytest.mark.gpu

@@ -65,6 +65,7 @@ __device__ __forceinline__ void group_sync(int gid) {
 }  // namespace tsu
 
 #include "tsu_packed.cuh"
+#include "tsu_wide.cuh"
 
 namespace tsu {
 
@@ -850,6 +851,27 @@ __global__ void __launch_bounds__(kProbeThreads, 5) probe_kernel(ProbeArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
 #endif
   probe_packed<kModel>(a, smem_raw);
+}
+
+template <int kModel>
+__global__ void __launch_bounds__(kProbeThreads, 4) wide_probe_kernel(ProbeArgs a) {
+#ifdef TSU_WARP_EMU
+  unsigned char* smem_raw = emu::dyn_smem();
+#else
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+#endif
+  probe_wide<kModel>(a, smem_raw);
+}
+
+constexpr int kWideThreads = 512;
+template <bool kCigar, int kModel, typename ST>
+__global__ void __launch_bounds__(kWideThreads, 1) wide_kernel(AlignArgs a) {
+#ifdef TSU_WARP_EMU
+  unsigned char* smem_raw = emu::dyn_smem();
+#else
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+#endif
+  align_wide<kCigar, kModel, ST>(a, smem_raw);
 }
 
 }  // namespace tsu

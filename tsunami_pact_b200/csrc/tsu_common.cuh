@@ -174,6 +174,7 @@ struct AlignArgs {
   // that a path within the bound can use (end-to-end pairs only)
   const int32_t* bound;
   int group_bytes;  // bounded launches: shared memory per group
+  int wide_cell;    // bounded launches of the wide kernel: bytes of a ring cell (2, 4); 0: the shared ring
 };
 
 // The bound probe (tsu_packed.cuh).
@@ -263,6 +264,16 @@ __host__ __device__ inline int group_smem_bytes(const Pen& p, int ring_w, int mo
     b = ((b + 15) & ~15) + 16 + seq_cap * 4;
   }
   return (b + 15) & ~15;
+}
+
+// The wide kernel (tsu_wide.cuh): longest text of its 16-bit rows, bytes of a
+// row of d diagonals (one more for whole pairs, 4 cells on each side, whole
+// 16-byte pieces), shared memory per block and per warp of its probe.
+constexpr int kWide16MaxLen = 65532;
+__host__ __device__ constexpr int wide_row_bytes(int d, int cell) { return ((d + 2 + 8) * cell + 15) & ~15; }
+__host__ __device__ inline int wide_smem_bytes(const Pen& p) { return packed_head_bytes(p, 16); }
+__host__ __device__ inline int wide_probe_smem_bytes(const Pen& p) {
+  return 16 * (p.rm + p.re + p.re2) + (p.slots() + 1) * wide_row_bytes(kProbeW, 4);
 }
 
 // Shared memory per warp of the bound probe.

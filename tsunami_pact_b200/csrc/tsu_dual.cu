@@ -15,12 +15,16 @@ void launch_align_dual(bool cigar, int mode, int gw, int blocks, int threads, si
   launch_detail::launch<kModelDual>(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded);
 }
 
-cudaError_t probe_occupancy_dual(int threads, size_t smem, int optin, int* occ) {
-  return launch_detail::probe_occupancy<kModelDual>(threads, smem, optin, occ);
+cudaError_t probe_occupancy_dual(bool wide, int threads, size_t smem, int optin, int* occ) {
+  return launch_detail::probe_occupancy<kModelDual>(wide, threads, smem, optin, occ);
 }
 
-void launch_probe_dual(int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {
-  launch_detail::probe<kModelDual>(blocks, threads, smem, st, a);
+void launch_probe_dual(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {
+  launch_detail::probe<kModelDual>(wide, blocks, threads, smem, st, a);
+}
+
+void launch_wide_dual(bool cigar, int blocks, size_t smem, cudaStream_t st, const AlignArgs& a) {
+  launch_detail::wide<kModelDual>(cigar, blocks, smem, st, a);
 }
 
 }  // namespace tsu

@@ -46,7 +46,7 @@ struct HostBuf {
 // Launches of a call before the retry ladders: length bands, then classes of
 // pairs with a score bound and the bands of pairs whose bound did not help,
 // the latter twice (pairs bounded at once, pairs bounded after a first pass).
-constexpr int kRunSlots = tsu::kBands + 2 * (tsu::kBoundClasses + tsu::kBands);
+constexpr int kRunSlots = tsu::kBands + 2 * (tsu::kBoundClasses + 2 + tsu::kBands);
 // Streams beside the context's own for the launches of bounded classes.
 constexpr int kSideStreams = 3;
 
@@ -317,6 +317,14 @@ cudaError_t align_occupancy(const tsu_ctx* ctx, bool cigar, int mode, int gw, in
 void launch_align(const tsu_ctx* ctx, bool cigar, int mode, int gw, int blocks, int threads, size_t smem,
                   cudaStream_t st, const tsu::AlignArgs& a) {
   const bool lowmem = cigar && a.ckpt_k > 0, bounded = a.bound != nullptr;
+  if (a.wide_cell) {
+    switch (ctx->rp.model()) {
+      case tsu::kModelDual: tsu::launch_wide_dual(cigar, blocks, smem, st, a); break;
+      case tsu::kModelLinear: tsu::launch_wide_linear(cigar, blocks, smem, st, a); break;
+      default: tsu::launch_detail::wide<tsu::kModelAffine>(cigar, blocks, smem, st, a); break;
+    }
+    return;
+  }
   switch (ctx->rp.model()) {
     case tsu::kModelDual: tsu::launch_align_dual(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded); break;
     case tsu::kModelLinear: tsu::launch_align_linear(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded); break;
@@ -326,29 +334,32 @@ void launch_align(const tsu_ctx* ctx, bool cigar, int mode, int gw, int blocks, 
   }
 }
 
-// Launch shape of the bound probe (tsu_packed.cuh) over n pairs.
-int plan_probe(tsu_ctx* ctx, int seq_cap, int64_t n, int* blocks, size_t* smem) {
+// Launch shape of the bound probe (tsu_packed.cuh; wide: tsu_wide.cuh) over n
+// pairs.
+int plan_probe(tsu_ctx* ctx, bool wide, int seq_cap, int64_t n, int* blocks, size_t* smem) {
   const int wpb = tsu::kProbeThreads / 32;
-  *smem = (size_t)wpb * tsu::probe_smem_bytes(ctx->rp, seq_cap);
+  *smem = (size_t)wpb * (wide ? tsu::wide_probe_smem_bytes(ctx->rp) : tsu::probe_smem_bytes(ctx->rp, seq_cap));
+  *blocks = 0;  // does not fit
+  if (*smem > (size_t)ctx->smem_optin) return TSU_OK;
   int occ = 0;
   cudaError_t e = cudaSuccess;
   switch (ctx->rp.model()) {
-    case tsu::kModelDual: e = tsu::probe_occupancy_dual(tsu::kProbeThreads, *smem, ctx->smem_optin, &occ); break;
-    case tsu::kModelLinear: e = tsu::probe_occupancy_linear(tsu::kProbeThreads, *smem, ctx->smem_optin, &occ); break;
+    case tsu::kModelDual: e = tsu::probe_occupancy_dual(wide, tsu::kProbeThreads, *smem, ctx->smem_optin, &occ); break;
+    case tsu::kModelLinear: e = tsu::probe_occupancy_linear(wide, tsu::kProbeThreads, *smem, ctx->smem_optin, &occ); break;
     default:
-      e = tsu::launch_detail::probe_occupancy<tsu::kModelAffine>(tsu::kProbeThreads, *smem, ctx->smem_optin, &occ);
+      e = tsu::launch_detail::probe_occupancy<tsu::kModelAffine>(wide, tsu::kProbeThreads, *smem, ctx->smem_optin, &occ);
       break;
   }
   if (e != cudaSuccess) return set_err(ctx, TSU_EDEVICE, "probe occupancy query failed (%d)", (int)e);
-  *blocks = (int)std::min<int64_t>((int64_t)ctx->sms * occ, (n + wpb - 1) / wpb);  // 0: does not fit
+  *blocks = (int)std::min<int64_t>((int64_t)ctx->sms * occ, (n + wpb - 1) / wpb);
   return TSU_OK;
 }
 
-void launch_probe(const tsu_ctx* ctx, int blocks, size_t smem, cudaStream_t st, const tsu::ProbeArgs& a) {
+void launch_probe(const tsu_ctx* ctx, bool wide, int blocks, size_t smem, cudaStream_t st, const tsu::ProbeArgs& a) {
   switch (ctx->rp.model()) {
-    case tsu::kModelDual: tsu::launch_probe_dual(blocks, tsu::kProbeThreads, smem, st, a); break;
-    case tsu::kModelLinear: tsu::launch_probe_linear(blocks, tsu::kProbeThreads, smem, st, a); break;
-    default: tsu::launch_detail::probe<tsu::kModelAffine>(blocks, tsu::kProbeThreads, smem, st, a); break;
+    case tsu::kModelDual: tsu::launch_probe_dual(wide, blocks, tsu::kProbeThreads, smem, st, a); break;
+    case tsu::kModelLinear: tsu::launch_probe_linear(wide, blocks, tsu::kProbeThreads, smem, st, a); break;
+    default: tsu::launch_detail::probe<tsu::kModelAffine>(wide, blocks, tsu::kProbeThreads, smem, st, a); break;
   }
 }
 
@@ -364,9 +375,10 @@ int plan_groups(tsu_ctx* ctx, const tsu::PassGeom& g, int64_t n_pairs, bool want
   Pass p;
   p.g = g;
   const int gpc = g.groups_per_cta;
-  int occ = 0;
-  cudaError_t e =
-      align_occupancy(ctx, want_cigar, g.mode, g.gw, g.cta_threads, (size_t)gpc * g.group_smem, ctx->smem_optin, &occ,
+  int occ = 1;
+  cudaError_t e = cudaSuccess;
+  if (!g.wide_cell)  // (the wide kernel: one block per SM)
+    e = align_occupancy(ctx, want_cigar, g.mode, g.gw, g.cta_threads, (size_t)gpc * g.group_smem, ctx->smem_optin, &occ,
                       g.ckpt_k > 0, g.bounded);
   if (e != cudaSuccess || occ < 1) return set_err(ctx, TSU_EDEVICE, "occupancy query failed (%d)", (int)e);
   int64_t warps = (int64_t)ctx->sms * occ * gpc;  // groups
@@ -863,6 +875,11 @@ int run_bidir_cigar(tsu_ctx* ctx, const tsu::SeqView& sv, int32_t* d_score, int3
     const size_t fixed = ctx->held() - ctx->b_scratch.cap;
     const size_t avail = ctx->budget > fixed ? ctx->budget - fixed : 0;
     warps = std::min<int64_t>(warps, (int64_t)(avail / per_warp));
+    // The leaves of a few pairs (no more than SMs) run in the scratch that the
+    // breakpoint rings already hold, or on 32 warps: one 50 kbp pair's 130
+    // leaves would take 56 MB of history at once, three times its rings.
+    if (c <= ctx->sms)
+      warps = std::min<int64_t>(warps, std::max<int64_t>(32, (int64_t)(ctx->b_scratch.cap / per_warp)));
     if (warps < 1) {
       ctx->need_bytes = fixed + per_warp;
       return set_err(ctx, TSU_ENOMEM, "bidirectional mode: base-case history of one segment exceeds the budget");
@@ -1226,38 +1243,61 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   // counters: +8 the bound probe's queue head, +16 arena cursor, +24 work (cells, steps, extension bases), +64 + 8b queue head
   // and retry count of band slot b
   constexpr size_t kCounterBytes = 64 + 8 * kRunSlots;
-  constexpr size_t kProbeQueue = 8;  // the bound probe's queue head
+  constexpr size_t kProbeQueue = 8;  // the bound probes' queue heads (wide, packed)
   if ((rc = grow(ctx, ctx->b_counters, kCounterBytes))) return rc;
   // Pairs with a bound probe (tsu::wants_bound; end to end, history of every
   // score): they wait for their bounds, the others start at once.
-  const bool can_bound = !ctx->one_warp && h_plen && ctx->rp.rm <= tsu::kPackedMaxDepth && !(want_cigar && ctx->low_mem) &&
+  const bool low_mem = want_cigar && ctx->low_mem < 0;
+  const bool can_bound = !ctx->one_warp && h_plen && ctx->rp.rm <= tsu::kPackedMaxDepth &&
+                         !(want_cigar && ctx->low_mem > 0) &&
                          !(ctx->ends_free[0] | ctx->ends_free[1] | ctx->ends_free[2] | ctx->ends_free[3]);
+  // A list of pairs to probe: those of the wide probe (longer than
+  // kPackedMaxLen) first, each part longest first.
+  struct ProbePlan {
+    int64_t n_wide = 0;  // pairs of the wide probe
+    int seq = 0, blocks = 0, wide_blocks = 0;
+    size_t smem = 0, wide_smem = 0;
+  };
+  auto plan_probes = [&](std::vector<int32_t>* list, ProbePlan* p) -> int {
+    std::stable_sort(list->begin(), list->end(), [&](int32_t u, int32_t v) {
+      const bool wu = std::max(h_plen[u], h_tlen[u]) > tsu::kPackedMaxLen;
+      const bool wv = std::max(h_plen[v], h_tlen[v]) > tsu::kPackedMaxLen;
+      if (wu != wv) return wu;
+      return (int64_t)h_plen[u] + h_tlen[u] > (int64_t)h_plen[v] + h_tlen[v];
+    });
+    for (int32_t i : *list) {
+      if (std::max(h_plen[i], h_tlen[i]) > tsu::kPackedMaxLen)
+        ++p->n_wide;
+      else
+        p->seq = std::max(p->seq, (int)(2 * tsu::packed_words(h_plen[i]) + 2 * tsu::packed_words(h_tlen[i])));
+    }
+    const int64_t n_packed = (int64_t)list->size() - p->n_wide;
+    int rc2;
+    if (n_packed && (rc2 = plan_probe(ctx, false, p->seq, n_packed, &p->blocks, &p->smem))) return rc2;
+    if (p->n_wide && (rc2 = plan_probe(ctx, true, 0, p->n_wide, &p->wide_blocks, &p->wide_smem))) return rc2;
+    // rings too deep for a probe's block: those pairs keep their bands
+    if (n_packed && !p->blocks) list->resize((size_t)p->n_wide);
+    if (p->n_wide && !p->wide_blocks) {
+      list->erase(list->begin(), list->begin() + (ptrdiff_t)p->n_wide);
+      p->n_wide = 0;
+    }
+    return TSU_OK;
+  };
   std::vector<int32_t> probed;
+  ProbePlan probe;
   if (can_bound) {
     for (int64_t i = 0; i < n; ++i)
-      if (tsu::wants_bound(ctx->rp, h_plen[i], h_tlen[i])) probed.push_back((int32_t)i);
-    if ((int64_t)probed.size() <= ctx->sms)
+      if (tsu::wants_bound(ctx->rp, h_plen[i], h_tlen[i]) ||
+          (low_mem && std::max(h_plen[i], h_tlen[i]) >= tsu::kBoundLowMemLen && std::min(h_plen[i], h_tlen[i]) > 0))
+        probed.push_back((int32_t)i);
+    if ((int64_t)probed.size() <= ctx->sms && !low_mem)
       probed.erase(std::remove_if(probed.begin(), probed.end(),
                                   [&](int32_t i) { return std::max(h_plen[i], h_tlen[i]) < tsu::kBoundFewLen; }),
                    probed.end());
     if ((rc = grow(ctx, ctx->b_bound, sizeof(int32_t) * n))) return rc;
     if ((rc = host_grow(ctx, ctx->h_bound, sizeof(int32_t) * (size_t)n))) return rc;
-    std::stable_sort(probed.begin(), probed.end(), [&](int32_t u, int32_t v) {
-      return (int64_t)h_plen[u] + h_tlen[u] > (int64_t)h_plen[v] + h_tlen[v];
-    });
+    if ((rc = plan_probes(&probed, &probe))) return rc;
   }
-  struct ProbePlan {
-    int seq = 0, blocks = 0;
-    size_t smem = 0;
-  };
-  auto probe_plan = [&](const std::vector<int32_t>& list, ProbePlan* p) -> int {
-    for (int32_t i : list)
-      p->seq = std::max(p->seq, (int)(2 * tsu::packed_words(h_plen[i]) + 2 * tsu::packed_words(h_tlen[i])));
-    return list.empty() ? TSU_OK : plan_probe(ctx, p->seq, (int64_t)list.size(), &p->blocks, &p->smem);
-  };
-  ProbePlan probe;
-  if ((rc = probe_plan(probed, &probe))) return rc;
-  if (!probe.blocks) probed.clear();  // rings too deep for the probe's blocks
   const int64_t n_probed = (int64_t)probed.size();
   const int min_pen = ctx->rp.min_pen();
   int64_t arena_cap = 0;
@@ -1342,7 +1382,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       r.hint = ctx->err_hint;
       if (ctx->fit_start && !ctx->one_warp)
         r.pc = tsu::fit_start(r.pc, ctx->rp, r.bi.max_m, r.bi.max_n, r.hint, ctx->smem_optin);
-      if (!ctx->one_warp) r.pc = tsu::fill_warps(r.pc, r.n, ctx->sms);
+      if (!ctx->one_warp) r.pc = tsu::fill_warps(r.pc, r.n, std::max(r.bi.max_m, r.bi.max_n), ctx->sms);
       if ((rc = plan_pass_within(ctx, r.bi, r.n, r.pc, r.hint, want_cigar, avail, &r.ps))) return rc;
       need = std::max(need, scratch_bytes(r.ps, want_cigar));
     }
@@ -1388,6 +1428,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     a.ef_te = ctx->ends_free[3];
     a.bound = ps.g.bounded ? P<int32_t>(ctx->b_bound) : nullptr;
     a.group_bytes = ps.g.group_smem;
+    a.wide_cell = ps.g.wide_cell;
     return a;
   };
   // The bound probe over `count` pairs of the order from `off` on, their bounds
@@ -1397,14 +1438,23 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     tsu::ProbeArgs b{};
     b.seq = sv;
     b.pk = pk;
-    b.order = P<int32_t>(ctx->b_order) + off;
-    b.n_order = count;
     b.pen = ctx->rp;
     b.seq_cap = p.seq;
     b.bound = P<int32_t>(ctx->b_bound);
-    b.queue = reinterpret_cast<unsigned int*>(d_cnt + kProbeQueue);
-    launch_probe(ctx, p.blocks, p.smem, st, b);
-    CU(cudaGetLastError());
+    if (p.n_wide) {
+      b.order = P<int32_t>(ctx->b_order) + off;
+      b.n_order = p.n_wide;
+      b.queue = reinterpret_cast<unsigned int*>(d_cnt + kProbeQueue);
+      launch_probe(ctx, true, p.wide_blocks, p.wide_smem, st, b);
+      CU(cudaGetLastError());
+    }
+    if (count > p.n_wide) {
+      b.order = P<int32_t>(ctx->b_order) + off + p.n_wide;
+      b.n_order = count - p.n_wide;
+      b.queue = reinterpret_cast<unsigned int*>(d_cnt + kProbeQueue) + 1;
+      launch_probe(ctx, false, p.blocks, p.smem, st, b);
+      CU(cudaGetLastError());
+    }
     CU(cudaMemcpyAsync(ctx->h_bound.p, ctx->b_bound.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
     return TSU_OK;
   };
@@ -1418,29 +1468,34 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       std::vector<int32_t> pairs;
       BatchInfo bi;
       int bytes = 0;  // of shared memory, at 16 warps per pair
+      int width = 0;  // diagonals
       int32_t ub = 0;
       int64_t hist = 0;
     };
-    std::vector<Class> cls((size_t)tsu::kBoundClasses + tsu::kBands);
-    const size_t wide = (size_t)tsu::kBoundClasses;
+    // classes of the shared ring, of the wide kernel (16- and 32-bit rows), bands
+    constexpr int kWide = tsu::kBoundClasses, kBand0 = kWide + 2, kAll = kBand0 + tsu::kBands;
+    std::vector<Class> cls((size_t)kAll);
     for (int32_t i : list) {
       const int32_t m = h_plen[i], t = h_tlen[i], u = ub[i];
-      size_t c = wide + (size_t)tsu::length_band(std::max(m, t));
+      size_t c = (size_t)(kBand0 + tsu::length_band(std::max(m, t)));
       tsu::BoundNeed need;
       int bytes = 0;
       if (u != tsu::kNoBound) {
         need = tsu::bound_need(ctx->rp, m, t, u);
         bytes = tsu::bounded_bytes(ctx->rp, need.width, need.words, 16);
         int per_sm = 0;
-        if (tsu::packed_width(need.width) <= tsu::kPackedMaxW &&
+        if (std::max(m, t) <= tsu::kPackedMaxLen && tsu::packed_width(need.width) <= tsu::kPackedMaxW &&
             tsu::bounded_warps(bytes, INT32_MAX, ctx->sms, ctx->smem_optin, &per_sm))
           c = (size_t)tsu::bound_class(per_sm);
+        else if (need.hist <= tsu::kWideMaxHist)
+          c = (size_t)(t <= tsu::kWide16MaxLen ? kWide : kWide + 1);
       }
       Class& k = cls[c];
       k.pairs.push_back(i);
       k.bi.max_m = std::max(k.bi.max_m, m);
       k.bi.max_n = std::max(k.bi.max_n, t);
       k.bytes = std::max(k.bytes, bytes);
+      k.width = std::max(k.width, need.width);
       k.ub = std::max(k.ub, u);
       k.hist = std::max(k.hist, need.hist);
     }
@@ -1450,9 +1505,9 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     const size_t avail = ctx->budget > fixed ? ctx->budget - fixed : 0;
     size_t need_bytes = 0, each = 0;
     int rc2;
-    for (int j = 0; j < tsu::kBoundClasses + tsu::kBands; ++j) {
-      // unbounded bands first (longest first), then the widest class first
-      const int c = j < tsu::kBands ? tsu::kBoundClasses + tsu::kBands - 1 - j : j - tsu::kBands;
+    for (int c = kAll - 1, done = 0; done < kAll; ++done, c = c == kWide ? 0 : (c < kWide ? c + 1 : c - 1)) {
+      // bands without a bound first (longest first), the wide kernel's, then
+      // the shared rings', widest first
       Class& k = cls[(size_t)c];
       if (k.pairs.empty()) continue;
       BandRun r;
@@ -1462,17 +1517,36 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       r.bi = k.bi;
       r.bi.n = r.n;
       r.hint = ctx->err_hint;
-      int gw = 0;
-      if (c < tsu::kBoundClasses)
-        gw = tsu::bounded_warps(k.bytes, r.n, ctx->sms, ctx->smem_optin);
-      if (gw) {
-        r.pc = tsu::PassChoice{tsu::kModeShared, gw};
-        const tsu::PassGeom g = tsu::plan_bounded(k.bytes, k.ub, k.hist, gw, want_cigar);
-        if ((rc2 = plan_groups(ctx, g, r.n, want_cigar, avail, &r.ps))) return rc2;
-      } else {
-        r.band = c < tsu::kBoundClasses ? tsu::kBands - 1 : c - tsu::kBoundClasses;
-        r.pc = tsu::band_start_in(ctx->band_start, r.band, std::max(k.bi.max_m, k.bi.max_n));
-        if (ctx->fit_start) r.pc = tsu::fit_start(r.pc, ctx->rp, k.bi.max_m, k.bi.max_n, r.hint, ctx->smem_optin);
+      // the launch without a bound, and the scratch the bounded one may take:
+      // in low-memory mode no more than that one's
+      r.band = tsu::length_band(std::max(k.bi.max_m, k.bi.max_n));
+      tsu::PassChoice plain = tsu::band_start_in(ctx->band_start, r.band, std::max(k.bi.max_m, k.bi.max_n));
+      if (ctx->fit_start) plain = tsu::fit_start(plain, ctx->rp, k.bi.max_m, k.bi.max_n, r.hint, ctx->smem_optin);
+      size_t room = avail;
+      bool planned = false;
+      if (c < kBand0) {
+        if (low_mem) {
+          Pass old;
+          if (plan_pass_within(ctx, r.bi, r.n, plain, r.hint, want_cigar, avail, &old) == TSU_OK)
+            room = std::min(room, (size_t)old.groups * group_scratch_bytes(old.g));
+        }
+        tsu::PassGeom g;
+        if (c < kWide) {
+          const int gw = tsu::bounded_warps(k.bytes, r.n, ctx->sms, ctx->smem_optin);
+          r.pc = tsu::PassChoice{tsu::kModeShared, gw};
+          g = tsu::plan_bounded(k.bytes, k.ub, k.hist, gw, want_cigar);
+        } else {
+          r.pc = tsu::PassChoice{tsu::kModeGlobal, 16};
+          g = tsu::plan_wide(ctx->rp, k.bi.max_n, k.width, k.ub, k.hist, want_cigar);
+        }
+        // (a history beyond the budget: the plain launch has its own ways)
+        if (group_scratch_bytes(g) <= room) {
+          if ((rc2 = plan_groups(ctx, g, r.n, want_cigar, room, &r.ps))) return rc2;
+          planned = true;
+        }
+      }
+      if (!planned) {
+        r.pc = plain;
         if ((rc2 = plan_pass_within(ctx, r.bi, r.n, r.pc, r.hint, want_cigar, avail, &r.ps))) return rc2;
       }
       need_bytes = std::max(need_bytes, scratch_bytes(r.ps, want_cigar));
@@ -1554,7 +1628,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     return TSU_OK;
   });
   if (rc) return rc;
-  ctx->timing.kernel_launches += 3 + (int64_t)runs.size() + (n_probed ? 1 : 0);
+  ctx->timing.kernel_launches += 3 + (int64_t)runs.size() + (probe.n_wide ? 1 : 0) + (n_probed > probe.n_wide ? 1 : 0);
   CU(wait_stream(ctx, st));
   if (n_probed) {
     if ((rc = bounded_runs(probed, probe_off))) return rc;
@@ -1575,26 +1649,23 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       const int32_t* l = static_cast<const int32_t*>(ctx->h_list.p);
       const size_t before = again.size();
       for (unsigned int i = 0; i < c; ++i)
-        if (std::max(h_plen[l[i]], h_tlen[l[i]]) <= tsu::kPackedMaxLen && std::min(h_plen[l[i]], h_tlen[l[i]]) > 0)
-          again.push_back(l[i]);
+        if (std::min(h_plen[l[i]], h_tlen[l[i]]) > 0) again.push_back(l[i]);
       if (again.size() - before == c && c > (unsigned)ctx->sms)
         r.rebound = true;  // all of them
       else
         again.resize(before);
     }
     ProbePlan p;
-    if ((rc = probe_plan(again, &p))) return rc;
-    if (p.blocks) {
-      std::stable_sort(again.begin(), again.end(), [&](int32_t u, int32_t v) {
-        return (int64_t)h_plen[u] + h_tlen[u] > (int64_t)h_plen[v] + h_tlen[v];
-      });
+    const size_t asked = again.size();
+    if ((rc = plan_probes(&again, &p))) return rc;
+    if (asked && again.size() == asked) {
       if ((rc = host_grow(ctx, ctx->h_list, sizeof(int32_t) * again.size()))) return rc;
       memcpy(ctx->h_list.p, again.data(), sizeof(int32_t) * again.size());
       CU(cudaMemcpyAsync(P<int32_t>(ctx->b_order) + n, ctx->h_list.p, sizeof(int32_t) * again.size(),
                          cudaMemcpyHostToDevice, st));
       CU(cudaMemsetAsync(d_cnt + kProbeQueue, 0, 8, st));
       if ((rc = queue_probe(p, n, (int64_t)again.size()))) return rc;
-      ctx->timing.kernel_launches++;
+      ctx->timing.kernel_launches += (p.n_wide ? 1 : 0) + ((int64_t)again.size() > p.n_wide ? 1 : 0);
       ctx->timing.retried_pairs += (int64_t)again.size();
       CU(wait_stream(ctx, st));
       if ((rc = bounded_runs(again, n))) return rc;

@@ -31,24 +31,47 @@ void launch_align_linear(bool cigar, int mode, int gw, int blocks, int threads, 
                          const AlignArgs& a, bool lowmem, bool bounded);
 
 // The bound probe of each model (probe_kernel).
-cudaError_t probe_occupancy_dual(int threads, size_t smem, int optin, int* occ);
-void launch_probe_dual(int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a);
-cudaError_t probe_occupancy_linear(int threads, size_t smem, int optin, int* occ);
-void launch_probe_linear(int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a);
+// wide: of pairs of any length (wide_probe_kernel).
+cudaError_t probe_occupancy_dual(bool wide, int threads, size_t smem, int optin, int* occ);
+void launch_probe_dual(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a);
+cudaError_t probe_occupancy_linear(bool wide, int threads, size_t smem, int optin, int* occ);
+void launch_probe_linear(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a);
+// The wide kernel of each model (wide_kernel; one block of kWideThreads per
+// pair, a.wide_cell bytes per ring cell).
+void launch_wide_dual(bool cigar, int blocks, size_t smem, cudaStream_t st, const AlignArgs& a);
+void launch_wide_linear(bool cigar, int blocks, size_t smem, cudaStream_t st, const AlignArgs& a);
 
 namespace launch_detail {
 
 template <int kModel>
-cudaError_t probe_occupancy(int threads, size_t smem, int optin, int* occ) {
-  const cudaError_t e =
-      cudaFuncSetAttribute(probe_kernel<kModel>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+cudaError_t probe_occupancy(bool wide, int threads, size_t smem, int optin, int* occ) {
+  const void* const f = wide ? (const void*)wide_probe_kernel<kModel> : (const void*)probe_kernel<kModel>;
+  const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, probe_kernel<kModel>, threads, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, f, threads, smem);
 }
 
 template <int kModel>
-void probe(int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {
-  probe_kernel<kModel><<<blocks, threads, smem, st>>>(a);
+void probe(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {
+  if (wide)
+    wide_probe_kernel<kModel><<<blocks, threads, smem, st>>>(a);
+  else
+    probe_kernel<kModel><<<blocks, threads, smem, st>>>(a);
+}
+
+template <int kModel>
+void wide(bool cigar, int blocks, size_t smem, cudaStream_t st, const AlignArgs& a) {
+  if (a.wide_cell == 2) {
+    if (cigar)
+      wide_kernel<true, kModel, uint16_t><<<blocks, kWideThreads, smem, st>>>(a);
+    else
+      wide_kernel<false, kModel, uint16_t><<<blocks, kWideThreads, smem, st>>>(a);
+  } else {
+    if (cigar)
+      wide_kernel<true, kModel, uint32_t><<<blocks, kWideThreads, smem, st>>>(a);
+    else
+      wide_kernel<false, kModel, uint32_t><<<blocks, kWideThreads, smem, st>>>(a);
+  }
 }
 
 template <bool kCigar, int kMode, int GW, int kModel>

@@ -16,12 +16,16 @@ void launch_align_linear(bool cigar, int mode, int gw, int blocks, int threads, 
   launch_detail::launch<kModelLinear>(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded);
 }
 
-cudaError_t probe_occupancy_linear(int threads, size_t smem, int optin, int* occ) {
-  return launch_detail::probe_occupancy<kModelLinear>(threads, smem, optin, occ);
+cudaError_t probe_occupancy_linear(bool wide, int threads, size_t smem, int optin, int* occ) {
+  return launch_detail::probe_occupancy<kModelLinear>(wide, threads, smem, optin, occ);
 }
 
-void launch_probe_linear(int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {
-  launch_detail::probe<kModelLinear>(blocks, threads, smem, st, a);
+void launch_probe_linear(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {
+  launch_detail::probe<kModelLinear>(wide, blocks, threads, smem, st, a);
+}
+
+void launch_wide_linear(bool cigar, int blocks, size_t smem, cudaStream_t st, const AlignArgs& a) {
+  launch_detail::wide<kModelLinear>(cigar, blocks, smem, st, a);
 }
 
 }  // namespace tsu

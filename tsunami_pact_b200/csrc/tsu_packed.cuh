@@ -457,15 +457,15 @@ __device__ __forceinline__ int warp_lcp(smem_t pw, int v, smem_t tw, int h, int 
 // registers at a time (lane l holds score top - l: 16 diagonals around the
 // path; 8 with two gap pieces), each edit or gap written as one entry
 // (length << 4 | op) downwards from out + cap.  Then the replay from the
-// front: matches found again between the entries, runs written upwards from
+// front: matches found again between the entries (lcp(v, h, at most)), runs written upwards from
 // out.  Of e entries at most 2 e + 1 runs are written, 2 j + 1 of them before
 // entry j is read, so with cap >= 2 e + 2 they share the space.  Returns the
 // number of runs, or -1 on an inconsistency.
-template <int kModel>
+template <int kModel, class Lcp>
 __device__ __forceinline__ int packed_cigar(const uint32_t* hist, int64_t hist_chunks,
                                             const int2* table, int s_end, int k_fin, int m, int n,
-                                            const Pen& pen, int kbase, int lo0, int hi0, smem_t pw,
-                                            smem_t tw, uint32_t* out, int cap, int lane) {
+                                            const Pen& pen, int kbase, int lo0, int hi0, Lcp&& lcp,
+                                            uint32_t* out, int cap, int lane) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr bool kDual = kModel == kModelDual, kLin = kModel == kModelLinear;
   constexpr int kCS = kDual ? 1 : 2;  // log2 of pairs of diagonals per 32-bit chunk
@@ -553,7 +553,7 @@ __device__ __forceinline__ int packed_cigar(const uint32_t* hist, int64_t hist_c
   for (int j = 0;; ++j) {
     const int rem = min(m - v, n - h);
     if (rem < 0) return -1;
-    const int l = warp_lcp(pw, v, tw, h, rem, lane);
+    const int l = lcp(v, h, rem);
     put(kOpM, l);
     v += l;
     h += l;
@@ -862,8 +862,9 @@ __device__ __forceinline__ void align_packed(const AlignArgs& a, unsigned char* 
               st = kPairArena;
             } else {
               __syncwarp();
-              len = packed_cigar<kModel>(hist, hbase, table, s_end, k_fin, m, n, a.pen, kbase, lo0, hi0, pws, tws,
-                                         a.arena + at, (int)bound, lane);
+              len = packed_cigar<kModel>(
+                  hist, hbase, table, s_end, k_fin, m, n, a.pen, kbase, lo0, hi0,
+                  [&](int v, int h, int rem) { return warp_lcp(pws, v, tws, h, rem, lane); }, a.arena + at, (int)bound, lane);
               if (len < 0) {
                 st = kPairInternal;
                 len = 0;

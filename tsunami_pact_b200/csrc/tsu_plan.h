@@ -36,7 +36,8 @@ struct PassGeom {
   int ckpt_k = 0;          // low-memory mode: checkpoint interval (0: off)
   int ckpt_cap = 0;        // checkpoints per group
   int64_t ckpt_bytes = 0;  // bytes per checkpoint
-  bool bounded = false;    // pairs with score bounds (plan_bounded)
+  bool bounded = false;    // pairs with score bounds (plan_bounded, plan_wide)
+  int wide_cell = 0;       // of these, the wide kernel's: bytes of a ring cell (2 or 4)
 };
 
 constexpr int kSharedW1 = 384;         // shared-mode ring width for one warp per pair (diagonals)
@@ -257,7 +258,7 @@ constexpr int kBoundMinWidth = 420;
 constexpr int kBoundMinRing = 14 << 10;
 inline bool wants_bound(const Pen& pen, int32_t m, int32_t n) {
   const int64_t L = std::max(m, n);
-  if (L > kPackedMaxLen || std::min(m, n) <= 0) return false;
+  if (std::min(m, n) <= 0) return false;
   const int64_t ring = (int64_t)(pen.slots() + 1) * 2 * std::min<int64_t>((int64_t)m + n + 3, kSharedW1);
   return 2 * hint_score(pen, L, 0.04) / pen.min_ge() >= kBoundMinWidth || ring > kBoundMinRing;
 }
@@ -338,15 +339,44 @@ inline int bounded_warps(int bytes, int64_t n, int sms, int smem_optin, int* pai
   return best;
 }
 
+// Geometry of a launch of bounded pairs on the wide kernel: a ring of `width`
+// diagonals in device memory, one block per pair.
+inline PassGeom plan_wide(const Pen& pen, int32_t max_n, int width, int32_t max_ub, int64_t hist, bool want_cigar) {
+  PassGeom p;
+  p.mode = kModeGlobal;
+  p.bounded = true;
+  p.wide_cell = max_n <= kWide16MaxLen ? 2 : 4;
+  p.gw = 16;
+  p.cta_threads = 512;
+  p.groups_per_cta = 1;
+  p.min_blocks = 1;
+  p.group_smem = wide_smem_bytes(pen);
+  p.ring_ints = (int64_t)(pen.slots() + 1) * wide_row_bytes(width, p.wide_cell) / 4;
+  if (want_cigar) {
+    p.table_cap = max_ub + 2;
+    p.hist_cap = hist;
+  }
+  return p;
+}
+// Cells of history a wide launch may keep (32-bit words below 2^31).
+constexpr int64_t kWideMaxHist = INT32_MAX - 65536;
+
+// In low-memory mode (interval chosen here) every pair from this length on is
+// probed: with its bound a pair's whole history, 4 bits per cell of a band
+// that narrows again, takes less than the checkpoints and recomputed segment
+// planned from the error hint, and is computed once.
+constexpr int kBoundLowMemLen = 256;
+
 // Warps per pair of an unbounded shared-ring launch of n pairs: 16 when each
 // pair can have an SM to itself (one pair of 1 kbp: 0.21 ms on 1 warp, 0.14 on
 // 16; 148 of 8 kbp at 10 %: 3.1 ms, and 5.4 from 8 warps, whose ring they
 // outgrow), else those of the rung, doubled while the launch leaves an SM
-// fewer than 8 warps (600 pairs of 1 kbp: 0.22 ms on 1, 0.19 on 2, 0.26 on 4).
-inline PassChoice fill_warps(PassChoice pc, int64_t n, int sms) {
+// fewer than 8 warps (600 pairs of 1 kbp: 0.22 ms on 1, 0.19 on 2, 0.26 on 4);
+// at most one warp per 64 bases beyond the rung (20 pairs of 115 bp: 162 us a
+// call on 1 warp, 168 on 16).
+inline PassChoice fill_warps(PassChoice pc, int64_t n, int32_t maxlen, int sms) {
   if (pc.mode != kModeShared) return pc;
-  if (n <= sms) pc.gw = std::max(pc.gw, 16);
-  while (pc.gw < 16 && n * pc.gw * 2 <= (int64_t)sms * 8) pc.gw *= 2;
+  while (pc.gw < 16 && (n <= sms || n * pc.gw * 2 <= (int64_t)sms * 8) && pc.gw * 128 <= maxlen) pc.gw *= 2;
   return pc;
 }
 
