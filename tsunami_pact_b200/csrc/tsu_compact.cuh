@@ -8,9 +8,11 @@ namespace tsu {
 
 // One warp per pair, grid-stride.  The length comes from the status-masked
 // scan, so a pair that failed in this call contributes 0 runs even if its
-// cig_len slot holds a stale value.
+// cig_len slot holds a stale value.  Writes nothing when the runs are more
+// than cap: the kernel is queued before the host knows their number.
 static __global__ void compact_kernel(int64_t n, const uint32_t* __restrict__ arena, const int64_t* __restrict__ cig_pos,
-                               const int64_t* __restrict__ out_off, uint32_t* __restrict__ out) {
+                               const int64_t* __restrict__ out_off, uint32_t* __restrict__ out, int64_t cap = INT64_MAX) {
+  if (out_off[n] > cap) return;
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {

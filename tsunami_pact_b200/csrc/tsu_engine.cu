@@ -105,6 +105,7 @@ struct tsu_ctx {
   HostBuf h_status;   // int32 pair statuses (tsu_align_batch)
   HostBuf h_bidir;    // bidirectional mode: segments down, cuts and run counts up
   HostBuf h_bound;    // score bounds of the pairs
+  HostBuf h_lens;     // lengths of a device batch
   std::vector<void*> h_retired;  // outgrown page-locked buffers, freed at destroy
   // events of the host-buffer pipeline (tsu_align_batch): 8 chunks at most
   cudaEvent_t cev_up[8] = {}, cev_done[8] = {}, cev_down[8] = {}, cev_t[2] = {};
@@ -298,6 +299,20 @@ struct BatchInfo {
   int64_t n = 0;
   int32_t max_m = 0, max_n = 0;
   int64_t total_words = 0;
+  // of the pairs' longer sides and of both sides (set by add())
+  int32_t min_side = INT32_MAX, max_side = 0, min_sum = INT32_MAX, max_sum = 0;
+  int64_t len_sum = 0;
+  void add(int32_t m, int32_t t) {
+    max_m = std::max(max_m, m);
+    max_n = std::max(max_n, t);
+    total_words += tsu::packed_words(m) + tsu::packed_words(t);
+    const int32_t side = std::max(m, t), sum = m + t;
+    min_side = std::min(min_side, side);
+    max_side = std::max(max_side, side);
+    min_sum = std::min(min_sum, sum);
+    max_sum = std::max(max_sum, sum);
+    len_sum += sum;
+  }
 };
 
 // The align_kernel instantiations (tsu_launch.cuh): gap-affine kernels here,
@@ -435,7 +450,13 @@ struct BandSplit {
   int uniform_band = 0;
 };
 
-void split_bands(int64_t n, const int32_t* h_plen, const int32_t* h_tlen, BandSplit* out) {
+void split_bands(int64_t n, const int32_t* h_plen, const int32_t* h_tlen, BandSplit* out, const BatchInfo* info = nullptr) {
+  auto bits = [](uint32_t l) { return l ? 32 - __builtin_clz(l) : 0; };
+  if (n && info && bits((uint32_t)info->min_sum) == bits((uint32_t)info->max_sum) &&
+      tsu::length_band(info->min_side) == tsu::length_band(info->max_side)) {
+    out->uniform_band = tsu::length_band(info->max_side);
+    return;
+  }
   int64_t cnt[34] = {0};
   auto cls = [&](int64_t i) {
     const uint32_t l = (uint32_t)h_plen[i] + (uint32_t)h_tlen[i];
@@ -1230,6 +1251,11 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   if ((rc = grow(ctx, ctx->b_woff, sizeof(int64_t) * 2 * n))) return rc;
   size_t tmp_bytes = 0;
   cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, P<int64_t>(ctx->b_words_cnt), P<int64_t>(ctx->b_woff), (int)(2 * n), st);
+  size_t off_tmp = 0;  // the scan of run counts
+  if (want_cigar) {
+    cub::DeviceScan::ExclusiveSum(nullptr, off_tmp, P<int64_t>(ctx->b_clen64), d_out_off, (int)(n + 1), st);
+    tmp_bytes = std::max(tmp_bytes, off_tmp);
+  }
   if ((rc = grow(ctx, ctx->b_scan_tmp, tmp_bytes))) return rc;
   if ((rc = grow(ctx, ctx->b_words, sizeof(uint64_t) * (size_t)bi.total_words))) return rc;
   if ((rc = grow(ctx, ctx->b_nonacgt, (size_t)(2 * n)))) return rc;
@@ -1286,10 +1312,11 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   std::vector<int32_t> probed;
   ProbePlan probe;
   if (can_bound) {
-    for (int64_t i = 0; i < n; ++i)
-      if (tsu::wants_bound(ctx->rp, h_plen[i], h_tlen[i]) ||
-          (low_mem && std::max(h_plen[i], h_tlen[i]) >= tsu::kBoundLowMemLen && std::min(h_plen[i], h_tlen[i]) > 0))
-        probed.push_back((int32_t)i);
+    tsu::BoundLimits limits = tsu::bound_limits(ctx->rp);
+    if (low_mem) limits.side = std::min(limits.side, tsu::kBoundLowMemLen);
+    if (bi.max_side >= limits.side || bi.max_sum >= limits.sum)
+      for (int64_t i = 0; i < n; ++i)
+        if (limits.wants(h_plen[i], h_tlen[i])) probed.push_back((int32_t)i);
     if ((int64_t)probed.size() <= ctx->sms && !low_mem)
       probed.erase(std::remove_if(probed.begin(), probed.end(),
                                   [&](int32_t i) { return std::max(h_plen[i], h_tlen[i]) < tsu::kBoundFewLen; }),
@@ -1315,9 +1342,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   }
   // The compacted runs (at most the arena's, at most m + n per pair) are
   // allocated after the passes: each pass's scratch leaves room for them.
-  int64_t len_sum = 0;
-  for (int64_t i = 0; h_plen && i < n; ++i) len_sum += (int64_t)h_plen[i] + h_tlen[i];
-  if (!h_plen) len_sum = n * ((int64_t)bi.max_m + bi.max_n);
+  const int64_t len_sum = h_plen ? bi.len_sum : n * ((int64_t)bi.max_m + bi.max_n);
   auto out_reserve = [&]() -> size_t {
     if (!want_cigar || d_out_runs) return 0;
     const DevBuf& ob = out_buf ? *out_buf : ctx->b_out;
@@ -1340,7 +1365,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     bool rebound = false;  // the pairs that outgrew it have run again with bounds
   };
   BandSplit split;
-  if (!ctx->one_warp && h_plen) split_bands(n, h_plen, h_tlen, &split);
+  if (!ctx->one_warp && h_plen) split_bands(n, h_plen, h_tlen, &split, &bi);
   if (n_probed) drop_probed(n, h_plen, h_tlen, probed, &split);
   const bool all_pairs = ctx->one_warp || !h_plen || split.uniform;  // one band of every pair, input order
   std::vector<BandRun> runs;
@@ -1596,6 +1621,33 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
                std::to_string(ps.g.gw) + "x" + std::to_string(ps.groups) + ":" + std::to_string(pairs);
   };
 
+  // Run offsets of the pairs (scan of their run counts into d_out_off, the
+  // total to h_total), and the runs gathered into `runs` when they fit cap.
+  int64_t* const h_total = reinterpret_cast<int64_t*>(static_cast<char*>(ctx->h_scalars.p) + 2048);
+  auto queue_offsets = [&]() -> int {
+    tsu::cig_len64_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, st>>>(
+        n, P<int32_t>(ctx->b_clen), d_status, P<int64_t>(ctx->b_clen64));
+    CU(cudaMemsetAsync(P<int64_t>(ctx->b_clen64) + n, 0, sizeof(int64_t), st));
+    size_t tb = off_tmp;
+    CU(cub::DeviceScan::ExclusiveSum(ctx->b_scan_tmp.p, tb, P<int64_t>(ctx->b_clen64), d_out_off, (int)(n + 1), st));
+    CU(cudaMemcpyAsync(h_total, d_out_off + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    CU(cudaGetLastError());
+    return TSU_OK;
+  };
+  auto queue_runs = [&](uint32_t* runs, int64_t cap) -> int {
+    const int64_t blocks = std::min<int64_t>((n + 7) / 8, (int64_t)ctx->sms * 16);
+    tsu::compact_kernel<<<(int)blocks, 256, 0, st>>>(n, P<uint32_t>(ctx->b_arena), P<int64_t>(ctx->b_cpos), d_out_off,
+                                                    runs, cap);
+    CU(cudaGetLastError());
+    return TSU_OK;
+  };
+  // Without pairs to probe the offsets and runs are queued behind the graph
+  // while it runs: most calls have no retry, and then need no round trip
+  // between the passes and them.  A call with retries does this part again.
+  const bool early = want_cigar && n_probed == 0;
+  DevBuf& out_ctx = out_buf ? *out_buf : ctx->b_out;
+  uint32_t* const early_runs = d_out_runs ? d_out_runs : P<uint32_t>(out_ctx);
+  const int64_t early_cap = early_runs ? (d_out_runs ? out_cap : (int64_t)(out_ctx.cap / sizeof(uint32_t))) : 0;
   // ---- the fixed launch sequence of the call (one CUDA graph)
   rc = run_graph(ctx, st, [&]() -> int {
     CU(record(ctx, ctx->ev[2], st));
@@ -1628,6 +1680,12 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     return TSU_OK;
   });
   if (rc) return rc;
+  if (early) {
+    CU(cudaEventRecord(ctx->ev[5], st));
+    if ((rc = queue_offsets())) return rc;
+    if (early_cap > 0 && (rc = queue_runs(early_runs, early_cap))) return rc;
+    CU(cudaEventRecord(ctx->ev[6], st));
+  }
   ctx->timing.kernel_launches += 3 + (int64_t)runs.size() + (probe.n_wide ? 1 : 0) + (n_probed > probe.n_wide ? 1 : 0);
   CU(wait_stream(ctx, st));
   if (n_probed) {
@@ -1636,6 +1694,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   // Pairs that outgrew an unbounded shared ring get a bound, and a second
   // start with it: 20,000 pairs of 800 - 1,000 bp at 10 % took 13.2 ms through
   // the ladder.  (Few of them: the ladder's 16 warps are as good.)
+  bool rebound_any = false;
   if (can_bound) {
     std::vector<int32_t> again;
     const size_t first_runs = runs.size();
@@ -1667,6 +1726,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       if ((rc = queue_probe(p, n, (int64_t)again.size()))) return rc;
       ctx->timing.kernel_launches += (p.n_wide ? 1 : 0) + ((int64_t)again.size() > p.n_wide ? 1 : 0);
       ctx->timing.retried_pairs += (int64_t)again.size();
+      rebound_any = true;
       CU(wait_stream(ctx, st));
       if ((rc = bounded_runs(again, n))) return rc;
     } else {
@@ -1782,7 +1842,8 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       if (nretry == 0) break;
     }
   }
-  CU(cudaEventRecord(ctx->ev[5], st));
+  const bool done_early = early && !laddered && !rebound_any;
+  if (!done_early) CU(cudaEventRecord(ctx->ev[5], st));
   if (laddered) {
     CU(cudaMemcpyAsync(h_cnt + 24, d_work, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     CU(wait_stream(ctx, st));
@@ -1793,34 +1854,27 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
 
   // ---- CIGAR compaction
   if (want_cigar) {
-    if ((rc = grow(ctx, ctx->b_clen64, sizeof(int64_t) * (n + 1)))) return rc;
-    tsu::cig_len64_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, st>>>(
-        n, P<int32_t>(ctx->b_clen), d_status, P<int64_t>(ctx->b_clen64));
-    CU(cudaMemsetAsync(P<int64_t>(ctx->b_clen64) + n, 0, sizeof(int64_t), st));
-    ctx->timing.kernel_launches++;
-    size_t tb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb, P<int64_t>(ctx->b_clen64), d_out_off, (int)(n + 1), st);
-    if ((rc = grow(ctx, ctx->b_scan_tmp, tb))) return rc;
-    CU(cub::DeviceScan::ExclusiveSum(ctx->b_scan_tmp.p, tb, P<int64_t>(ctx->b_clen64), d_out_off, (int)(n + 1), st));
-    ctx->timing.kernel_launches++;
-    int64_t* h_total = reinterpret_cast<int64_t*>(static_cast<char*>(ctx->h_scalars.p) + 32);
-    CU(cudaMemcpyAsync(h_total, d_out_off + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    CU(wait_stream(ctx, st));
+    ctx->timing.kernel_launches += 2;
+    if (!done_early) {
+      if ((rc = queue_offsets())) return rc;
+      CU(wait_stream(ctx, st));
+    }
     const int64_t total = *h_total;
     if (runs_needed) *runs_needed = total;
+    if (done_early && early_cap > 0 && total <= early_cap) {
+      if (!d_out_runs && out_used) *out_used = early_runs;
+      ctx->timing.kernel_launches++;
+      return TSU_OK;
+    }
     if (!d_out_runs) {
-      DevBuf& ob = out_buf ? *out_buf : ctx->b_out;
-      if ((rc = grow(ctx, ob, sizeof(uint32_t) * (size_t)std::max<int64_t>(total, 1)))) return rc;
-      d_out_runs = P<uint32_t>(ob);
+      if ((rc = grow(ctx, out_ctx, sizeof(uint32_t) * (size_t)std::max<int64_t>(total, 1)))) return rc;
+      d_out_runs = P<uint32_t>(out_ctx);
       out_cap = total;
       if (out_used) *out_used = d_out_runs;
     }
     if (total > out_cap) return TSU_EOVERFLOW;
-    const int64_t blocks = std::min<int64_t>((n + 7) / 8, (int64_t)ctx->sms * 16);
-    tsu::compact_kernel<<<(int)blocks, 256, 0, st>>>(n, P<uint32_t>(ctx->b_arena), P<int64_t>(ctx->b_cpos), d_out_off,
-                                                    d_out_runs);
+    if ((rc = queue_runs(d_out_runs, out_cap))) return rc;
     ctx->timing.kernel_launches++;
-    CU(cudaGetLastError());
   }
   CU(cudaEventRecord(ctx->ev[6], st));
   return TSU_OK;
@@ -2226,7 +2280,7 @@ int tsu_destroy(tsu_ctx* ctx) {
   if (ctx->wait_ev) cudaEventDestroy(ctx->wait_ev);
   for (auto& ev : ctx->bev) cudaEventDestroy(ev);
   if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
-  for (HostBuf* hb : {&ctx->h_scalars, &ctx->h_list, &ctx->h_status, &ctx->h_bidir, &ctx->h_bound})
+  for (HostBuf* hb : {&ctx->h_scalars, &ctx->h_list, &ctx->h_status, &ctx->h_bidir, &ctx->h_bound, &ctx->h_lens})
     if (hb->p) cudaFreeHost(hb->p);
   for (void* p : ctx->h_retired) cudaFreeHost(p);
   if (ctx->h2d_stream && ctx->h2d_stream != ctx->stream) cudaStreamDestroy(ctx->h2d_stream);
@@ -2305,9 +2359,7 @@ int tsu_align_batch(tsu_ctx* ctx, const tsu_batch* b, tsu_result* res, uint32_t 
       p1 = std::max(p1, b->pattern_off[i] + m);
       t0 = std::min(t0, b->text_off[i]);
       t1 = std::max(t1, b->text_off[i] + t);
-      ci.max_m = std::max(ci.max_m, m);
-      ci.max_n = std::max(ci.max_n, t);
-      ci.total_words += tsu::packed_words(m) + tsu::packed_words(t);
+      ci.add(m, t);
     }
     if (p1 > p0) {
       CU(cudaMemcpyAsync(P<char>(ctx->b_pat) + p0, b->pattern + p0, (size_t)(p1 - p0), cudaMemcpyHostToDevice,
@@ -2441,20 +2493,18 @@ int tsu_align_batch_device(tsu_ctx* ctx, const tsu_batch* b, tsu_result* res, ui
   // batch info: lengths are on the device; bring them over once.
   BatchInfo bi;
   bi.n = n;
-  std::vector<int32_t> pl((size_t)n), tl((size_t)n);
-  {
-    if (n) {
-      CU(cudaMemcpyAsync(pl.data(), b->pattern_len, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
-      CU(cudaMemcpyAsync(tl.data(), b->text_len, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
-      CU(wait_stream(ctx, st));
-    }
-    for (int64_t i = 0; i < n; ++i) {
-      if (pl[(size_t)i] < 0 || tl[(size_t)i] < 0 || pl[(size_t)i] > max_len(ctx) || tl[(size_t)i] > max_len(ctx))
-        return set_err(ctx, TSU_EINVAL, "pair %lld: bad length", (long long)i);
-      bi.max_m = std::max(bi.max_m, pl[(size_t)i]);
-      bi.max_n = std::max(bi.max_n, tl[(size_t)i]);
-      bi.total_words += tsu::packed_words(pl[(size_t)i]) + tsu::packed_words(tl[(size_t)i]);
-    }
+  if (int rc = host_grow(ctx, ctx->h_lens, 2 * sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1))) return rc;
+  int32_t* const pl = static_cast<int32_t*>(ctx->h_lens.p);
+  int32_t* const tl = pl + n;
+  if (n) {
+    CU(cudaMemcpyAsync(pl, b->pattern_len, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
+    CU(cudaMemcpyAsync(tl, b->text_len, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
+    CU(wait_stream(ctx, st));
+  }
+  for (int64_t i = 0; i < n; ++i) {
+    if (pl[i] < 0 || tl[i] < 0 || pl[i] > max_len(ctx) || tl[i] > max_len(ctx))
+      return set_err(ctx, TSU_EINVAL, "pair %lld: bad length", (long long)i);
+    bi.add(pl[i], tl[i]);
   }
   CU(cudaEventRecord(ctx->ev[0], st));
   CU(cudaEventRecord(ctx->ev[1], st));
@@ -2468,22 +2518,20 @@ int tsu_align_batch_device(tsu_ctx* ctx, const tsu_batch* b, tsu_result* res, ui
   }
   int64_t needed = 0;
   int rc = run_device(ctx, sv, want_cigar, res->score, d_status, res->cigar, res->cigar_capacity, res->cigar_offset,
-                      &needed, bi, pl.data(), tl.data());
+                      &needed, bi, pl, tl);
   res->cigar_needed = needed;
   if (rc) return rc;
   CU(cudaEventRecord(ctx->ev[7], st));
+  if ((rc = host_grow(ctx, ctx->h_status, sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1)))) return rc;
+  int32_t* const hs = static_cast<int32_t*>(ctx->h_status.p);
+  if (n) CU(cudaMemcpyAsync(hs, d_status, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
   CU(wait_stream(ctx, st));
   ctx->timing.pack_ms = n ? ev_ms(ctx->ev[2], ctx->ev[3]) : 0;
   ctx->timing.align_ms = n ? ev_ms(ctx->ev[4], ctx->ev[5]) : 0;
   ctx->timing.compact_ms = (n && want_cigar) ? ev_ms(ctx->ev[5], ctx->ev[6]) : 0;
   ctx->timing.total_ms = ev_ms(ctx->ev[0], ctx->ev[7]);
   ctx->timing.device_bytes = (int64_t)ctx->peak_held;
-  // statuses
-  std::vector<int32_t> hs((size_t)n);
-  if (n) {
-    CU(cudaMemcpy(hs.data(), d_status, sizeof(int32_t) * n, cudaMemcpyDeviceToHost));
-  }
-  return collect_status(ctx, hs.data(), n);
+  return collect_status(ctx, hs, n);
 }
 
 int tsu_set_ends_free(tsu_ctx* ctx, int32_t pattern_begin_free, int32_t pattern_end_free, int32_t text_begin_free,

@@ -256,11 +256,28 @@ inline int64_t arena_runs(const Pen& pen, int64_t n, int32_t max_m, int32_t max_
 // costs about what it saves.
 constexpr int kBoundMinWidth = 420;
 constexpr int kBoundMinRing = 14 << 10;
-inline bool wants_bound(const Pen& pen, int32_t m, int32_t n) {
-  const int64_t L = std::max(m, n);
-  if (std::min(m, n) <= 0) return false;
-  const int64_t ring = (int64_t)(pen.slots() + 1) * 2 * std::min<int64_t>((int64_t)m + n + 3, kSharedW1);
-  return 2 * hint_score(pen, L, 0.04) / pen.min_ge() >= kBoundMinWidth || ring > kBoundMinRing;
+// (In terms of the longer side and of both: pairs from the limits up, found
+// once per call.)
+struct BoundLimits {
+  int32_t side = INT32_MAX, sum = INT32_MAX;
+  bool wants(int32_t m, int32_t n) const {
+    return std::min(m, n) > 0 && (std::max(m, n) >= side || m + n >= sum);
+  }
+};
+inline BoundLimits bound_limits(const Pen& pen) {
+  BoundLimits b;
+  int32_t lo = 0, hi = 1 << 27;  // the shortest side whose expected width reaches kBoundMinWidth
+  while (lo < hi) {
+    const int32_t L = lo + (hi - lo) / 2;
+    if (2 * hint_score(pen, L, 0.04) / pen.min_ge() >= kBoundMinWidth)
+      hi = L;
+    else
+      lo = L + 1;
+  }
+  b.side = lo;
+  const int64_t d = kBoundMinRing / (2 * ((int64_t)pen.slots() + 1)) + 1;  // diagonals that take more than kBoundMinRing
+  if (d <= kSharedW1) b.sum = (int32_t)std::max<int64_t>(d - 3, 1);
+  return b;
 }
 // With no more such pairs than SMs each has an SM to itself, and a probe (0.35
 // us per score on one warp) adds what the narrower search saves (148 x 8 kbp
