@@ -864,14 +864,14 @@ __global__ void __launch_bounds__(kProbeThreads, 4) wide_probe_kernel(ProbeArgs 
 }
 
 constexpr int kWideThreads = 512;
-template <bool kCigar, int kModel, typename ST>
+template <bool kCigar, int kModel, typename ST, bool kCluster = false>
 __global__ void __launch_bounds__(kWideThreads, 1) wide_kernel(AlignArgs a) {
 #ifdef TSU_WARP_EMU
   unsigned char* smem_raw = emu::dyn_smem();
 #else
   extern __shared__ __align__(16) unsigned char smem_raw[];
 #endif
-  align_wide<kCigar, kModel, ST>(a, smem_raw);
+  align_wide<kCigar, kModel, ST, kCluster>(a, smem_raw);
 }
 
 }  // namespace tsu

@@ -23,8 +23,8 @@ void launch_probe_dual(bool wide, int blocks, int threads, size_t smem, cudaStre
   launch_detail::probe<kModelDual>(wide, blocks, threads, smem, st, a);
 }
 
-void launch_wide_dual(bool cigar, int blocks, size_t smem, cudaStream_t st, const AlignArgs& a) {
-  launch_detail::wide<kModelDual>(cigar, blocks, smem, st, a);
+void launch_wide_dual(bool cigar, int blocks, int cluster, size_t smem, cudaStream_t st, const AlignArgs& a) {
+  launch_detail::wide<kModelDual>(cigar, blocks, cluster, smem, st, a);
 }
 
 }  // namespace tsu

@@ -104,8 +104,10 @@ struct tsu_ctx {
   HostBuf h_list;     // int32 pass order / retry list
   HostBuf h_status;   // int32 pair statuses (tsu_align_batch)
   HostBuf h_bidir;    // bidirectional mode: segments down, cuts and run counts up
-  HostBuf h_bound;    // score bounds of the pairs
-  HostBuf h_lens;     // lengths of a device batch
+  // Lengths and statuses of a device batch, score bounds: read back once per
+  // call into memory kept by the context (page-locking them would cost a
+  // first call more than every later one gains)
+  std::vector<int32_t> h_lens, h_stat, h_bound;
   std::vector<void*> h_retired;  // outgrown page-locked buffers, freed at destroy
   // events of the host-buffer pipeline (tsu_align_batch): 8 chunks at most
   cudaEvent_t cev_up[8] = {}, cev_done[8] = {}, cev_down[8] = {}, cev_t[2] = {};
@@ -330,13 +332,13 @@ cudaError_t align_occupancy(const tsu_ctx* ctx, bool cigar, int mode, int gw, in
 }
 
 void launch_align(const tsu_ctx* ctx, bool cigar, int mode, int gw, int blocks, int threads, size_t smem,
-                  cudaStream_t st, const tsu::AlignArgs& a) {
+                  cudaStream_t st, const tsu::AlignArgs& a, int cluster = 1) {
   const bool lowmem = cigar && a.ckpt_k > 0, bounded = a.bound != nullptr;
   if (a.wide_cell) {
     switch (ctx->rp.model()) {
-      case tsu::kModelDual: tsu::launch_wide_dual(cigar, blocks, smem, st, a); break;
-      case tsu::kModelLinear: tsu::launch_wide_linear(cigar, blocks, smem, st, a); break;
-      default: tsu::launch_detail::wide<tsu::kModelAffine>(cigar, blocks, smem, st, a); break;
+      case tsu::kModelDual: tsu::launch_wide_dual(cigar, blocks, cluster, smem, st, a); break;
+      case tsu::kModelLinear: tsu::launch_wide_linear(cigar, blocks, cluster, smem, st, a); break;
+      default: tsu::launch_detail::wide<tsu::kModelAffine>(cigar, blocks, cluster, smem, st, a); break;
     }
     return;
   }
@@ -652,7 +654,7 @@ int bidir_gw(int32_t side) { return side < 2048 ? 1 : (side < 16384 ? 4 : 16); }
 // One persistent launch of the breakpoint kernel (tsu_bidir.cuh) over c
 // segments (device) of one size class, one group per segment at a time (gw
 // = 1, 4 or 16 warps), both rings of a group in device memory (2 directions
-// x ring depth x 4 components x (max_bases + 3) values, int16 below 16 warps
+// x ring depth x 4 components x (max_bases + 3) values, an even number, int16 below 16 warps
 // and int32 at 16, from the scratch buffer).  Writes T, comp, k, h at out + 0, out + stride, out + 2 stride,
 // out + 3 stride and the statuses; adds cells and steps to d_work[0..1].
 int bidir_split(tsu_ctx* ctx, const tsu::SeqView& sv, const tsu::PackView& pk, const tsu::PackView& pkr,
@@ -667,7 +669,7 @@ int bidir_split(tsu_ctx* ctx, const tsu::SeqView& sv, const tsu::PackView& pk, c
   int occ = 0;
   CU(tsu::bidir_occupancy(gw, threads, smem, &occ));
   if (occ < 1) return set_err(ctx, TSU_EDEVICE, "bidirectional kernel: no occupancy");
-  const int ring_w = max_bases + 3;
+  const int ring_w = (max_bases + 4) & ~1;  // at least m + n + 3, rows of whole words
   const int64_t ring_stride = (int64_t)2 * rp.rm * 4 * ring_w;  // elements per group
   const size_t ring_bytes = (size_t)tsu::bidir_ring_bytes(gw) * (size_t)ring_stride;
   int64_t groups = std::min<int64_t>((int64_t)ctx->sms * occ * gpb, c);
@@ -1321,9 +1323,8 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       probed.erase(std::remove_if(probed.begin(), probed.end(),
                                   [&](int32_t i) { return std::max(h_plen[i], h_tlen[i]) < tsu::kBoundFewLen; }),
                    probed.end());
-    if ((rc = grow(ctx, ctx->b_bound, sizeof(int32_t) * n))) return rc;
-    if ((rc = host_grow(ctx, ctx->h_bound, sizeof(int32_t) * (size_t)n))) return rc;
     if ((rc = plan_probes(&probed, &probe))) return rc;
+    if (!probed.empty() && (rc = grow(ctx, ctx->b_bound, sizeof(int32_t) * n))) return rc;
   }
   const int64_t n_probed = (int64_t)probed.size();
   const int min_pen = ctx->rp.min_pen();
@@ -1456,8 +1457,8 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     a.wide_cell = ps.g.wide_cell;
     return a;
   };
-  // The bound probe over `count` pairs of the order from `off` on, their bounds
-  // to ctx->h_bound.
+  // The bound probe over `count` pairs of the order from `off` on;
+  // fetch_bounds: their bounds to ctx->h_bound.
   auto queue_probe = [&](const ProbePlan& p, int64_t off, int64_t count) -> int {
     CU(cudaMemsetAsync(ctx->b_bound.p, 0x7f, sizeof(int32_t) * n, st));  // kNoBound
     tsu::ProbeArgs b{};
@@ -1480,7 +1481,12 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       launch_probe(ctx, false, p.blocks, p.smem, st, b);
       CU(cudaGetLastError());
     }
-    CU(cudaMemcpyAsync(ctx->h_bound.p, ctx->b_bound.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
+    return TSU_OK;
+  };
+  auto fetch_bounds = [&]() -> int {
+    if (ctx->h_bound.size() < (size_t)n) ctx->h_bound.resize((size_t)n);
+    CU(cudaMemcpyAsync(ctx->h_bound.data(), ctx->b_bound.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
+    CU(wait_stream(ctx, st));
     return TSU_OK;
   };
   // The probed pairs, their bounds in ctx->h_bound: classes by the width their
@@ -1488,7 +1494,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   // pairs without a bound, or too wide for a block's ring, by length band as
   // the others.  Appends to runs and reads the counters back.
   auto bounded_runs = [&](const std::vector<int32_t>& list, int64_t off) -> int {
-    const int32_t* ub = static_cast<const int32_t*>(ctx->h_bound.p);
+    const int32_t* ub = ctx->h_bound.data();
     struct Class {
       std::vector<int32_t> pairs;
       BatchInfo bi;
@@ -1563,6 +1569,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
         } else {
           r.pc = tsu::PassChoice{tsu::kModeGlobal, 16};
           g = tsu::plan_wide(ctx->rp, k.bi.max_n, k.width, k.ub, k.hist, want_cigar);
+          g.cluster = tsu::wide_cluster(r.n, ctx->sms);
         }
         // (a history beyond the budget: the plain launch has its own ways)
         if (group_scratch_bytes(g) <= room) {
@@ -1592,7 +1599,14 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     memcpy(ctx->h_list.p, order.data(), sizeof(int32_t) * order.size());
     CU(cudaMemcpyAsync(P<int32_t>(ctx->b_order) + off, ctx->h_list.p, sizeof(int32_t) * order.size(),
                        cudaMemcpyHostToDevice, st));
-    if (side) CU(cudaEventRecord(ctx->fork_ev, st));
+    for (size_t j = first; j < runs.size(); ++j)
+      for (int e = 0; e < 2; ++e)
+        if (!ctx->bev[2 * runs[j].slot + e]) CU(cudaEventCreate(&ctx->bev[2 * runs[j].slot + e]));
+    if (side) {
+      for (auto& sd : ctx->side)
+        if (!sd) CU(cudaStreamCreateWithFlags(&sd, cudaStreamNonBlocking));
+      CU(cudaEventRecord(ctx->fork_ev, st));
+    }
     size_t at = 0;
     for (size_t j = first; j < runs.size(); ++j) {
       const BandRun& r = runs[j];
@@ -1605,7 +1619,8 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
         if (cs != st) CU(cudaStreamWaitEvent(cs, ctx->fork_ev, 0));
       }
       CU(cudaEventRecord(ctx->bev[2 * r.slot], cs));
-      launch_align(ctx, want_cigar, r.ps.g.mode, r.ps.g.gw, r.ps.blocks, r.ps.threads, r.ps.smem_bytes, cs, a);
+      launch_align(ctx, want_cigar, r.ps.g.mode, r.ps.g.gw, r.ps.blocks * r.ps.g.cluster, r.ps.threads, r.ps.smem_bytes, cs, a,
+                   r.ps.g.cluster);
       CU(cudaGetLastError());
       CU(cudaEventRecord(ctx->bev[2 * r.slot + 1], cs));
       if (cs != st) CU(cudaStreamWaitEvent(st, ctx->bev[2 * r.slot + 1], 0));
@@ -1680,16 +1695,21 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     return TSU_OK;
   });
   if (rc) return rc;
+  cudaEvent_t early_ev = nullptr;
   if (early) {
     CU(cudaEventRecord(ctx->ev[5], st));
     if ((rc = queue_offsets())) return rc;
+    // the host goes on from here (the caller queues the copies of the results
+    // while the runs are gathered)
+    early_ev = ctx->blocking_sync ? ctx->wait_ev : ctx->fork_ev;
+    CU(cudaEventRecord(early_ev, st));
     if (early_cap > 0 && (rc = queue_runs(early_runs, early_cap))) return rc;
     CU(cudaEventRecord(ctx->ev[6], st));
   }
   ctx->timing.kernel_launches += 3 + (int64_t)runs.size() + (probe.n_wide ? 1 : 0) + (n_probed > probe.n_wide ? 1 : 0);
-  CU(wait_stream(ctx, st));
+  CU(early_ev ? cudaEventSynchronize(early_ev) : wait_stream(ctx, st));
   if (n_probed) {
-    if ((rc = bounded_runs(probed, probe_off))) return rc;
+    if ((rc = fetch_bounds()) || (rc = bounded_runs(probed, probe_off))) return rc;
   }
   // Pairs that outgrew an unbounded shared ring get a bound, and a second
   // start with it: 20,000 pairs of 800 - 1,000 bp at 10 % took 13.2 ms through
@@ -1722,13 +1742,13 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       memcpy(ctx->h_list.p, again.data(), sizeof(int32_t) * again.size());
       CU(cudaMemcpyAsync(P<int32_t>(ctx->b_order) + n, ctx->h_list.p, sizeof(int32_t) * again.size(),
                          cudaMemcpyHostToDevice, st));
+      if ((rc = grow(ctx, ctx->b_bound, sizeof(int32_t) * n))) return rc;
       CU(cudaMemsetAsync(d_cnt + kProbeQueue, 0, 8, st));
       if ((rc = queue_probe(p, n, (int64_t)again.size()))) return rc;
       ctx->timing.kernel_launches += (p.n_wide ? 1 : 0) + ((int64_t)again.size() > p.n_wide ? 1 : 0);
       ctx->timing.retried_pairs += (int64_t)again.size();
       rebound_any = true;
-      CU(wait_stream(ctx, st));
-      if ((rc = bounded_runs(again, n))) return rc;
+      if ((rc = fetch_bounds()) || (rc = bounded_runs(again, n))) return rc;
     } else {
       for (BandRun& r : runs) r.rebound = false;
     }
@@ -1981,7 +2001,7 @@ int predict_bytes(tsu_ctx* ctx, const BatchShape& sh, uint32_t flags, double hin
       const int gws[3] = {1, 4, 16};
       for (int k = 0; k < 3; ++k) {
         if (!cls_n[k]) continue;
-        const size_t ring = (size_t)tsu::bidir_ring_bytes(gws[k]) * 2 * (size_t)rp.rm * 4 * ((size_t)cls_bases[k] + 3);
+        const size_t ring = (size_t)tsu::bidir_ring_bytes(gws[k]) * 2 * (size_t)rp.rm * 4 * ((size_t)cls_bases[k] + 4);
         const int64_t groups = std::min<int64_t>(cls_n[k], (int64_t)ctx->sms * (gws[k] <= 4 ? 5 * (4 / gws[k]) : 1));
         scratch_full = std::max(scratch_full, (size_t)groups * ring);
         scratch_min = std::max(scratch_min, ring);
@@ -2152,10 +2172,9 @@ int create(const Spec& spec, const tsu_config* cfg, bool single_stream, tsu_ctx*
     cudaStreamCreateWithFlags(&ctx->h2d_stream, cudaStreamNonBlocking);
     cudaStreamCreateWithFlags(&ctx->d2h_stream, cudaStreamNonBlocking);
   }
-  for (auto& sd : ctx->side) cudaStreamCreateWithFlags(&sd, cudaStreamNonBlocking);
   cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming);
   ctx->pool = device_pool(ctx->device);
-  for (auto& ev : ctx->bev) cudaEventCreate(&ev);
+  for (int i = 0; i < 2 * tsu::kBands; ++i) cudaEventCreate(&ctx->bev[i]);  // (the others with their first use)
   {
     // TSU_GRAPH=0 queues the launch sequence directly instead of as a graph
     const char* gv = getenv("TSU_GRAPH");
@@ -2278,9 +2297,10 @@ int tsu_destroy(tsu_ctx* ctx) {
   }
   for (auto& ev : ctx->cev_t) cudaEventDestroy(ev);
   if (ctx->wait_ev) cudaEventDestroy(ctx->wait_ev);
-  for (auto& ev : ctx->bev) cudaEventDestroy(ev);
+  for (auto& ev : ctx->bev)
+    if (ev) cudaEventDestroy(ev);
   if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
-  for (HostBuf* hb : {&ctx->h_scalars, &ctx->h_list, &ctx->h_status, &ctx->h_bidir, &ctx->h_bound, &ctx->h_lens})
+  for (HostBuf* hb : {&ctx->h_scalars, &ctx->h_list, &ctx->h_status, &ctx->h_bidir})
     if (hb->p) cudaFreeHost(hb->p);
   for (void* p : ctx->h_retired) cudaFreeHost(p);
   if (ctx->h2d_stream && ctx->h2d_stream != ctx->stream) cudaStreamDestroy(ctx->h2d_stream);
@@ -2493,8 +2513,8 @@ int tsu_align_batch_device(tsu_ctx* ctx, const tsu_batch* b, tsu_result* res, ui
   // batch info: lengths are on the device; bring them over once.
   BatchInfo bi;
   bi.n = n;
-  if (int rc = host_grow(ctx, ctx->h_lens, 2 * sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1))) return rc;
-  int32_t* const pl = static_cast<int32_t*>(ctx->h_lens.p);
+  if (ctx->h_lens.size() < 2 * (size_t)n) ctx->h_lens.resize(2 * (size_t)n);
+  int32_t* const pl = ctx->h_lens.data();
   int32_t* const tl = pl + n;
   if (n) {
     CU(cudaMemcpyAsync(pl, b->pattern_len, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
@@ -2522,8 +2542,8 @@ int tsu_align_batch_device(tsu_ctx* ctx, const tsu_batch* b, tsu_result* res, ui
   res->cigar_needed = needed;
   if (rc) return rc;
   CU(cudaEventRecord(ctx->ev[7], st));
-  if ((rc = host_grow(ctx, ctx->h_status, sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1)))) return rc;
-  int32_t* const hs = static_cast<int32_t*>(ctx->h_status.p);
+  if (ctx->h_stat.size() < (size_t)n) ctx->h_stat.resize((size_t)n);
+  int32_t* const hs = ctx->h_stat.data();
   if (n) CU(cudaMemcpyAsync(hs, d_status, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
   CU(wait_stream(ctx, st));
   ctx->timing.pack_ms = n ? ev_ms(ctx->ev[2], ctx->ev[3]) : 0;

@@ -37,9 +37,9 @@ void launch_probe_dual(bool wide, int blocks, int threads, size_t smem, cudaStre
 cudaError_t probe_occupancy_linear(bool wide, int threads, size_t smem, int optin, int* occ);
 void launch_probe_linear(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a);
 // The wide kernel of each model (wide_kernel; one block of kWideThreads per
-// pair, a.wide_cell bytes per ring cell).
-void launch_wide_dual(bool cigar, int blocks, size_t smem, cudaStream_t st, const AlignArgs& a);
-void launch_wide_linear(bool cigar, int blocks, size_t smem, cudaStream_t st, const AlignArgs& a);
+// pair, or `cluster` of them; a.wide_cell bytes per ring cell).
+void launch_wide_dual(bool cigar, int blocks, int cluster, size_t smem, cudaStream_t st, const AlignArgs& a);
+void launch_wide_linear(bool cigar, int blocks, int cluster, size_t smem, cudaStream_t st, const AlignArgs& a);
 
 namespace launch_detail {
 
@@ -59,19 +59,35 @@ void probe(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, con
     probe_kernel<kModel><<<blocks, threads, smem, st>>>(a);
 }
 
-template <int kModel>
-void wide(bool cigar, int blocks, size_t smem, cudaStream_t st, const AlignArgs& a) {
-  if (a.wide_cell == 2) {
-    if (cigar)
-      wide_kernel<true, kModel, uint16_t><<<blocks, kWideThreads, smem, st>>>(a);
-    else
-      wide_kernel<false, kModel, uint16_t><<<blocks, kWideThreads, smem, st>>>(a);
-  } else {
-    if (cigar)
-      wide_kernel<true, kModel, uint32_t><<<blocks, kWideThreads, smem, st>>>(a);
-    else
-      wide_kernel<false, kModel, uint32_t><<<blocks, kWideThreads, smem, st>>>(a);
+template <bool kCigar, int kModel, typename ST>
+void wide_one(int blocks, int cluster, size_t smem, cudaStream_t st, const AlignArgs& a) {
+  if (cluster <= 1) {
+    wide_kernel<kCigar, kModel, ST><<<blocks, kWideThreads, smem, st>>>(a);
+    return;
   }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3(kWideThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)cluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, wide_kernel<kCigar, kModel, ST, true>, a);
+}
+
+// blocks: of all clusters together
+template <int kModel>
+void wide(bool cigar, int blocks, int cluster, size_t smem, cudaStream_t st, const AlignArgs& a) {
+  if (a.wide_cell == 2)
+    cigar ? wide_one<true, kModel, uint16_t>(blocks, cluster, smem, st, a)
+          : wide_one<false, kModel, uint16_t>(blocks, cluster, smem, st, a);
+  else
+    cigar ? wide_one<true, kModel, uint32_t>(blocks, cluster, smem, st, a)
+          : wide_one<false, kModel, uint32_t>(blocks, cluster, smem, st, a);
 }
 
 template <bool kCigar, int kMode, int GW, int kModel>

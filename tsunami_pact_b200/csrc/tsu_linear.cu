@@ -24,8 +24,8 @@ void launch_probe_linear(bool wide, int blocks, int threads, size_t smem, cudaSt
   launch_detail::probe<kModelLinear>(wide, blocks, threads, smem, st, a);
 }
 
-void launch_wide_linear(bool cigar, int blocks, size_t smem, cudaStream_t st, const AlignArgs& a) {
-  launch_detail::wide<kModelLinear>(cigar, blocks, smem, st, a);
+void launch_wide_linear(bool cigar, int blocks, int cluster, size_t smem, cudaStream_t st, const AlignArgs& a) {
+  launch_detail::wide<kModelLinear>(cigar, blocks, cluster, smem, st, a);
 }
 
 }  // namespace tsu

@@ -44,6 +44,7 @@
 
 #include "tsu_common.cuh"
 #include "tsu_extend.cuh"
+#include "tsu_half2.cuh"
 
 namespace tsu {
 
@@ -56,49 +57,6 @@ constexpr uint32_t kZeroPlain = 32768u, kZeroBound = 24576u;
 static_assert(2 * kPackedMaxW <= kZeroBound && kZeroPlain + 2 * kPackedPlainLen + 32 <= 65535 &&
                   kZeroBound + 2 * kPackedMaxLen + 32 <= 65535,
               "16-bit offsets");
-
-// ---- halfword pairs ------------------------------------------------------
-#ifdef TSU_WARP_EMU
-template <class F>
-inline uint32_t h2_each(uint32_t a, uint32_t b, uint32_t c, F f) {
-  const uint16_t lo = f((uint16_t)a, (uint16_t)b, (uint16_t)c);
-  const uint16_t hi = f((uint16_t)(a >> 16), (uint16_t)(b >> 16), (uint16_t)(c >> 16));
-  return (uint32_t)lo | ((uint32_t)hi << 16);
-}
-inline uint32_t h2_addmax(uint32_t a, uint32_t b, uint32_t c) {
-  return h2_each(a, b, c, [](uint16_t x, uint16_t y, uint16_t z) { return std::max<uint16_t>((uint16_t)(x + y), z); });
-}
-inline uint32_t h2_addmin(uint32_t a, uint32_t b, uint32_t c) {
-  return h2_each(a, b, c, [](uint16_t x, uint16_t y, uint16_t z) { return std::min<uint16_t>((uint16_t)(x + y), z); });
-}
-inline uint32_t h2_max(uint32_t a, uint32_t b) { return h2_addmax(a, 0, b); }
-inline uint32_t h2_min(uint32_t a, uint32_t b) { return h2_addmin(a, 0, b); }
-inline uint32_t h2_next(uint32_t a, uint32_t b) { return (a >> 16) | (b << 16); }
-inline uint32_t h2_signmask(uint32_t a) { return ((a & 0x8000u) ? 0xffffu : 0u) | ((a & 0x80000000u) ? 0xffff0000u : 0u); }
-inline int h2_tz(uint32_t d) { return d ? __builtin_ctz(d) : 32; }
-inline uint32_t h2_sum(uint32_t a, uint32_t acc) { return acc + (a & 0xffffu) + (a >> 16); }
-#else
-// max(a + b, c), min(a + b, c) per halfword, the sum modulo 2^16
-__device__ __forceinline__ uint32_t h2_addmax(uint32_t a, uint32_t b, uint32_t c) { return __viaddmax_u16x2(a, b, c); }
-__device__ __forceinline__ uint32_t h2_addmin(uint32_t a, uint32_t b, uint32_t c) { return __viaddmin_u16x2(a, b, c); }
-__device__ __forceinline__ uint32_t h2_max(uint32_t a, uint32_t b) { return __vmaxu2(a, b); }
-__device__ __forceinline__ uint32_t h2_min(uint32_t a, uint32_t b) { return __vminu2(a, b); }
-// (high half of a, low half of b)
-__device__ __forceinline__ uint32_t h2_next(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x5432); }
-// 0xffff in each half whose bit 15 is set (prmt replicates the sign of bytes 1 and 3)
-__device__ __forceinline__ uint32_t h2_signmask(uint32_t a) {
-  uint32_t r;
-  asm("prmt.b32 %0, %1, %1, 0xbb99;" : "=r"(r) : "r"(a));
-  return r;
-}
-// trailing zero bits, 32 for 0
-__device__ __forceinline__ int h2_tz(uint32_t d) { return __clz((int)__brev(d)); }
-// acc + both halves (below 2^15 each)
-__device__ __forceinline__ uint32_t h2_sum(uint32_t a, uint32_t acc) {
-  return (uint32_t)__dp2a_lo((int)a, 0x0101, (int)acc);
-}
-#endif
-__device__ __forceinline__ uint32_t h2_dup(uint32_t v) { return (v & 0xffffu) * 0x10001u; }
 
 // ---- shared memory by byte address --------------------------------------------
 // One address register per group, taken once: accesses are a register and a
@@ -452,6 +410,15 @@ __device__ __forceinline__ int warp_lcp(smem_t pw, int v, smem_t tw, int h, int 
   return rem;
 }
 
+template <class T>
+__device__ __forceinline__ T ld_l2(const T* p) {
+#ifdef TSU_WARP_EMU
+  return *p;
+#else
+  return __ldcg(p);
+#endif
+}
+
 // The CIGAR of a finished pair, by one warp.  First the walk: from the end
 // (s_end, k_fin) along the source bits to score 0, 32 scores of history in
 // registers at a time (lane l holds score top - l: 16 diagonals around the
@@ -483,10 +450,11 @@ __device__ __forceinline__ int packed_cigar(const uint32_t* hist, int64_t hist_c
       c0 = (pos - (1 << kCS)) >> (kCS + 1);
       d0 = d1 = 0;
       if (s - lane > 0) {
-        const int2 te = table[s - lane];
+        // (past L1: the blocks of a cluster write one history)
+        const int2 te = ld_l2(table + s - lane);
         const int64_t i = (int64_t)te.y + c0 - te.x;
-        if (i >= 0 && i < hist_chunks) d0 = hist[i];
-        if (i + 1 >= 0 && i + 1 < hist_chunks) d1 = hist[i + 1];
+        if (i >= 0 && i < hist_chunks) d0 = ld_l2(hist + i);
+        if (i + 1 >= 0 && i + 1 < hist_chunks) d1 = ld_l2(hist + i + 1);
       }
     }
     const uint32_t word = __shfl_sync(FULL, ch == c0 ? d0 : d1, top - s);

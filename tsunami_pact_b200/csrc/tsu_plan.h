@@ -38,6 +38,7 @@ struct PassGeom {
   int64_t ckpt_bytes = 0;  // bytes per checkpoint
   bool bounded = false;    // pairs with score bounds (plan_bounded, plan_wide)
   int wide_cell = 0;       // of these, the wide kernel's: bytes of a ring cell (2 or 4)
+  int cluster = 1;         // blocks per pair (wide kernel)
 };
 
 constexpr int kSharedW1 = 384;         // shared-mode ring width for one warp per pair (diagonals)
@@ -374,6 +375,13 @@ inline PassGeom plan_wide(const Pen& pen, int32_t max_n, int width, int32_t max_
     p.hist_cap = hist;
   }
   return p;
+}
+// Blocks per pair of a wide launch of n pairs (a cluster): as many as keep
+// the clusters within 7 of every 8 SMs (a GPC's SMs rarely divide evenly).
+inline int wide_cluster(int64_t n, int sms) {
+  int c = 1;
+  while (c < 8 && n * c * 2 <= (int64_t)sms * 7 / 8) c *= 2;
+  return c;
 }
 // Cells of history a wide launch may keep (32-bit words below 2^31).
 constexpr int64_t kWideMaxHist = INT32_MAX - 65536;

@@ -7,7 +7,8 @@
 // 16 warps, rows of h + 1 (0: absent) in 16 bits for texts of up to 65,532
 // bases and 32 bits for longer ones.  What bounds it is the ring's L2 traffic
 // (five loads and three stores per cell), so 16-bit rows halve the time of the
-// widest scores, and U = 4 cells per lane are in flight to cover its latency.
+// widest scores, and U = 4 cells per lane are in flight to cover its latency; few pairs are
+// spread over clusters of up to 8 blocks.
 // The sequences are read through L1 (a few neighbouring words per warp).
 #pragma once
 
@@ -30,7 +31,16 @@ struct WidePair {
 // I, D and M of U diagonals (positions w[u] of the window) from the source
 // rows into the score's rows.  m1: M as h + 1 (0: absent); bits: source bits
 // as packed_words_step's; ext: bases matched.
-template <int kModel, typename ST, int U>
+// kL2: read the ring past L1 (other blocks of the cluster write it).
+template <bool kL2, typename ST>
+__device__ __forceinline__ uint32_t wide_ld(const ST* p) {
+#ifndef TSU_WARP_EMU
+  if constexpr (kL2) return (uint32_t)__ldcg(p);
+#endif
+  return (uint32_t)*p;
+}
+
+template <int kModel, typename ST, int U, bool kL2>
 __device__ __forceinline__ void wide_cells(unsigned char* base, const PackedRows& r, const WidePair& q, const int (&w)[U],
                                            uint32_t (&m1)[U], uint32_t (&bits)[U], uint32_t (&ext)[U]) {
   constexpr bool kDual = kModel == kModelDual, kLin = kModel == kModelLinear;
@@ -38,20 +48,19 @@ __device__ __forceinline__ void wide_cells(unsigned char* base, const PackedRows
   uint32_t mo_l[U], mo_r[U], mx[U], ie[U], de[U], mo2_l[U], mo2_r[U], ie2[U], de2[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    const ST* mo = wide_row<ST>(base, r.r_mo);
-    mo_l[u] = mo[w[u] - 1];
-    mo_r[u] = mo[w[u] + 1];
-    mx[u] = wide_row<ST>(base, r.r_mx)[w[u]];
+    auto ld = [&](int row, int at) -> uint32_t { return wide_ld<kL2, ST>(wide_row<ST>(base, row) + at); };
+    mo_l[u] = ld(r.r_mo, w[u] - 1);
+    mo_r[u] = ld(r.r_mo, w[u] + 1);
+    mx[u] = ld(r.r_mx, w[u]);
     if constexpr (!kLin) {
-      ie[u] = wide_row<ST>(base, r.r_ie)[w[u] - 1];
-      de[u] = wide_row<ST>(base, r.r_de)[w[u] + 1];
+      ie[u] = ld(r.r_ie, w[u] - 1);
+      de[u] = ld(r.r_de, w[u] + 1);
     }
     if constexpr (kDual) {
-      const ST* mo2 = wide_row<ST>(base, r.r_mo2);
-      mo2_l[u] = mo2[w[u] - 1];
-      mo2_r[u] = mo2[w[u] + 1];
-      ie2[u] = wide_row<ST>(base, r.r_ie2)[w[u] - 1];
-      de2[u] = wide_row<ST>(base, r.r_de2)[w[u] + 1];
+      mo2_l[u] = ld(r.r_mo2, w[u] - 1);
+      mo2_r[u] = ld(r.r_mo2, w[u] + 1);
+      ie2[u] = ld(r.r_ie2, w[u] - 1);
+      de2[u] = ld(r.r_de2, w[u] + 1);
     }
   }
   // twice h + 1, bit 0 set by the side that wins ties; 0 and 1: absent
@@ -134,25 +143,79 @@ __device__ __forceinline__ int wide_warp_lcp(const WidePair& q, int v, int h, in
   return rem;
 }
 
+// The blocks of a cluster that share a pair.
+#ifdef TSU_WARP_EMU
+inline unsigned cluster_size() { return 1; }
+inline unsigned cluster_rank() { return 0; }
+inline void cluster_sync() {}
+inline void cluster_sts32(smem_t a, unsigned, uint32_t v) { sts32(a, v); }
+#else
+__device__ __forceinline__ unsigned cluster_size() {
+  unsigned v;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(v));
+  return v;
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned v;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
+  return v;
+}
+// Every thread of every block of the cluster; what they wrote before it
+// (shared and global memory) is visible after it.
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Store to the same shared memory address in block `rank` of the cluster.
+__device__ __forceinline__ void cluster_sts32(smem_t a, unsigned rank, uint32_t v) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(r), "r"(v) : "memory");
+}
+#endif
+
 // Scores (and CIGARs) of pairs with score bounds (a.bound), end to end, one
-// block per pair; a.ring_global, a.ring_stride (int32): the ring.
-template <bool kCigar, int kModel, typename ST>
+// block per pair, or one cluster of blocks (kCluster); a.ring_global,
+// a.ring_stride (int32): the ring.  A step of a 50 kbp pair at 20 % (16,000
+// cells) is 6 us of issue slots on one SM, and few pairs are that long: with a
+// cluster each block computes every csize-th run of words of a score, reads
+// the ring past L1, and a cluster barrier ends the score (11 pairs of 21 - 50
+// kbp: 201 ms one block each, 78 ms on clusters of 8).
+template <bool kCigar, int kModel, typename ST, bool kCluster>
 __device__ __forceinline__ void align_wide(const AlignArgs& a, unsigned char* smem_raw) {
   constexpr unsigned FULL = 0xffffffffu;
-  constexpr int GW = 16, GT = 32 * GW, U = 4;
+  constexpr int GW = 16, U = 4;
+  const int csize = kCluster ? (int)cluster_size() : 1, crank = kCluster ? (int)cluster_rank() : 0;
+  const int GT = 32 * GW * csize;  // threads per pair
+  auto sync = [&]() {
+    if constexpr (kCluster)
+      cluster_sync();
+    else
+      group_sync<GW>(0);
+  };
+  // a word of every block's shared memory
+  auto tell = [&](smem_t at, uint32_t v) {
+    if constexpr (kCluster) {
+      for (int c = 0; c < csize; ++c) cluster_sts32(at, (unsigned)c, v);
+    } else {
+      sts32(at, v);
+    }
+  };
   constexpr bool kDual = kModel == kModelDual;
   constexpr int kCS = kDual ? 1 : 2;  // log2 of pairs of diagonals per 32-bit history chunk
-  const int gt = threadIdx.x, lane = gt & 31, wig = gt >> 5;
+  const int gt = threadIdx.x + 32 * GW * crank, lane = gt & 31, wig = gt >> 5;  // in the pair's threads
+  const int64_t grp = blockIdx.x / csize;
   const int rows = a.pen.slots() + 1;
   const smem_t bc = smem_addr(smem_raw);  // broadcast words: queue, end flag
   const smem_t tables = bc + packed_head_bytes(Pen(), GW);
-  unsigned char* const ring = reinterpret_cast<unsigned char*>(a.ring_global + (int64_t)blockIdx.x * a.ring_stride);
-  uint32_t* const hist = kCigar ? a.hist + (int64_t)blockIdx.x * a.hist_cap : nullptr;
+  unsigned char* const ring = reinterpret_cast<unsigned char*>(a.ring_global + grp * a.ring_stride);
+  uint32_t* const hist = kCigar ? a.hist + grp * a.hist_cap : nullptr;
   const int hist_cap = (int)a.hist_cap;
-  int2* const table = kCigar ? a.table + (int64_t)blockIdx.x * a.table_cap : nullptr;
+  int2* const table = kCigar ? a.table + grp * (int64_t)a.table_cap : nullptr;
+  if constexpr (kCluster) cluster_sync();  // every block runs before another stores into it
   for (;;) {
-    if (gt == 0) sts32(bc, atomicAdd(a.queue, 1u));
-    group_sync<GW>(0);
+    if (gt == 0) tell(bc, atomicAdd(a.queue, 1u));
+    sync();
     const unsigned qi = lds32(bc);
     if ((int64_t)qi >= a.n_order) break;
     const int64_t pair = a.order[qi];
@@ -173,21 +236,21 @@ __device__ __forceinline__ void align_wide(const AlignArgs& a, unsigned char* sm
       const WidePair q{reinterpret_cast<const uint32_t*>(a.pk.words + a.pk.woff[pair]),
                        reinterpret_cast<const uint32_t*>(a.pk.words + a.pk.woff[a.seq.n + pair]), m, n, kbase};
       unsigned char* const ring0 = ring + 4 * sizeof(ST);  // position 0 of row 0
-      packed_tables<kDual>(a.pen, RB, tables, gt, GT);
+      packed_tables<kDual>(a.pen, RB, tables, (int)threadIdx.x, 32 * GW);
       {
         uint32_t* const z = reinterpret_cast<uint32_t*>(ring);
         const int words = rows * RB / 4;
         for (int i = gt; i < words; i += GT) z[i] = 0u;
       }
-      group_sync<GW>(0);
+      sync();
       if (wig == 0) {
         const int l = wide_warp_lcp(q, 0, 0, min(m, n), lane);
         if (lane == 0) {
           wide_row<ST>(ring0, 0)[-kbase] = (ST)(l + 1);
-          sts32(bc + 4, l >= n && k_end == 0 ? 0u : 0xffffffffu);  // the score that ended, none yet
+          tell(bc + 4, l >= n && k_end == 0 ? 0u : 0xffffffffu);  // the score that ended, none yet
         }
       }
-      group_sync<GW>(0);
+      sync();
       n_cells = 1;
       if (lds32(bc + 4) == 0) s_end = 0;
       const int64_t bound = score_bound(m, n, a.pen);
@@ -244,12 +307,12 @@ __device__ __forceinline__ void align_wide(const AlignArgs& a, unsigned char* sm
           uint32_t m1[U], f[U], ext[U];
 #pragma unroll
           for (int u = 0; u < U; ++u) w[u] = min(w0 + u * GT + lane, whi);
-          wide_cells<kModel, ST, U>(ring0, r, q, w, m1, f, ext);
+          wide_cells<kModel, ST, U, kCluster>(ring0, r, q, w, m1, f, ext);
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const bool own = w0 + u * GT + lane <= whi;
             if (own) n_ext += ext[u];
-            if (w[u] == pend && m1[u] >= end_val) sts32(bc + 4, (uint32_t)s);
+            if (w[u] == pend && m1[u] >= end_val) tell(bc + 4, (uint32_t)s);
             if constexpr (kCigar) {
               if constexpr (kDual) {
                 if (own) hrow[w[u]] = (uint8_t)f[u];
@@ -261,7 +324,7 @@ __device__ __forceinline__ void align_wide(const AlignArgs& a, unsigned char* sm
           }
         }
         n_cells += (unsigned)(hi - lo + 1);
-        group_sync<GW>(0);
+        sync();
         if (lds32(bc + 4) == (uint32_t)s) s_end = s;
       }
       n_steps += (uint32_t)s + (st == kPairOk ? 1u : 0u);
@@ -309,7 +372,7 @@ __device__ __forceinline__ void align_wide(const AlignArgs& a, unsigned char* sm
         atomicAdd(a.work + 1, (unsigned long long)n_steps);
       }
     }
-    group_sync<GW>(0);  // the block's ring and flags are free for the next pair
+    sync();  // the block's ring and flags are free for the next pair
   }
 }
 
@@ -363,7 +426,7 @@ __device__ __forceinline__ void probe_wide(const ProbeArgs& a, unsigned char* sm
         uint32_t m1[U], f[U], ext[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) w[u] = min(wlo + 32 * u + lane, whi);
-        wide_cells<kModel, uint32_t, U>(ring0, r, q, w, m1, f, ext);
+        wide_cells<kModel, uint32_t, U, false>(ring0, r, q, w, m1, f, ext);
         __syncwarp();
         const int pend = k_end - q.kbase;
         if (pend >= wlo && pend <= whi && wide_row<uint32_t>(ring0, r.w_m)[pend] >= (uint32_t)n + 1u) found = s;
