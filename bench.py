@@ -661,14 +661,13 @@ def measure(args, workload, rank, world, local, dist, with_plain, with_cpu, e2e_
 
 # Integer-issue model of the align kernel (see the kernel roofline section of
 # the design notes): the fewest thread instructions the algorithm as written
-# needs per (score, diagonal) cell (five ring loads, the I/D/M maxima and
-# source bits, the bounds test, one 16-base extend window, the end test, the
-# trimming bounds, three ring stores with their int16 clamps, the history
-# word, the loop), per further 16-base extend window, and the warp
-# instructions of one score step of a pair (source limits, envelope, seven
-# warp reductions, limit stores, step table) and of one CIGAR run of the
-# backtrace walk (one lane).
-C_CELL, C_EXT, C_STEP, C_RUN = 76, 16, 70, 24
+# needs per (score, diagonal) cell, half of those of a word of two diagonals
+# (8 ring loads, 4 halfword selects, 9 maxima with their source bits, 6 clamps,
+# 28 for two 16-base windows of both sequences, 6 to count the matches, 6 to
+# combine them, 3 stores, 8 for the history bits), per further 16-base extend
+# window, and the warp instructions of one score step of a pair (rows, range,
+# limits, step table, end test) and of one CIGAR run (walk and replay).
+C_CELL, C_EXT, C_STEP, C_RUN = 39, 16, 60, 60
 
 
 def roofline(workload, n_pairs, plen, tlen, nruns, work_cells, work_steps, ext_bases, a_ms, clk, want_cigar,
@@ -678,8 +677,8 @@ def roofline(workload, n_pairs, plen, tlen, nruns, work_cells, work_steps, ext_b
     algorithmic warp instructions (the model above times the counted cells,
     extension bases, steps and runs) per second against 148 SMs x 4
     schedulers x the sampled SM clock.  Secondary: HBM, algorithmic bytes
-    (packed input, scores, CIGAR runs, one 4-byte backtrace word per
-    wavefront cell) per second against the measured copy bandwidth, with the
+    (packed input, scores, CIGAR runs, 4 bits of history per wavefront
+    cell; 8 with two gap pieces) per second against the measured copy bandwidth, with the
     DRAM traffic of an ncu capture of the same kernel scaled by pairs."""
     import torch
 
@@ -695,7 +694,7 @@ def roofline(workload, n_pairs, plen, tlen, nruns, work_cells, work_steps, ext_b
     words = float(np.sum((plen.astype(np.int64) + 31) // 32 + 1) + np.sum((tlen.astype(np.int64) + 31) // 32 + 1))
     packed_in = words * 8
     out_bytes = n_pairs * 4 + 4 * nruns
-    hist_bytes = 4 * work_cells if want_cigar else 0
+    hist_bytes = work_cells * (1.0 if len(PEN) == 5 else 0.5) if want_cigar else 0
     algo = packed_in + out_bytes + hist_bytes
     achieved = algo / (a_ms / 1e3) / 1e9
     model = "_" + METRIC_NAME if METRIC_NAME else ("_dual" if len(PEN) == 5 else "")

@@ -1,5 +1,9 @@
 // tsu_align.cuh -- the persistent gap-affine WFA kernel.
 //
+// align_kernel in shared mode is align_packed (tsu_packed.cuh: two diagonals
+// per thread), except for low-memory CIGARs; those and global mode are
+// align_ring, described here.
+//
 // Re-design of the reference kernel wfa_dispatcher (wfa_gpu.cu:191-722):
 //   * persistent grid; each group of GW warps pulls pairs from a device work
 //     queue (the reference launched one 32-thread block per pair,
@@ -14,8 +18,8 @@
 //     and, with kCigar, streams one backtrace word per (score, diagonal) to
 //     HBM; the ends of M, I and D are trimmed with warp min/max reductions
 //     combined across the group's warps (wfa_gpu.cu:636-719);
-//   * kModeShared: the ring of the last max(x, o+e)+1 scores is int16 in
-//     shared memory (offsets clamped to [null, n+1], which changes no valid
+//   * kModeShared (low-memory CIGARs): the ring of the last max(x, o+e)+1
+//     scores is int16 in shared memory (offsets clamped to [null, n+1], which changes no valid
 //     cell: validity depends only on the value and the diagonal, so a clamped
 //     out-of-bounds candidate still loses every max to -- or stays invalid
 //     against -- any valid one) and the pair's packed sequences are staged

@@ -1588,8 +1588,9 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     }
     // The launches run side by side, each in its own part of the scratch, so
     // that one class's last pairs and the next one's first share the SMs; one
-    // after the other when the budget does not hold them all at once.
-    const bool side = runs.size() - first > 1 && each <= avail;
+    // after the other when the budget does not hold them all at once, or the
+    // context keeps to one stream (the request server's workers).
+    const bool side = runs.size() - first > 1 && each <= avail && ctx->h2d_stream != ctx->stream;
     if (side) need_bytes = each;
     if (need_bytes > ctx->b_scratch.cap) {
       release(ctx, ctx->b_scratch);

@@ -7,12 +7,13 @@
 // scheduler; ncu: 75 % busy in the one-diagonal form), so the layout is
 // chosen to spend few ALU instructions per cell:
 //   * an offset h is held as 2 h + kZero: an absent cell is any halfword below
-//     it, and bit 0 is free.  A candidate enters a
-//     maximum with bit 0 set when it wins ties, so one add-max both takes the
-//     maximum and records which side won; I, D and M of two cells take nine
-//     such instructions with all their source bits;
+//     kZero, and bit 0 is free.  A candidate enters a maximum with bit 0 set
+//     when it wins ties, so one add-max both takes the maximum and records
+//     which side won; I, D and M of two cells take nine such instructions with
+//     all their source bits;
 //   * absent cells stay below kZero: M rows store absent as 0, I climbs by 2
-//     per diagonal it moves, at most 2 ring_w < kZero;
+//     per diagonal it moves, at most 2 ring_w <= kZero (an I past the matrix
+//     edge may wrap past 2^16 to absent, and climbs from there);
 //   * every row has the same diagonal-to-position map (position = k - kbase)
 //     and is all absent before its first write, so no read needs a range
 //     test; a source row that does not exist at this score is a permanent
@@ -36,8 +37,11 @@
 // gap-affine on 8 warps 42.5 -> 15.4 ms.  A cell pair takes 75 warp
 // instructions scored (90 with history) and a step 145, against 175 per 32
 // cells before; issue slots are 86 % and the ALU pipe 68 % busy.
-// Limits: sides of at most kPackedMaxLen bases, ACGT only, at most 64 score
-// steps of ring depth; other pairs go to the global ring (tsu_align.cuh).
+// Within a score bound (kBound): 1,000 x 10 kbp at 15 % 50.5 -> 27.1 ms with
+// the probe, on 8 warps; two words per lane 32.0 -> 25.2 ms without it.
+// Limits: sides of at most kPackedPlainLen bases (kPackedMaxLen with a bound),
+// ACGT only, at most 64 score steps of ring depth; other pairs go to
+// tsu_wide.cuh (with a bound) or the global ring (tsu_align.cuh).
 #pragma once
 
 #include <type_traits>
@@ -386,12 +390,6 @@ struct PackedSteps {
   }
 };
 
-// Bytes of history per pair of diagonals.
-template <bool kDual>
-constexpr int hist_pair_bytes() {
-  return kDual ? 2 : 1;
-}
-
 // Longest common prefix of pattern[v..] and text[h..], at most rem, by a
 // whole warp: 512 bases per comparison.
 __device__ __forceinline__ int warp_lcp(smem_t pw, int v, smem_t tw, int h, int rem, int lane) {
@@ -558,7 +556,6 @@ __device__ __forceinline__ void align_packed(const AlignArgs& a, unsigned char* 
   constexpr int GT = 32 * GW;
   constexpr uint32_t kZero = kBound ? kZeroBound : kZeroPlain;
   constexpr int kMaxLen = kBound ? kPackedMaxLen : kPackedPlainLen;
-  constexpr int kHB = hist_pair_bytes<kDual>();
   constexpr int kCS = kDual ? 1 : 2;  // log2 of diagonal pairs per 32-bit history chunk
   const int tid = threadIdx.x;
   const int gid = tid / GT;

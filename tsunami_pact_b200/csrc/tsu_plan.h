@@ -337,12 +337,14 @@ inline int bound_class(int pairs_per_sm) {
   return c;
 }
 
-// Warps per pair of a bounded launch of n pairs: the fewest that keep 16 warps
-// on an SM with the pairs its shared memory holds (a step costs every warp of
-// a group the same bookkeeping, so fewer warps do less work: 4,000 x 2 kbp at
-// 5 % took 1.7 ms on 2 warps, 2.3 on 4, 2.7 on 8), and as many as fill 8 per
-// SM when there are few pairs (148 x 1 kbp: 0.21 ms on 1 warp, 0.15 on 4 to
-// 16; 600: 0.19 on 2, 0.26 on 4).  0: the ring does not fit a block.
+// Warps per pair of a bounded launch of n pairs whose shared memory is
+// `bytes`: the fewest that keep 16 warps on an SM with the pairs it holds, and
+// as many as fill 8 per SM when there are few pairs.  A step costs every warp
+// of a group the same bookkeeping, so fewer warps do less work; below 16 they
+// no longer cover the latency of a step (1,000 x 10 kbp at 15 % and 8,000
+// uneven pairs, align ms, with at least 8: 31.5 and 42.1, 12: 27.0 and 38.3,
+// 16: 27.1 and 38.5, 20: 38.1 and 47.1; 20,000 x 1 kbp dual gap-affine 8.7,
+// 8.6, 8.5, 12.4).  0: the bytes do not fit a block.
 inline int bounded_warps(int bytes, int64_t n, int sms, int smem_optin, int* pairs_per_sm = nullptr) {
   int best = 0;
   for (int gw = 1; gw <= 16; gw *= 2) {
