@@ -1313,16 +1313,19 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   };
   std::vector<int32_t> probed;
   ProbePlan probe;
+  int32_t few_side = INT32_MAX;  // sides from which few pairs get a bound when they outgrow a ring
   if (can_bound) {
-    tsu::BoundLimits limits = tsu::bound_limits(ctx->rp);
+    tsu::BoundLimits limits = tsu::bound_limits(ctx->rp, ctx->smem_optin);
     if (low_mem) limits.side = std::min(limits.side, tsu::kBoundLowMemLen);
     if (bi.max_side >= limits.side || bi.max_sum >= limits.sum)
       for (int64_t i = 0; i < n; ++i)
         if (limits.wants(h_plen[i], h_tlen[i])) probed.push_back((int32_t)i);
-    if ((int64_t)probed.size() <= ctx->sms && !low_mem)
+    if ((int64_t)probed.size() <= ctx->sms && !low_mem) {
+      few_side = limits.few_side;
       probed.erase(std::remove_if(probed.begin(), probed.end(),
-                                  [&](int32_t i) { return std::max(h_plen[i], h_tlen[i]) < tsu::kBoundFewLen; }),
+                                  [&](int32_t i) { return std::max(h_plen[i], h_tlen[i]) <= tsu::kPackedBandLen; }),
                    probed.end());
+    }
     if ((rc = plan_probes(&probed, &probe))) return rc;
     if (!probed.empty() && (rc = grow(ctx, ctx->b_bound, sizeof(int32_t) * n))) return rc;
   }
@@ -1363,6 +1366,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     tsu::PassChoice pc;
     double hint = 0;
     Pass ps;
+    bool few = false;      // few long pairs: those that outgrow it get a bound
     bool rebound = false;  // the pairs that outgrew it have run again with bounds
   };
   BandSplit split;
@@ -1408,6 +1412,8 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       r.hint = ctx->err_hint;
       if (ctx->fit_start && !ctx->one_warp)
         r.pc = tsu::fit_start(r.pc, ctx->rp, r.bi.max_m, r.bi.max_n, r.hint, ctx->smem_optin);
+      r.few = r.n <= ctx->sms && std::max(r.bi.max_m, r.bi.max_n) >= few_side;
+      if (r.few) r.pc = tsu::few_start(r.pc, ctx->rp, std::max(r.bi.max_m, r.bi.max_n));
       if (!ctx->one_warp) r.pc = tsu::fill_warps(r.pc, r.n, std::max(r.bi.max_m, r.bi.max_n), ctx->sms);
       if ((rc = plan_pass_within(ctx, r.bi, r.n, r.pc, r.hint, want_cigar, avail, &r.ps))) return rc;
       need = std::max(need, scratch_bytes(r.ps, want_cigar));
@@ -1714,7 +1720,8 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   }
   // Pairs that outgrew an unbounded shared ring get a bound, and a second
   // start with it: 20,000 pairs of 800 - 1,000 bp at 10 % took 13.2 ms through
-  // the ladder.  (Few of them: the ladder's 16 warps are as good.)
+  // the ladder.  (Few of them, whose full wavefronts fit 16 warps' ring: the
+  // ladder's 16 warps are as good.)
   bool rebound_any = false;
   if (can_bound) {
     std::vector<int32_t> again;
@@ -1730,7 +1737,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       const size_t before = again.size();
       for (unsigned int i = 0; i < c; ++i)
         if (std::min(h_plen[l[i]], h_tlen[l[i]]) > 0) again.push_back(l[i]);
-      if (again.size() - before == c && c > (unsigned)ctx->sms)
+      if (again.size() - before == c && (r.few || c > (unsigned)ctx->sms))
         r.rebound = true;  // all of them
       else
         again.resize(before);

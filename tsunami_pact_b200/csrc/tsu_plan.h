@@ -261,30 +261,39 @@ constexpr int kBoundMinRing = 14 << 10;
 // once per call.)
 struct BoundLimits {
   int32_t side = INT32_MAX, sum = INT32_MAX;
+  int32_t few_side = INT32_MAX;  // the longer side from which few pairs get a bound (below)
   bool wants(int32_t m, int32_t n) const {
     return std::min(m, n) > 0 && (std::max(m, n) >= side || m + n >= sum);
   }
 };
-inline BoundLimits bound_limits(const Pen& pen) {
+// With no more such pairs than SMs each has an SM to itself, and a probe (0.35
+// us per score on one warp) costs more than the narrower search saves until a
+// pair outgrows the widest shared ring (148 x 8 kbp at 10 %: 3.1 ms either
+// way; 100 of 12 kbp at 1 %: 0.53 ms without, 0.88 with): they start in that
+// ring, and those that outgrow it get a bound when their full wavefronts at
+// 16 % edits do not fit it anyway (few_side; gap-affine 4/6/2: from 8.2 kbp;
+// 4/6/2/24/1, whose 37 rows leave 2,900 diagonals: from 1.1 kbp).  Only sides
+// beyond that ring's offsets (kPackedBandLen) are probed at once.
+inline BoundLimits bound_limits(const Pen& pen, int smem_optin) {
   BoundLimits b;
-  int32_t lo = 0, hi = 1 << 27;  // the shortest side whose expected width reaches kBoundMinWidth
-  while (lo < hi) {
-    const int32_t L = lo + (hi - lo) / 2;
-    if (2 * hint_score(pen, L, 0.04) / pen.min_ge() >= kBoundMinWidth)
-      hi = L;
-    else
-      lo = L + 1;
-  }
-  b.side = lo;
+  // the shortest side whose expected width at `rate` edits reaches `width`
+  auto from = [&](int64_t width, double rate) -> int32_t {
+    int32_t lo = 0, hi = 1 << 27;
+    while (lo < hi) {
+      const int32_t L = lo + (hi - lo) / 2;
+      if (2 * hint_score(pen, L, rate) / pen.min_ge() >= width)
+        hi = L;
+      else
+        lo = L + 1;
+    }
+    return lo;
+  };
+  b.side = from(kBoundMinWidth, 0.04);
   const int64_t d = kBoundMinRing / (2 * ((int64_t)pen.slots() + 1)) + 1;  // diagonals that take more than kBoundMinRing
   if (d <= kSharedW1) b.sum = (int32_t)std::max<int64_t>(d - 3, 1);
+  b.few_side = from(std::max(shared_ring_width(pen, 16, kSharedSeqWordsN, smem_optin), 64), 0.163);
   return b;
 }
-// With no more such pairs than SMs each has an SM to itself, and a probe (0.35
-// us per score on one warp) adds what the narrower search saves (148 x 8 kbp
-// at 10 %: 3.1 ms either way; one 8 kbp pair at 1 %: 0.56 ms without, 0.60
-// with): only pairs that may not fit the widest shared ring at all are probed.
-constexpr int kBoundFewLen = 8192;
 
 // What a pair of score bound ub needs: diagonals of the ring's window,
 // 32-bit sequence words, and 32-bit history words (each side of the band grows
@@ -393,6 +402,20 @@ constexpr int64_t kWideMaxHist = INT32_MAX - 65536;
 // that narrows again, takes less than the checkpoints and recomputed segment
 // planned from the error hint, and is computed once.
 constexpr int kBoundLowMemLen = 256;
+
+// First launch of no more pairs than SMs whose length starts in the global
+// ring: the widest shared ring instead, as far as its offsets reach; the ones
+// that outgrow it get a bound.  Measured on one B200, 100 pairs each, global
+// ring / probe at once / this: gap-affine 4/6/2 of 12 kbp at 1 % 0.97 / 0.88 /
+// 0.53 ms, at 5 % 5.2 / 3.0 / 2.4, at 15 % 23 / 9.4 / 10.4; 4/6/2/24/1 of 1.2
+// kbp at 4 % 0.83 / - / 0.39, of 2.5 kbp at 10 % 8.3 / 2.3 / 1.9, of 9 kbp at
+// 1 % 8.0 / 1.2 / 0.74, at 4 % 40 / 4.1 / 5.8.  (A rung that the caller set
+// stays.)
+inline PassChoice few_start(PassChoice pc, const Pen& pen, int32_t maxlen) {
+  const PassChoice d = band_start_in(band_start_table(pen.dual()), length_band(maxlen), maxlen);
+  if (pc.mode == kModeGlobal && pc.mode == d.mode && pc.gw == d.gw && maxlen <= kPackedBandLen) return {kModeShared, 16};
+  return pc;
+}
 
 // Warps per pair of an unbounded shared-ring launch of n pairs: 16 when each
 // pair can have an SM to itself (one pair of 1 kbp: 0.21 ms on 1 warp, 0.14 on
