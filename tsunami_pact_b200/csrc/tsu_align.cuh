@@ -248,7 +248,7 @@ __device__ __forceinline__ void align_ring(const AlignArgs& a, unsigned char* sm
         if (gt == 0) {
           const int rem = m < n ? m : n;
           const int32_t o0 =
-              (kMode == kModeGlobal && bytemode) ? lcp8(pb, m, 0, tb, n, 0, rem) : lcp16(P, 0, T, 0, rem);
+              (kMode == kModeGlobal && bytemode) ? lcp8(pb, 0, tb, 0, rem) : lcp16(P, 0, T, 0, rem);
           store(0, o0);
           s_lo[0] = 0;
           s_hi[0] = 0;
@@ -281,7 +281,7 @@ __device__ __forceinline__ void align_ring(const AlignArgs& a, unsigned char* sm
           const int vv = p0 - k;
           const int rem = min(m - vv, n - p0);
           const int32_t om =
-              p0 + ((kMode == kModeGlobal && bytemode) ? lcp8(pb, m, vv, tb, n, p0, rem) : lcp16(P, vv, T, p0, rem));
+              p0 + ((kMode == kModeGlobal && bytemode) ? lcp8(pb, vv, tb, p0, rem) : lcp16(P, vv, T, p0, rem));
           store(k - lo0, om);
           if (kCigar) hist[k - lo0] = (uint32_t)p0 << (kDual ? 8 : 4);
           const int ov = om - k;
@@ -516,7 +516,7 @@ __device__ __forceinline__ void align_ring(const AlignArgs& a, unsigned char* sm
               const int rem = vm ? min(m - vv, n - p) : 0;
               int lx;
               if (kMode == kModeGlobal && bytemode) {
-                lx = lcp8(pb, m, vv, tb, n, hh, rem);
+                lx = lcp8(pb, vv, tb, hh, rem);
               } else {
                 const uint32_t d0 = win16(P, vv) ^ win16(T, hh);
                 lx = d0 ? (__ffs(d0) - 1) >> 1 : 16;
@@ -535,7 +535,7 @@ __device__ __forceinline__ void align_ring(const AlignArgs& a, unsigned char* sm
             } else if (in_bounds(p, k, m, n)) {
               const int vv = p - k;
               const int rem = min(m - vv, n - p);
-              const int lx = (kMode == kModeGlobal && bytemode) ? lcp8(pb, m, vv, tb, n, p, rem) : lcp16(P, vv, T, p, rem);
+              const int lx = (kMode == kModeGlobal && bytemode) ? lcp8(pb, vv, tb, p, rem) : lcp16(P, vv, T, p, rem);
               om = p + lx;
               n_ext += (uint32_t)lx;
               fm = min(fm, k);

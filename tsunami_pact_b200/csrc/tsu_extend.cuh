@@ -51,31 +51,25 @@ __device__ __forceinline__ int lcp16(const S& pw, int v, const S& tw, int h, int
   return l < rem ? l : rem;
 }
 
-// Byte path for pairs with bytes outside ACGT: bounded byte loads, 8 per
-// window (no reads outside the caller's sequences).
-__device__ __forceinline__ uint64_t win8(const uint8_t* __restrict__ s, int len, int pos) {
-  uint64_t r = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int p = pos + i;
-    const uint64_t c = p < len ? (uint64_t)s[p] : 0ull;
-    r |= c << (8 * i);
-  }
-  return r;
-}
-
-__device__ __forceinline__ int lcp8(const uint8_t* __restrict__ p, int m, int v, const uint8_t* __restrict__ t, int n,
-                                    int h, int rem) {
+// Byte path for pairs with bytes outside ACGT: LCP of p[v..] and t[h..], at
+// most rem characters, 8 per step; reads only the rem bytes compared.  (The
+// windows were once built as 64-bit words of bytes guarded by the sequences'
+// lengths.  Compiled into the two-piece CIGAR kernels of 2 to 16 warps, that
+// form took the second window for different when it held the last 3 bases of
+// both sequences, one mismatch too many, and otherwise changed from run to
+// run; the same source was right in every other kernel and on the CPU.)
+__device__ __forceinline__ int lcp8(const uint8_t* __restrict__ p, int v, const uint8_t* __restrict__ t, int h, int rem) {
   int l = 0;
   while (l < rem) {
-    const uint64_t d = win8(p, m, v + l) ^ win8(t, n, h + l);
-    if (d) {
-      l += (__ffsll((long long)d) - 1) >> 3;
-      break;
-    }
+    const int c = rem - l;
+    int first = 8;  // the first of 8 that differ
+#pragma unroll
+    for (int i = 7; i >= 0; --i)
+      if (i < c && p[v + l + i] != t[h + l + i]) first = i;
+    if (first < 8) return l + first;
     l += 8;
   }
-  return l < rem ? l : rem;
+  return rem;
 }
 
 }  // namespace tsu
