@@ -1,8 +1,9 @@
 // tsu_align.cuh -- the persistent gap-affine WFA kernel.
 //
 // align_kernel in shared mode is align_packed (tsu_packed.cuh: two diagonals
-// per thread), except for low-memory CIGARs; those and global mode are
-// align_ring, described here.
+// per thread), except for low-memory CIGARs, rings deeper than 128 scores and
+// sides of 16,352 - 32,000 bases; those and global mode are align_ring,
+// described here.
 //
 // Re-design of the reference kernel wfa_dispatcher (wfa_gpu.cu:191-722):
 //   * persistent grid; each group of GW warps pulls pairs from a device work
@@ -18,7 +19,7 @@
 //     and, with kCigar, streams one backtrace word per (score, diagonal) to
 //     HBM; the ends of M, I and D are trimmed with warp min/max reductions
 //     combined across the group's warps (wfa_gpu.cu:636-719);
-//   * kModeShared (low-memory CIGARs): the ring of the last max(x, o+e)+1
+//   * kModeShared: the ring of the last max(x, o+e)+1
 //     scores is int16 in shared memory (offsets clamped to [null, n+1], which changes no valid
 //     cell: validity depends only on the value and the diagonal, so a clamped
 //     out-of-bounds candidate still loses every max to -- or stays invalid
@@ -82,7 +83,8 @@ constexpr int cta_min_blocks() {
   return kMode == kModeShared ? (GW == 1 ? 6 : (GW <= 4 ? 6 : (GW == 8 ? 3 : 1))) : (GW <= 4 ? 4 : (GW == 8 ? 2 : 1));
 }
 
-// The body of align_kernel for the global ring and for low-memory CIGARs.
+// The body of align_kernel for the global ring, for low-memory CIGARs and for
+// shared rings beyond align_packed's (kSingleFlag).
 template <bool kCigar, int kMode, int GW, int kModel>
 __device__ __forceinline__ void align_ring(const AlignArgs& a, unsigned char* smem_raw) {
   static_assert(GW == 1 || GW == 2 || GW == 4 || GW == 8 || GW == 16 || GW == 32, "warps per pair");
@@ -123,7 +125,7 @@ __device__ __forceinline__ void align_ring(const AlignArgs& a, unsigned char* sm
   const int ns = a.pen.slots();
   const int W = a.ring_w;
   const int rm = a.pen.rm, re = a.pen.re;
-  unsigned char* gsm = smem_raw + (size_t)gid * group_smem_bytes(a.pen, W, kMode, a.seq_cap, GW);
+  unsigned char* gsm = smem_raw + (size_t)gid * group_smem_bytes(a.pen, W, kMode, a.seq_cap, GW, false);
   int* s_lo = reinterpret_cast<int*>(gsm);
   int* s_hi = s_lo + ns;
   int* s_alo = s_hi + ns;
@@ -830,7 +832,18 @@ __device__ __forceinline__ void align_ring(const AlignArgs& a, unsigned char* sm
 // registers, 16 warps per SM.
 template <int kMode, int GW, int kModel>
 constexpr int kernel_min_blocks() {
-  return (kModel & kBoundFlag) ? (GW <= 4 ? 4 : (GW == 8 ? 2 : 1)) : cta_min_blocks<kMode, GW>();
+  if (kModel & kBoundFlag) return GW <= 4 ? 4 : (GW == 8 ? 2 : 1);
+  if (kMode == kModeShared && GW == 1 && (kModel & (kLowMemFlag | kSingleFlag))) return 7;  // 72 registers
+  return cta_min_blocks<kMode, GW>();
+}
+
+// (The CPU emulation's drivers know no kDeepFlag.)
+constexpr bool deep_kernel(int model) {
+#ifdef TSU_WARP_EMU
+  return true;
+#else
+  return (model & kDeepFlag) != 0;
+#endif
 }
 
 template <bool kCigar, int kMode, int GW, int kModel = kModelAffine>
@@ -840,8 +853,14 @@ __global__ void __launch_bounds__(cta_threads<GW>(), (kernel_min_blocks<kMode, G
 #else
   extern __shared__ __align__(16) unsigned char smem_raw[];
 #endif
-  if constexpr (kMode == kModeShared && !(kModel & kLowMemFlag))
-    align_packed<kCigar, GW, kModel & 7, (kModel & kBoundFlag) != 0>(a, smem_raw);
+#ifdef TSU_WARP_EMU
+  if (kMode == kModeShared && !packed_fits(a.pen)) {  // (its driver knows no kSingleFlag)
+    align_ring<kCigar, kMode, GW, kModel>(a, smem_raw);
+    return;
+  }
+#endif
+  if constexpr (kMode == kModeShared && !(kModel & (kLowMemFlag | kSingleFlag)))
+    align_packed<kCigar, GW, kModel & 7, (kModel & kBoundFlag) != 0, deep_kernel(kModel)>(a, smem_raw);
   else
     align_ring<kCigar, kMode, GW, kModel>(a, smem_raw);
 }
@@ -854,7 +873,7 @@ __global__ void __launch_bounds__(kProbeThreads, 5) probe_kernel(ProbeArgs a) {
 #else
   extern __shared__ __align__(16) unsigned char smem_raw[];
 #endif
-  probe_packed<kModel>(a, smem_raw);
+  probe_packed<kModel & 7, deep_kernel(kModel)>(a, smem_raw);
 }
 
 template <int kModel>

@@ -34,6 +34,13 @@ enum : int { kLowMemFlag = 8 };
 // added to a model: the shared-ring kernels of pairs with score bounds
 // (AlignArgs::bound)
 enum : int { kBoundFlag = 16 };
+// added to a model: the shared-ring kernels of one diagonal per thread, for
+// rings and sides beyond the packed kernel's (PassGeom::single)
+enum : int { kSingleFlag = 32 };
+// added to a model: the packed kernels of rings deeper than 64 scores, whose
+// record of the last scores takes a second word (in every packed kernel it cost
+// 1 - 2 % of 1 kbp batches: 18.0 -> 18.3 ms with CIGARs)
+enum : int { kDeepFlag = 64 };
 
 struct SeqView {
   int64_t n;  // pairs
@@ -223,15 +230,18 @@ __host__ __device__ inline int64_t ckpt_bytes_for(const Pen& p, int ring_w, int 
 __host__ __device__ inline int partial_words(const Pen& p) { return p.dual() ? 16 : 8; }
 
 // The shared-ring kernel (tsu_packed.cuh): longest side its 16-bit offsets
-// hold (tsu_packed.cuh),
-// deepest ring its 64-bit record of the last scores covers, 32-bit words per
+// hold, deepest ring and longest extension its records of the last scores
+// cover, 32-bit words per
 // ring row (ring_w halfwords and 4 on each side) and bytes before the ring
 // (4 broadcast words, 2 gw partials, 16 bytes of row offsets per M slot and
 // per I / D slot pair).
 constexpr int kPackedPlainLen = 16351;  // launches without score bounds
 constexpr int kPackedMaxLen = 20463;    // launches with them, and the probe
 constexpr int kPackedMaxW = 12288;  // diagonals per ring row (absent I cells climb 2 per diagonal, below offset 0)
-constexpr int kPackedMaxDepth = 64;
+constexpr int kPackedMaxDepth = 128, kPackedMaxExt = 63;
+__host__ __device__ inline bool packed_fits(const Pen& p) {
+  return p.rm <= kPackedMaxDepth && (p.linear() || (p.ge <= kPackedMaxExt && p.ge2 <= kPackedMaxExt));
+}
 __host__ __device__ constexpr int packed_row_words(int ring_w) { return (ring_w + 8) / 2; }
 __host__ __device__ inline int packed_head_bytes(const Pen& p, int gw) {
   return ((16 + 8 * gw + 15) & ~15) + 16 * (p.rm + p.re + p.re2);
@@ -246,20 +256,20 @@ __host__ __device__ inline int bounded_bytes(const Pen& p, int d, int words, int
   return (packed_head_bytes(p, gw) + (p.slots() + 1) * packed_row_words(packed_width(d)) * 4 + words * 4 + 15) & ~15;
 }
 
-// Shared memory per group of gw warps, in bytes.  Global mode and the
-// low-memory kernels: slot limits (lo, hi, alo per slot), warp partials
-// [2][gw][partial_words] (gw > 1), 4 broadcast words, then in shared mode an
-// int16 ring of slots * ring_w and seq_cap sequence words; in global mode with
-// seq_cap > 0, at the next 16-byte boundary, 16 reserved bytes and seq_cap
-// sequence words.  Shared mode takes the larger of that and of the packed
-// kernel's head, slots + 1 rows and sequence words.
-__host__ __device__ inline int group_smem_bytes(const Pen& p, int ring_w, int mode, int seq_cap, int gw) {
+// Shared memory per group of gw warps, in bytes.  Global mode, the low-memory
+// kernels and those of one diagonal per thread: slot limits (lo, hi, alo per
+// slot), warp partials [2][gw][partial_words] (gw > 1), 4 broadcast words, then
+// in shared mode an int16 ring of slots * ring_w and seq_cap sequence words; in
+// global mode with seq_cap > 0, at the next 16-byte boundary, 16 reserved bytes
+// and seq_cap sequence words.  packed (shared mode): the larger of that and of
+// the packed kernel's head, slots + 1 rows and sequence words.
+__host__ __device__ inline int group_smem_bytes(const Pen& p, int ring_w, int mode, int seq_cap, int gw, bool packed) {
   const int ns = p.slots();
   int b = 3 * ns * 4 + (gw > 1 ? 2 * partial_words(p) * gw * 4 : 0) + 16;
   if (mode == kModeShared) {
     b += ((ns * ring_w * 2 + 15) & ~15) + seq_cap * 4;
-    const int packed = packed_head_bytes(p, gw) + (ns + 1) * packed_row_words(ring_w) * 4 + seq_cap * 4;
-    if (packed > b) b = packed;
+    const int rows = packed_head_bytes(p, gw) + (ns + 1) * packed_row_words(ring_w) * 4 + seq_cap * 4;
+    if (packed && rows > b) b = rows;
   } else if (seq_cap > 0) {
     b = ((b + 15) & ~15) + 16 + seq_cap * 4;
   }

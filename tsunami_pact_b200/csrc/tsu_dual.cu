@@ -5,18 +5,17 @@
 
 namespace tsu {
 
-cudaError_t align_occupancy_dual(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ,
-                                 bool lowmem, bool bounded) {
-  return launch_detail::occupancy<kModelDual>(cigar, mode, gw, threads, smem, optin, occ, lowmem, bounded);
+cudaError_t align_occupancy_dual(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ, int flag) {
+  return launch_detail::occupancy<kModelDual>(cigar, mode, gw, threads, smem, optin, occ, flag);
 }
 
 void launch_align_dual(bool cigar, int mode, int gw, int blocks, int threads, size_t smem, cudaStream_t st,
-                       const AlignArgs& a, bool lowmem, bool bounded) {
-  launch_detail::launch<kModelDual>(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded);
+                       const AlignArgs& a, int flag) {
+  launch_detail::launch<kModelDual>(cigar, mode, gw, blocks, threads, smem, st, a, flag);
 }
 
-cudaError_t probe_occupancy_dual(bool wide, int threads, size_t smem, int optin, int* occ) {
-  return launch_detail::probe_occupancy<kModelDual>(wide, threads, smem, optin, occ);
+cudaError_t probe_occupancy_dual(bool wide, bool deep, int threads, size_t smem, int optin, int* occ) {
+  return launch_detail::probe_occupancy<kModelDual>(wide, deep, threads, smem, optin, occ);
 }
 
 void launch_probe_dual(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {

@@ -319,21 +319,30 @@ struct BatchInfo {
 
 // The align_kernel instantiations (tsu_launch.cuh): gap-affine kernels here,
 // dual gap-affine ones in tsu_dual.cu, gap-linear ones in tsu_linear.cu.
-// lowmem: the checkpointed-history variant (CIGAR passes of a low-memory
-// context).
-cudaError_t align_occupancy(const tsu_ctx* ctx, bool cigar, int mode, int gw, int threads, size_t smem, int optin,
-                            int* occ, bool lowmem, bool bounded) {
+// The variant that a pass runs (tsu_launch.cuh): of a low-memory context's
+// CIGAR passes, of pairs with score bounds, of deep rings, of one diagonal per
+// thread.
+int pass_flag(const tsu_ctx* ctx, const tsu::PassGeom& g, bool cigar) {
+  if (cigar && g.ckpt_k > 0) return tsu::kLowMemFlag;
+  if (g.mode == tsu::kModeGlobal) return 0;
+  if (g.single) return tsu::kSingleFlag;
+  return (g.bounded ? tsu::kBoundFlag : 0) | (ctx->rp.rm > 64 ? tsu::kDeepFlag : 0);
+}
+
+cudaError_t align_occupancy(const tsu_ctx* ctx, bool cigar, const tsu::PassGeom& g, size_t smem, int optin, int* occ) {
+  const int mode = g.mode, gw = g.gw, threads = g.cta_threads, flag = pass_flag(ctx, g, cigar);
   switch (ctx->rp.model()) {
-    case tsu::kModelDual: return tsu::align_occupancy_dual(cigar, mode, gw, threads, smem, optin, occ, lowmem, bounded);
-    case tsu::kModelLinear: return tsu::align_occupancy_linear(cigar, mode, gw, threads, smem, optin, occ, lowmem, bounded);
+    case tsu::kModelDual: return tsu::align_occupancy_dual(cigar, mode, gw, threads, smem, optin, occ, flag);
+    case tsu::kModelLinear: return tsu::align_occupancy_linear(cigar, mode, gw, threads, smem, optin, occ, flag);
     default:
-      return tsu::launch_detail::occupancy<tsu::kModelAffine>(cigar, mode, gw, threads, smem, optin, occ, lowmem, bounded);
+      return tsu::launch_detail::occupancy<tsu::kModelAffine>(cigar, mode, gw, threads, smem, optin, occ, flag);
   }
 }
 
-void launch_align(const tsu_ctx* ctx, bool cigar, int mode, int gw, int blocks, int threads, size_t smem,
-                  cudaStream_t st, const tsu::AlignArgs& a, int cluster = 1) {
-  const bool lowmem = cigar && a.ckpt_k > 0, bounded = a.bound != nullptr;
+void launch_align(const tsu_ctx* ctx, bool cigar, const Pass& ps, cudaStream_t st, const tsu::AlignArgs& a) {
+  const int mode = ps.g.mode, gw = ps.g.gw, cluster = ps.g.cluster, blocks = ps.blocks * cluster, threads = ps.threads;
+  const size_t smem = ps.smem_bytes;
+  const int flag = pass_flag(ctx, ps.g, cigar);
   if (a.wide_cell) {
     switch (ctx->rp.model()) {
       case tsu::kModelDual: tsu::launch_wide_dual(cigar, blocks, cluster, smem, st, a); break;
@@ -343,10 +352,10 @@ void launch_align(const tsu_ctx* ctx, bool cigar, int mode, int gw, int blocks, 
     return;
   }
   switch (ctx->rp.model()) {
-    case tsu::kModelDual: tsu::launch_align_dual(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded); break;
-    case tsu::kModelLinear: tsu::launch_align_linear(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded); break;
+    case tsu::kModelDual: tsu::launch_align_dual(cigar, mode, gw, blocks, threads, smem, st, a, flag); break;
+    case tsu::kModelLinear: tsu::launch_align_linear(cigar, mode, gw, blocks, threads, smem, st, a, flag); break;
     default:
-      tsu::launch_detail::launch<tsu::kModelAffine>(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded);
+      tsu::launch_detail::launch<tsu::kModelAffine>(cigar, mode, gw, blocks, threads, smem, st, a, flag);
       break;
   }
 }
@@ -358,13 +367,14 @@ int plan_probe(tsu_ctx* ctx, bool wide, int seq_cap, int64_t n, int* blocks, siz
   *smem = (size_t)wpb * (wide ? tsu::wide_probe_smem_bytes(ctx->rp) : tsu::probe_smem_bytes(ctx->rp, seq_cap));
   *blocks = 0;  // does not fit
   if (*smem > (size_t)ctx->smem_optin) return TSU_OK;
+  const bool deep = ctx->rp.rm > 64;
   int occ = 0;
   cudaError_t e = cudaSuccess;
   switch (ctx->rp.model()) {
-    case tsu::kModelDual: e = tsu::probe_occupancy_dual(wide, tsu::kProbeThreads, *smem, ctx->smem_optin, &occ); break;
-    case tsu::kModelLinear: e = tsu::probe_occupancy_linear(wide, tsu::kProbeThreads, *smem, ctx->smem_optin, &occ); break;
+    case tsu::kModelDual: e = tsu::probe_occupancy_dual(wide, deep, tsu::kProbeThreads, *smem, ctx->smem_optin, &occ); break;
+    case tsu::kModelLinear: e = tsu::probe_occupancy_linear(wide, deep, tsu::kProbeThreads, *smem, ctx->smem_optin, &occ); break;
     default:
-      e = tsu::launch_detail::probe_occupancy<tsu::kModelAffine>(wide, tsu::kProbeThreads, *smem, ctx->smem_optin, &occ);
+      e = tsu::launch_detail::probe_occupancy<tsu::kModelAffine>(wide, deep, tsu::kProbeThreads, *smem, ctx->smem_optin, &occ);
       break;
   }
   if (e != cudaSuccess) return set_err(ctx, TSU_EDEVICE, "probe occupancy query failed (%d)", (int)e);
@@ -395,8 +405,7 @@ int plan_groups(tsu_ctx* ctx, const tsu::PassGeom& g, int64_t n_pairs, bool want
   int occ = 1;
   cudaError_t e = cudaSuccess;
   if (!g.wide_cell)  // (the wide kernel: one block per SM)
-    e = align_occupancy(ctx, want_cigar, g.mode, g.gw, g.cta_threads, (size_t)gpc * g.group_smem, ctx->smem_optin, &occ,
-                      g.ckpt_k > 0, g.bounded);
+    e = align_occupancy(ctx, want_cigar, g, (size_t)gpc * g.group_smem, ctx->smem_optin, &occ);
   if (e != cudaSuccess || occ < 1) return set_err(ctx, TSU_EDEVICE, "occupancy query failed (%d)", (int)e);
   int64_t warps = (int64_t)ctx->sms * occ * gpc;  // groups
   const size_t per_warp = group_scratch_bytes(g);
@@ -428,7 +437,7 @@ int plan_groups(tsu_ctx* ctx, const tsu::PassGeom& g, int64_t n_pairs, bool want
 int plan_pass_within(tsu_ctx* ctx, const BatchInfo& bi, int64_t n_pairs, tsu::PassChoice pc, double hint,
                      bool want_cigar, size_t avail, Pass* out) {
   const tsu::PassGeom g = tsu::plan_geometry(ctx->rp, bi.max_m, bi.max_n, pc.mode, pc.gw, hint, want_cigar,
-                                             ctx->smem_optin, want_cigar ? ctx->low_mem : 0);
+                                             ctx->smem_optin, want_cigar ? ctx->low_mem : 0, pc.single);
   return plan_groups(ctx, g, n_pairs, want_cigar, avail, out);
 }
 
@@ -1276,7 +1285,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   // Pairs with a bound probe (tsu::wants_bound; end to end, history of every
   // score): they wait for their bounds, the others start at once.
   const bool low_mem = want_cigar && ctx->low_mem < 0;
-  const bool can_bound = !ctx->one_warp && h_plen && ctx->rp.rm <= tsu::kPackedMaxDepth &&
+  const bool can_bound = !ctx->one_warp && h_plen && tsu::packed_fits(ctx->rp) &&
                          !(want_cigar && ctx->low_mem > 0) &&
                          !(ctx->ends_free[0] | ctx->ends_free[1] | ctx->ends_free[2] | ctx->ends_free[3]);
   // A list of pairs to probe: those of the wide probe (longer than
@@ -1414,7 +1423,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
         r.pc = tsu::fit_start(r.pc, ctx->rp, r.bi.max_m, r.bi.max_n, r.hint, ctx->smem_optin);
       r.few = r.n <= ctx->sms && std::max(r.bi.max_m, r.bi.max_n) >= few_side;
       if (r.few) r.pc = tsu::few_start(r.pc, ctx->rp, std::max(r.bi.max_m, r.bi.max_n));
-      if (!ctx->one_warp) r.pc = tsu::fill_warps(r.pc, r.n, std::max(r.bi.max_m, r.bi.max_n), ctx->sms);
+      if (!ctx->one_warp) r.pc = tsu::fill_warps(r.pc, ctx->rp, r.n, std::max(r.bi.max_m, r.bi.max_n), ctx->sms);
       if ((rc = plan_pass_within(ctx, r.bi, r.n, r.pc, r.hint, want_cigar, avail, &r.ps))) return rc;
       need = std::max(need, scratch_bytes(r.ps, want_cigar));
     }
@@ -1626,8 +1635,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
         if (cs != st) CU(cudaStreamWaitEvent(cs, ctx->fork_ev, 0));
       }
       CU(cudaEventRecord(ctx->bev[2 * r.slot], cs));
-      launch_align(ctx, want_cigar, r.ps.g.mode, r.ps.g.gw, r.ps.blocks * r.ps.g.cluster, r.ps.threads, r.ps.smem_bytes, cs, a,
-                   r.ps.g.cluster);
+      launch_align(ctx, want_cigar, r.ps, cs, a);
       CU(cudaGetLastError());
       CU(cudaEventRecord(ctx->bev[2 * r.slot + 1], cs));
       if (cs != st) CU(cudaStreamWaitEvent(st, ctx->bev[2 * r.slot + 1], 0));
@@ -1694,7 +1702,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       const tsu::AlignArgs a = align_args(r.ps, all_pairs ? nullptr : P<int32_t>(ctx->b_order) + r.off, r.n, r.slot,
                                           P<int32_t>(ctx->b_retry) + r.off);
       CU(record(ctx, ctx->bev[2 * r.slot], st));
-      launch_align(ctx, want_cigar, r.ps.g.mode, r.ps.g.gw, r.ps.blocks, r.ps.threads, r.ps.smem_bytes, st, a);
+      launch_align(ctx, want_cigar, r.ps, st, a);
       CU(cudaGetLastError());
       CU(record(ctx, ctx->bev[2 * r.slot + 1], st));
     }
@@ -1853,7 +1861,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       CU(cudaMemsetAsync(d_slot, 0, 8, st));  // queue head + retry count
       const tsu::AlignArgs a = align_args(ps, d_order, nretry, r.slot, d_retry);
       CU(cudaEventRecord(ctx->pev[0], st));
-      launch_align(ctx, want_cigar, ps.g.mode, ps.g.gw, ps.blocks, ps.threads, ps.smem_bytes, st, a);
+      launch_align(ctx, want_cigar, ps, st, a);
       ctx->timing.kernel_launches++;
       CU(cudaGetLastError());
       CU(cudaEventRecord(ctx->pev[1], st));

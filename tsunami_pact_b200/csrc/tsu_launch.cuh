@@ -19,22 +19,24 @@ namespace tsu {
 
 // The dual gap-affine kernels (tsu_dual.cu) and the gap-linear ones
 // (tsu_linear.cu).
-// lowmem: the low-memory variant of the CIGAR kernel (cigar is then
-// ignored); bounded: the shared-ring variant of pairs with score bounds.
+// flag: 0, or a variant: kLowMemFlag (CIGARs; cigar is then ignored),
+// kBoundFlag (shared ring, pairs with score bounds), kDeepFlag (shared ring,
+// with or without kBoundFlag), kSingleFlag (shared ring, one diagonal per
+// thread).
 cudaError_t align_occupancy_dual(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ,
-                                 bool lowmem, bool bounded);
+                                 int flag);
 void launch_align_dual(bool cigar, int mode, int gw, int blocks, int threads, size_t smem, cudaStream_t st,
-                       const AlignArgs& a, bool lowmem, bool bounded);
+                       const AlignArgs& a, int flag);
 cudaError_t align_occupancy_linear(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ,
-                                   bool lowmem, bool bounded);
+                                   int flag);
 void launch_align_linear(bool cigar, int mode, int gw, int blocks, int threads, size_t smem, cudaStream_t st,
-                         const AlignArgs& a, bool lowmem, bool bounded);
+                         const AlignArgs& a, int flag);
 
 // The bound probe of each model (probe_kernel).
 // wide: of pairs of any length (wide_probe_kernel).
-cudaError_t probe_occupancy_dual(bool wide, int threads, size_t smem, int optin, int* occ);
+cudaError_t probe_occupancy_dual(bool wide, bool deep, int threads, size_t smem, int optin, int* occ);
 void launch_probe_dual(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a);
-cudaError_t probe_occupancy_linear(bool wide, int threads, size_t smem, int optin, int* occ);
+cudaError_t probe_occupancy_linear(bool wide, bool deep, int threads, size_t smem, int optin, int* occ);
 void launch_probe_linear(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a);
 // The wide kernel of each model (wide_kernel; one block of kWideThreads per
 // pair, or `cluster` of them; a.wide_cell bytes per ring cell).
@@ -44,8 +46,10 @@ void launch_wide_linear(bool cigar, int blocks, int cluster, size_t smem, cudaSt
 namespace launch_detail {
 
 template <int kModel>
-cudaError_t probe_occupancy(bool wide, int threads, size_t smem, int optin, int* occ) {
-  const void* const f = wide ? (const void*)wide_probe_kernel<kModel> : (const void*)probe_kernel<kModel>;
+cudaError_t probe_occupancy(bool wide, bool deep, int threads, size_t smem, int optin, int* occ) {
+  const void* const f = wide   ? (const void*)wide_probe_kernel<kModel>
+                        : deep ? (const void*)probe_kernel<kModel | kDeepFlag>
+                               : (const void*)probe_kernel<kModel>;
   const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, f, threads, smem);
@@ -55,6 +59,8 @@ template <int kModel>
 void probe(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {
   if (wide)
     wide_probe_kernel<kModel><<<blocks, threads, smem, st>>>(a);
+  else if (a.pen.rm > 64)
+    probe_kernel<kModel | kDeepFlag><<<blocks, threads, smem, st>>>(a);
   else
     probe_kernel<kModel><<<blocks, threads, smem, st>>>(a);
 }
@@ -121,20 +127,31 @@ cudaError_t occ_gw(int gw, int threads, size_t smem, int optin, int* occ) {
   }
 }
 
+// f(flag as a compile-time constant) for the shared ring's variants.
+template <class F>
+auto with_flag(int flag, F&& f) {
+  switch (flag) {
+    case kBoundFlag: return f(std::integral_constant<int, kBoundFlag>{});
+    case kBoundFlag | kDeepFlag: return f(std::integral_constant<int, kBoundFlag | kDeepFlag>{});
+    case kDeepFlag: return f(std::integral_constant<int, kDeepFlag>{});
+    case kSingleFlag: return f(std::integral_constant<int, kSingleFlag>{});
+    default: return f(std::integral_constant<int, 0>{});
+  }
+}
+
 template <int kModel>
-cudaError_t occupancy(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ, bool lowmem,
-                      bool bounded) {
-  if (bounded)
-    return cigar ? occ_gw<true, kModeShared, kModel | kBoundFlag>(gw, threads, smem, optin, occ)
-                 : occ_gw<false, kModeShared, kModel | kBoundFlag>(gw, threads, smem, optin, occ);
-  if (lowmem)
+cudaError_t occupancy(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ, int flag) {
+  if (flag == kLowMemFlag)
     return mode == kModeShared ? occ_gw<true, kModeShared, kModel | kLowMemFlag>(gw, threads, smem, optin, occ)
                                : occ_gw<true, kModeGlobal, kModel | kLowMemFlag>(gw, threads, smem, optin, occ);
-  if (cigar)
-    return mode == kModeShared ? occ_gw<true, kModeShared, kModel>(gw, threads, smem, optin, occ)
-                               : occ_gw<true, kModeGlobal, kModel>(gw, threads, smem, optin, occ);
-  return mode == kModeShared ? occ_gw<false, kModeShared, kModel>(gw, threads, smem, optin, occ)
-                             : occ_gw<false, kModeGlobal, kModel>(gw, threads, smem, optin, occ);
+  if (mode == kModeGlobal)
+    return cigar ? occ_gw<true, kModeGlobal, kModel>(gw, threads, smem, optin, occ)
+                 : occ_gw<false, kModeGlobal, kModel>(gw, threads, smem, optin, occ);
+  return with_flag(flag, [&](auto f) {
+    constexpr int kM = kModel | decltype(f)::value;
+    return cigar ? occ_gw<true, kModeShared, kM>(gw, threads, smem, optin, occ)
+                 : occ_gw<false, kModeShared, kM>(gw, threads, smem, optin, occ);
+  });
 }
 
 template <bool kCigar, int kMode, int kModel>
@@ -154,27 +171,25 @@ void launch_gw(int gw, int blocks, int threads, size_t smem, cudaStream_t st, co
 
 template <int kModel>
 void launch(bool cigar, int mode, int gw, int blocks, int threads, size_t smem, cudaStream_t st, const AlignArgs& a,
-            bool lowmem, bool bounded) {
-  if (bounded) {
-    if (cigar)
-      launch_gw<true, kModeShared, kModel | kBoundFlag>(gw, blocks, threads, smem, st, a);
-    else
-      launch_gw<false, kModeShared, kModel | kBoundFlag>(gw, blocks, threads, smem, st, a);
-  } else if (lowmem) {
+            int flag) {
+  if (flag == kLowMemFlag) {
     if (mode == kModeShared)
       launch_gw<true, kModeShared, kModel | kLowMemFlag>(gw, blocks, threads, smem, st, a);
     else
       launch_gw<true, kModeGlobal, kModel | kLowMemFlag>(gw, blocks, threads, smem, st, a);
-  } else if (cigar) {
-    if (mode == kModeShared)
-      launch_gw<true, kModeShared, kModel>(gw, blocks, threads, smem, st, a);
-    else
+  } else if (mode == kModeGlobal) {
+    if (cigar)
       launch_gw<true, kModeGlobal, kModel>(gw, blocks, threads, smem, st, a);
-  } else {
-    if (mode == kModeShared)
-      launch_gw<false, kModeShared, kModel>(gw, blocks, threads, smem, st, a);
     else
       launch_gw<false, kModeGlobal, kModel>(gw, blocks, threads, smem, st, a);
+  } else {
+    with_flag(flag, [&](auto f) {
+      constexpr int kM = kModel | decltype(f)::value;
+      if (cigar)
+        launch_gw<true, kModeShared, kM>(gw, blocks, threads, smem, st, a);
+      else
+        launch_gw<false, kModeShared, kM>(gw, blocks, threads, smem, st, a);
+    });
   }
 }
 

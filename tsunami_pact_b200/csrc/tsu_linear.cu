@@ -6,18 +6,17 @@
 
 namespace tsu {
 
-cudaError_t align_occupancy_linear(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ,
-                                   bool lowmem, bool bounded) {
-  return launch_detail::occupancy<kModelLinear>(cigar, mode, gw, threads, smem, optin, occ, lowmem, bounded);
+cudaError_t align_occupancy_linear(bool cigar, int mode, int gw, int threads, size_t smem, int optin, int* occ, int flag) {
+  return launch_detail::occupancy<kModelLinear>(cigar, mode, gw, threads, smem, optin, occ, flag);
 }
 
 void launch_align_linear(bool cigar, int mode, int gw, int blocks, int threads, size_t smem, cudaStream_t st,
-                         const AlignArgs& a, bool lowmem, bool bounded) {
-  launch_detail::launch<kModelLinear>(cigar, mode, gw, blocks, threads, smem, st, a, lowmem, bounded);
+                         const AlignArgs& a, int flag) {
+  launch_detail::launch<kModelLinear>(cigar, mode, gw, blocks, threads, smem, st, a, flag);
 }
 
-cudaError_t probe_occupancy_linear(bool wide, int threads, size_t smem, int optin, int* occ) {
-  return launch_detail::probe_occupancy<kModelLinear>(wide, threads, smem, optin, occ);
+cudaError_t probe_occupancy_linear(bool wide, bool deep, int threads, size_t smem, int optin, int* occ) {
+  return launch_detail::probe_occupancy<kModelLinear>(wide, deep, threads, smem, optin, occ);
 }
 
 void launch_probe_linear(bool wide, int blocks, int threads, size_t smem, cudaStream_t st, const ProbeArgs& a) {

@@ -101,12 +101,10 @@ size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 // The kernel's dynamic shared memory limit is set to the device maximum, the
 // value the engine's contexts set too, so concurrent callers never lower it
 // under each other's launches.
-template <int kMode>
-cudaError_t occupancy(int threads, size_t smem, int optin, int* occ) {
-  cudaError_t e =
-      cudaFuncSetAttribute(tsu::align_kernel<false, kMode, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+cudaError_t occupancy(void (*kernel)(tsu::AlignArgs), int threads, size_t smem, int optin, int* occ) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, tsu::align_kernel<false, kMode, 1>, threads, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kernel, threads, smem);
 }
 
 }  // namespace
@@ -209,8 +207,11 @@ extern "C" int tsu_align_scores_noalloc(const tsu_penalties* pen, const tsu_batc
     // does not fit a block, and every pair takes the global pass
     if (pass == 0 && geo.mode == tsu::kModeShared && (size_t)wpb * geo.group_smem > (size_t)smem_optin) continue;
     int occ = 0;
-    NA_CU(geo.mode == tsu::kModeShared ? occupancy<tsu::kModeShared>(32 * wpb, (size_t)wpb * geo.group_smem, smem_optin, &occ)
-                                       : occupancy<tsu::kModeGlobal>(32 * wpb, (size_t)wpb * geo.group_smem, smem_optin, &occ));
+    void (*const kernel)(tsu::AlignArgs) =
+        geo.mode != tsu::kModeShared ? &tsu::align_kernel<false, tsu::kModeGlobal, 1>
+        : rp.rm > 64                 ? &tsu::align_kernel<false, tsu::kModeShared, 1, tsu::kModelAffine | tsu::kDeepFlag>
+                                     : &tsu::align_kernel<false, tsu::kModeShared, 1>;
+    NA_CU(occupancy(kernel, 32 * wpb, (size_t)wpb * geo.group_smem, smem_optin, &occ));
     if (occ < 1) {
       if (pass == 0) continue;
       return TSU_EDEVICE;
@@ -239,10 +240,7 @@ extern "C" int tsu_align_scores_noalloc(const tsu_penalties* pen, const tsu_batc
     a.retry_count = queue + 1;
     NA_CU(cudaMemsetAsync(queue, 0, 2 * sizeof(unsigned int), st));
     const size_t smem = (size_t)bw * geo.group_smem;
-    if (geo.mode == tsu::kModeShared)
-      tsu::align_kernel<false, tsu::kModeShared, 1><<<(int)(warps / bw), 32 * bw, smem, st>>>(a);
-    else
-      tsu::align_kernel<false, tsu::kModeGlobal, 1><<<(int)(warps / bw), 32 * bw, smem, st>>>(a);
+    kernel<<<(int)(warps / bw), 32 * bw, smem, st>>>(a);
     NA_CU(cudaGetLastError());
     unsigned int nretry = 0;
     NA_CU(cudaMemcpyAsync(&nretry, queue + 1, sizeof nretry, cudaMemcpyDeviceToHost, st));

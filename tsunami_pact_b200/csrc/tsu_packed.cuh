@@ -40,8 +40,10 @@
 // Within a score bound (kBound): 1,000 x 10 kbp at 15 % 50.5 -> 27.1 ms with
 // the probe, on 8 warps; two words per lane 32.0 -> 25.2 ms without it.
 // Limits: sides of at most kPackedPlainLen bases (kPackedMaxLen with a bound),
-// ACGT only, at most 64 score steps of ring depth; other pairs go to
-// tsu_wide.cuh (with a bound) or the global ring (tsu_align.cuh).
+// ACGT only, at most 128 score steps of ring depth; other pairs go to
+// tsu_wide.cuh (with a bound), to the shared ring of one diagonal per thread
+// (deeper rings with CIGARs, sides up to 32,000) or to the global ring
+// (tsu_align.cuh).
 #pragma once
 
 #include <type_traits>
@@ -306,8 +308,9 @@ __device__ __forceinline__ void packed_tables(const Pen& pen, int RB, smem_t tab
 }
 
 // A pair's score by score bookkeeping, the same for every lane: the step's
-// rows, the diagonals gained, which wavefronts exist.
-template <int kModel>
+// rows, the diagonals gained, which wavefronts exist (kDeep: rings deeper than
+// 64 scores, of up to 128).
+template <int kModel, bool kDeep>
 struct PackedSteps {
   static constexpr bool kDual = kModel == kModelDual, kLin = kModel == kModelLinear;
   smem_t tab_m, tab_g, tab_g2, tab_end;
@@ -315,9 +318,10 @@ struct PackedSteps {
   int none_row;                // the row of absent cells
   int grow, grow_at;           // diagonals gained on each side, next score that gains one
   int grow2, grow2_at;         // the second gap piece
-  // which of the last 64 scores have an M (an I or D) wavefront; once every
-  // score in reach has all of them it stays so (full)
-  unsigned long long has_m, has_g, has_g2;
+  // which of the last 64 scores (kDeep: had_m, the 64 before them) have an M
+  // wavefront, which of the last 64 an I or D; once every score in reach has
+  // all of them it stays so (full)
+  unsigned long long has_m, had_m, has_g, has_g2;
   bool full;
 
   __device__ __forceinline__ void begin(const Pen& pen, smem_t tables, int none) {
@@ -329,7 +333,7 @@ struct PackedSteps {
     grow = grow2 = 0;
     grow_at = pen.go;
     grow2_at = kDual ? pen.go2 : INT_MAX;
-    has_m = 1, has_g = 0, has_g2 = 0;
+    has_m = 1, had_m = 0, has_g = 0, has_g2 = 0;
     full = false;
   }
   __device__ __forceinline__ int gained() const { return kDual ? max(grow, grow2) : grow; }
@@ -365,18 +369,24 @@ struct PackedSteps {
   // cells.
   __device__ __forceinline__ bool present(const Pen& pen, PackedRows* r) {
     if (full) return true;
-    const bool px = (has_m >> (pen.x - 1)) & 1, po = (has_m >> (pen.go - 1)) & 1;
+    auto m_at = [&](int back) -> bool {
+      return (((!kDeep || back <= 64) ? has_m >> (back - 1) : had_m >> (back - 65)) & 1) != 0;
+    };
+    const bool px = m_at(pen.x), po = m_at(pen.go);
     const bool pe = !kLin && ((has_g >> (pen.ge - 1)) & 1);
-    const bool po2 = kDual && ((has_m >> (pen.go2 - 1)) & 1);
+    const bool po2 = kDual && m_at(pen.go2);
     const bool pe2 = kDual && ((has_g2 >> (pen.ge2 - 1)) & 1);
     const bool pm = px | po | pe | po2 | pe2;
+    if constexpr (kDeep) had_m = (had_m << 1) | (has_m >> 63);
     has_m = (has_m << 1) | (pm ? 1u : 0u);
     if constexpr (!kLin) has_g = (has_g << 1) | ((po | pe) ? 1u : 0u);
     if constexpr (kDual) has_g2 = (has_g2 << 1) | ((po2 | pe2) ? 1u : 0u);
     if (!pm) return false;
-    const unsigned long long dm = (1ull << (pen.rm - 1)) - 1, dg = (1ull << pen.ge) - 1,
+    const unsigned long long dm = kDeep && pen.rm > 64 ? ~0ull : (1ull << (pen.rm - 1)) - 1,
+                             dh = kDeep ? (1ull << max(pen.rm - 65, 0)) - 1 : 0,
+                             dg = kLin ? 0 : (1ull << pen.ge) - 1,
                              dg2 = kDual ? (1ull << pen.ge2) - 1 : 0;
-    full = (has_m & dm) == dm && (kLin || (has_g & dg) == dg) && (!kDual || (has_g2 & dg2) == dg2);
+    full = (has_m & dm) == dm && (!kDeep || (had_m & dh) == dh) && (kLin || (has_g & dg) == dg) && (!kDual || (has_g2 & dg2) == dg2);
     if (!px) r->r_mx = none_row;
     if (!po) r->r_mo = none_row;
     if constexpr (!kLin) {
@@ -547,8 +557,8 @@ __device__ __forceinline__ int packed_cigar(const uint32_t* hist, int64_t hist_c
 }
 
 // The body of align_kernel for the shared ring (see the head of this file).
-// kBound: the pairs have score bounds (a.bound), end to end.
-template <bool kCigar, int GW, int kModel, bool kBound>
+// kBound: the pairs have score bounds (a.bound), end to end; kDeep: PackedSteps.
+template <bool kCigar, int GW, int kModel, bool kBound, bool kDeep>
 __device__ __forceinline__ void align_packed(const AlignArgs& a, unsigned char* smem_raw) {
   constexpr bool kDual = kModel == kModelDual;
   constexpr bool kLin = kModel == kModelLinear;
@@ -568,7 +578,7 @@ __device__ __forceinline__ void align_packed(const AlignArgs& a, unsigned char* 
   // 4 broadcast words, 2 GW partials of the free-end test, the row tables,
   // the ring, the sequences.  Bounded pairs share out the group's bytes each
   // by its own width and lengths.
-  const int gbytes = kBound ? a.group_bytes : group_smem_bytes(a.pen, a.ring_w, kModeShared, a.seq_cap, GW);
+  const int gbytes = kBound ? a.group_bytes : group_smem_bytes(a.pen, a.ring_w, kModeShared, a.seq_cap, GW, true);
   const smem_t bc = smem_addr(smem_raw) + (size_t)gid * gbytes;
   const smem_t part = bc + 16;
   const smem_t tab_m = bc + packed_head_bytes(Pen(), GW);
@@ -698,7 +708,7 @@ __device__ __forceinline__ void align_packed(const AlignArgs& a, unsigned char* 
       // 2 k + kZero of the diagonals at word w: kw0 + 4 w in each half, below
       // 2^16, so plain adds carry nothing
       const uint32_t kw0 = (uint32_t)((int)kZero + 2 * kbase) + ((uint32_t)((int)kZero + 2 * kbase + 2) << 16);
-      PackedSteps<kModel> steps;
+      PackedSteps<kModel, kDeep> steps;
       steps.begin(a.pen, tab_m, (rows - 1) * RB);
       PackedRows r{};
       // With a bound: a path on diagonal k at score s still pays at least one
@@ -872,7 +882,7 @@ __device__ __forceinline__ void align_packed(const AlignArgs& a, unsigned char* 
 // whatever the pair: a latency chain of about 0.3 us per score, 1/20 of the
 // work of the full wavefronts of a 10 kbp pair at 15 %, for which it halves
 // the cells (see align_packed).
-template <int kModel>
+template <int kModel, bool kDeep>
 __device__ __forceinline__ void probe_packed(const ProbeArgs& a, unsigned char* smem_raw) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr uint32_t kZero = kZeroBound;
@@ -916,7 +926,7 @@ __device__ __forceinline__ void probe_packed(const ProbeArgs& a, unsigned char* 
       const int s_max = (int)(sb < INT_MAX - 1 ? sb : INT_MAX - 1);
       const PackedPair pp{pws, tws, h2_dup(2 * (uint32_t)m), h2_dup((uint32_t)((int)kZero + 2 * k_end))};
       const uint32_t end_val = 2 * (uint32_t)n + kZero;
-      PackedSteps<kModel> steps;
+      PackedSteps<kModel, kDeep> steps;
       steps.begin(a.pen, tables, (rows - 1) * RB);
       PackedRows r{};
       for (int s = 1; s <= s_max && found == kNoBound; ++s) {

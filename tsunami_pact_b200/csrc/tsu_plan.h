@@ -16,9 +16,12 @@
 
 namespace tsu {
 
-// A rung of the pass ladder: ring mode and warps per pair.
+// A rung of the pass ladder: ring mode and warps per pair; single: on the
+// shared ring, the kernel of one diagonal per thread whatever the pairs
+// (shared_single).
 struct PassChoice {
   int mode, gw;
+  bool single = false;
 };
 
 struct PassGeom {
@@ -26,7 +29,6 @@ struct PassGeom {
   int gw = 1;              // warps per pair
   int cta_threads = 128;   // threads per block
   int groups_per_cta = 4;  // pairs in flight per block
-  int min_blocks = 6;      // blocks per SM the kernel is compiled for
   int ring_w = 0;          // diagonals per ring slot
   int seq_cap = 0;         // staged sequence words per group (shared mode)
   int64_t hist_cap = 0;    // backtrace words per group
@@ -36,6 +38,7 @@ struct PassGeom {
   int ckpt_k = 0;          // low-memory mode: checkpoint interval (0: off)
   int ckpt_cap = 0;        // checkpoints per group
   int64_t ckpt_bytes = 0;  // bytes per checkpoint
+  bool single = false;     // shared ring, one diagonal per thread (shared_single)
   bool bounded = false;    // pairs with score bounds (plan_bounded, plan_wide)
   int wide_cell = 0;       // of these, the wide kernel's: bytes of a ring cell (2 or 4)
   int cluster = 1;         // blocks per pair (wide kernel)
@@ -44,13 +47,14 @@ struct PassGeom {
 constexpr int kSharedW1 = 384;         // shared-mode ring width for one warp per pair (diagonals)
 constexpr int kSharedSeqWords1 = 544;  // staging area for one warp per pair (uint32 words)
 constexpr int kSharedSeqWordsN = 4096; // staging area for a group of warps
-constexpr int kSharedMaxLen = 32000;   // int16 ring limit of the low-memory kernels
+constexpr int kSharedMaxLen = 32000;   // int16 ring limit
 // A launch of the packed kernel takes pairs up to the end of their length
 // band; the few beyond kPackedPlainLen are handed back one by one.
 constexpr int kPackedBandLen = 16383;
-// widest shared ring (kPackedMaxW; the low-memory kernels' int16 ring holds
-// 16,368: a negative I value grows by one per diagonal and must stay negative)
-constexpr int kSharedMaxW = kPackedMaxW;
+// widest int16 ring of one diagonal per thread: a negative (invalid) I value
+// grows by one per diagonal of the ring's width and must stay negative (the
+// kernel's store clamp); the packed kernel's: kPackedMaxW
+constexpr int kSharedMaxW = 16368;
 constexpr int kSmemPerSM = 228 * 1024; // B200 shared memory per SM (bytes)
 
 // Reduced-unit score expected at edit rate `hint` for a pair of length L.
@@ -60,19 +64,33 @@ inline int64_t hint_score(const Pen& pen, int64_t L, double hint) {
 
 inline int cta_threads_for(int gw) { return gw <= 4 ? 128 : 32 * gw; }
 inline int min_blocks_for(int mode, int gw) {
-  return mode == kModeShared ? (gw == 1 ? 7 : (gw <= 4 ? 6 : (gw == 8 ? 3 : 1))) : (gw <= 4 ? 4 : (gw == 8 ? 2 : 1));
+  return mode == kModeShared ? (gw <= 4 ? 6 : (gw == 8 ? 3 : 1)) : (gw <= 4 ? 4 : (gw == 8 ? 2 : 1));
+}
+
+// Whether a shared-ring launch over sides of up to maxlen runs the kernel of
+// one diagonal per thread: rings deeper than the packed kernel's record of
+// scores, and sides past its offsets.  (One warp stages at most 8,700 bases of
+// both sides and hands longer pairs back either way: packed.)  Scores alone of
+// the deepest rings go to the global ring instead, which holds more pairs (5,000
+// pairs of 1 kbp at 1 and 5 %, penalties 5/200/4, shared against global: with
+// CIGARs 50 and 234 ms, 97 and 922; scores 37 and 189, 12 and 93).  Depths of 65
+// - 128 in the packed kernel, with bounds, against this one: 20,000 x 1 kbp,
+// 5/60/4, 7.8 and 47 ms, 21 and 341; scores 7.1 and 38, 14 and 285.
+inline bool shared_single(const Pen& pen, int64_t maxlen, int gw) {
+  return !packed_fits(pen) || (gw > 1 && maxlen > kPackedBandLen);
 }
 
 // Ring width a shared-mode group of gw warps can hold with seq_cap staged
-// words, at the block count the kernel is compiled for.
-inline int shared_ring_width(const Pen& pen, int gw, int seq_cap, int smem_optin) {
+// words, at the block count the kernel is compiled for (packed: two diagonals
+// per thread).
+inline int shared_ring_width(const Pen& pen, int gw, int seq_cap, int smem_optin, bool packed) {
   const int ns = pen.slots();
   const int blocks = min_blocks_for(kModeShared, gw);
   const int per_cta = std::min(smem_optin, kSmemPerSM / blocks - 1024);
   const int gpc = cta_threads_for(gw) / (32 * gw);
   const int per_group = per_cta / gpc;
-  const int fixed = group_smem_bytes(pen, 0, kModeShared, seq_cap, gw) + 16;
-  const int w = std::min((per_group - fixed) / (2 * (ns + 1)), kSharedMaxW);
+  const int fixed = group_smem_bytes(pen, 0, kModeShared, seq_cap, gw, packed) + 16;
+  const int w = std::min((per_group - fixed) / (2 * (packed ? ns + 1 : ns)), packed ? kPackedMaxW : kSharedMaxW);
   return std::max(0, w & ~15);
 }
 
@@ -80,20 +98,21 @@ inline int shared_ring_width(const Pen& pen, int gw, int seq_cap, int smem_optin
 // width (kSharedW1), unless penalties with a very deep ring leave four such
 // groups unable to fit one block; then the width one block can hold (below
 // 64 diagonals the pass takes the global ring).
-inline int shared_cap(const Pen& pen, int gw, int seq_cap, int smem_optin) {
-  if (gw != 1) return shared_ring_width(pen, gw, seq_cap, smem_optin);
+inline int shared_cap(const Pen& pen, int gw, int seq_cap, int smem_optin, bool packed) {
+  if (gw != 1) return shared_ring_width(pen, gw, seq_cap, smem_optin, packed);
   const int gpc = cta_threads_for(1) / 32;
-  if (gpc * group_smem_bytes(pen, kSharedW1, kModeShared, seq_cap, 1) <= smem_optin) return kSharedW1;
-  const int w = (smem_optin / gpc - group_smem_bytes(pen, 0, kModeShared, seq_cap, 1) - 16) / (2 * (pen.slots() + 1));
+  if (gpc * group_smem_bytes(pen, kSharedW1, kModeShared, seq_cap, 1, packed) <= smem_optin) return kSharedW1;
+  const int w = (smem_optin / gpc - group_smem_bytes(pen, 0, kModeShared, seq_cap, 1, packed) - 16) /
+                (2 * (pen.slots() + (packed ? 1 : 0)));
   return std::max(0, w & ~15);
 }
 
 // mode/gw: the configuration of this pass.  Shared mode needs lengths within
 // the int16 ring; otherwise the pass falls back to the global ring.
 // low_mem (CIGAR passes): 0 off; > 0 checkpoint every low_mem scores; < 0
-// an interval chosen here.
+// an interval chosen here.  single: PassChoice::single.
 inline PassGeom plan_geometry(const Pen& pen, int32_t max_m, int32_t max_n, int mode, int gw, double hint,
-                              bool want_cigar, int smem_optin, int low_mem = 0) {
+                              bool want_cigar, int smem_optin, int low_mem = 0, bool single = false) {
   PassGeom p;
   const bool lowmem = want_cigar && low_mem != 0;
   const int ns = pen.slots();
@@ -105,14 +124,16 @@ inline PassGeom plan_geometry(const Pen& pen, int32_t max_m, int32_t max_n, int 
   p.gw = gw;
   p.cta_threads = cta_threads_for(gw);
   p.groups_per_cta = p.cta_threads / (32 * gw);
-  const bool fits = lowmem ? maxlen <= kSharedMaxLen : (maxlen <= kPackedBandLen && pen.rm <= kPackedMaxDepth);
-  p.mode = (mode == kModeShared && fits) ? kModeShared : kModeGlobal;
+  const bool fits = maxlen <= kSharedMaxLen && (want_cigar || packed_fits(pen));
+  p.mode = mode == kModeShared && fits ? kModeShared : kModeGlobal;
+  p.single = p.mode == kModeShared && !lowmem && (single || shared_single(pen, maxlen, gw));
+  const bool packed = p.mode == kModeShared && !lowmem && !p.single;
   if (p.mode == kModeShared) {
     const int64_t seqw = 2 * packed_words(max_m) + 2 * packed_words(max_n);
     p.seq_cap = (int)std::min<int64_t>(seqw, gw == 1 ? kSharedSeqWords1 : kSharedSeqWordsN);
-    const int cap = shared_cap(pen, gw, p.seq_cap, smem_optin);
+    const int cap = shared_cap(pen, gw, p.seq_cap, smem_optin, packed);
     p.ring_w = (int)std::max<int64_t>(16, (std::min<int64_t>(full_w, cap) + 15) & ~15);
-    if (cap < 64) p.mode = kModeGlobal;
+    if (cap < 64) p.mode = kModeGlobal, p.single = false;
   }
   if (p.mode == kModeGlobal) {
     p.ring_w = (int)full_w;
@@ -122,11 +143,10 @@ inline PassGeom plan_geometry(const Pen& pen, int32_t max_m, int32_t max_n, int 
     const int64_t seqw = 2 * packed_words(max_m) + 2 * packed_words(max_n);
     const int per_cta = std::min(smem_optin, kSmemPerSM / min_blocks_for(kModeGlobal, gw) - 1024);
     const int gpc = cta_threads_for(gw) / (32 * gw);
-    const int64_t room = per_cta / gpc - group_smem_bytes(pen, 0, kModeGlobal, 0, gw) - 48;
+    const int64_t room = per_cta / gpc - group_smem_bytes(pen, 0, kModeGlobal, 0, gw, false) - 48;
     p.seq_cap = (gw < 32 && seqw * 4 <= room) ? (int)seqw : 0;
   }
-  p.min_blocks = min_blocks_for(p.mode, gw);
-  p.group_smem = group_smem_bytes(pen, p.ring_w, p.mode, p.seq_cap, gw);
+  p.group_smem = group_smem_bytes(pen, p.ring_w, p.mode, p.seq_cap, gw, packed);
   // Backtrace words up to score s: sum_j (2j/ge + 1) ~= s^2/ge + 2s.
   p.table_cap = want_cigar ? (int)std::min<int64_t>(s_hint + 1, INT32_MAX / 2) : 0;
   if (want_cigar) {
@@ -134,7 +154,7 @@ inline PassGeom plan_geometry(const Pen& pen, int32_t max_m, int32_t max_n, int 
     int64_t cells = std::min<int64_t>(sq, (s_hint + 1) * width_hint);
     // the packed kernel keeps 4 bits per cell (8 with two gap pieces), each
     // score's row rounded out to whole words at both ends
-    if (p.mode == kModeShared && !lowmem) cells = std::min<int64_t>(cells / (pen.dual() ? 4 : 8) + 3 * (s_hint + 1) + 64, INT32_MAX - 65536);
+    if (packed && p.mode == kModeShared) cells = std::min<int64_t>(cells / (pen.dual() ? 4 : 8) + 3 * (s_hint + 1) + 64, INT32_MAX - 65536);
     p.hist_cap = std::min<int64_t>(cells, INT32_MAX - 64);
   }
   p.ring_ints = p.mode == kModeShared ? 0 : (int64_t)ns * p.ring_w;
@@ -167,15 +187,21 @@ inline PassGeom plan_geometry(const Pen& pen, int32_t max_m, int32_t max_n, int 
 inline PassChoice next_pass(PassChoice prev, const Pen& pen, int32_t max_m, int32_t max_n, int smem_optin,
                             int global_gw = 16) {
   const int64_t need_w = (int64_t)max_m + max_n + 3;
-  if (prev.mode == kModeShared && std::max(max_m, max_n) <= kPackedPlainLen && pen.rm <= kPackedMaxDepth) {
+  const int64_t maxlen = std::max(max_m, max_n);
+  if (prev.mode == kModeShared && maxlen <= kSharedMaxLen) {
+    // sides past the packed kernel's offsets, handed back by it: the kernel of
+    // one diagonal per thread, from the same warps on
+    const bool single = prev.single || maxlen > kPackedPlainLen;
+    const int least = maxlen > kPackedPlainLen && !prev.single && !shared_single(pen, maxlen, prev.gw) ? prev.gw : prev.gw + 1;
+    const bool packed = !single && packed_fits(pen);
     const int64_t seqw =
         std::min<int64_t>(2 * packed_words(max_m) + 2 * packed_words(max_n), kSharedSeqWordsN);
     static const int kGW[] = {2, 4, 8, 16};
     for (int gw : kGW) {
-      if (gw <= prev.gw) continue;
-      if (shared_ring_width(pen, gw, (int)seqw, smem_optin) >= need_w) return {kModeShared, gw};
+      if (gw < least) continue;
+      if (shared_ring_width(pen, gw, (int)seqw, smem_optin, packed) >= need_w) return {kModeShared, gw, single};
     }
-    if (prev.gw < 16) return {kModeShared, 16};
+    if (least <= 16) return {kModeShared, 16, single};
   }
   return {kModeGlobal, global_gw};
 }
@@ -192,13 +218,13 @@ inline PassChoice fit_start(PassChoice pc, const Pen& pen, int32_t max_m, int32_
   const int64_t w =
       std::min<int64_t>((int64_t)max_m + max_n + 3, 2 * hint_score(pen, maxlen, hint) / pen.min_ge() + 3);
   if (pc.mode != kModeShared) return {kModeGlobal, w > 16384 ? 32 : pc.gw};
-  if (maxlen > kPackedPlainLen || pen.rm > kPackedMaxDepth) return {kModeGlobal, w > 16384 ? 32 : std::max(8, pc.gw)};
+  if (maxlen > kSharedMaxLen) return {kModeGlobal, w > 16384 ? 32 : std::max(8, pc.gw)};
   const int64_t seqw = 2 * packed_words(max_m) + 2 * packed_words(max_n);
   static const int kGW[] = {1, 2, 4, 8, 16};
   for (int gw : kGW) {
     if (gw < pc.gw) continue;
     if (seqw > (gw == 1 ? kSharedSeqWords1 : kSharedSeqWordsN)) continue;
-    const int cap = shared_cap(pen, gw, (int)seqw, smem_optin);
+    const int cap = shared_cap(pen, gw, (int)seqw, smem_optin, !shared_single(pen, maxlen, gw));
     if (cap >= w && cap >= 64) return {kModeShared, gw};
   }
   // wavefronts wider than 16,384 diagonals: 32 warps (one 1024-thread block)
@@ -222,7 +248,7 @@ inline int length_band(int32_t L) {
 // compiled one), adjusted for lengths beyond the int16 shared ring.
 inline PassChoice band_start_in(const PassChoice* table, int band, int32_t maxlen) {
   PassChoice r = table[band < 0 ? 0 : (band >= kBands ? kBands - 1 : band)];
-  if (r.mode == kModeShared && maxlen > kPackedBandLen) r = {kModeGlobal, r.gw >= 8 ? r.gw : 8};
+  if (r.mode == kModeShared && maxlen > kSharedMaxLen) r = {kModeGlobal, r.gw >= 8 ? r.gw : 8};
   return r;
 }
 inline const PassChoice* band_start_table(bool dual = false) {
@@ -291,7 +317,7 @@ inline BoundLimits bound_limits(const Pen& pen, int smem_optin) {
   b.side = from(kBoundMinWidth, 0.04);
   const int64_t d = kBoundMinRing / (2 * ((int64_t)pen.slots() + 1)) + 1;  // diagonals that take more than kBoundMinRing
   if (d <= kSharedW1) b.sum = (int32_t)std::max<int64_t>(d - 3, 1);
-  b.few_side = from(std::max(shared_ring_width(pen, 16, kSharedSeqWordsN, smem_optin), 64), 0.163);
+  b.few_side = from(std::max(shared_ring_width(pen, 16, kSharedSeqWordsN, smem_optin, true), 64), 0.163);
   return b;
 }
 
@@ -325,7 +351,6 @@ inline PassGeom plan_bounded(int bytes, int32_t max_ub, int64_t hist, int gw, bo
   p.gw = gw;
   p.cta_threads = cta_threads_for(gw);
   p.groups_per_cta = p.cta_threads / (32 * gw);
-  p.min_blocks = min_blocks_for(kModeShared, gw);
   p.group_smem = bytes;
   if (want_cigar) {
     p.table_cap = max_ub + 2;
@@ -378,7 +403,6 @@ inline PassGeom plan_wide(const Pen& pen, int32_t max_n, int width, int32_t max_
   p.gw = 16;
   p.cta_threads = 512;
   p.groups_per_cta = 1;
-  p.min_blocks = 1;
   p.group_smem = wide_smem_bytes(pen);
   p.ring_ints = (int64_t)(pen.slots() + 1) * wide_row_bytes(width, p.wide_cell) / 4;
   if (want_cigar) {
@@ -423,9 +447,10 @@ inline PassChoice few_start(PassChoice pc, const Pen& pen, int32_t maxlen) {
 // outgrow), else those of the rung, doubled while the launch leaves an SM
 // fewer than 8 warps (600 pairs of 1 kbp: 0.22 ms on 1, 0.19 on 2, 0.26 on 4);
 // at most one warp per 64 bases beyond the rung (20 pairs of 115 bp: 162 us a
-// call on 1 warp, 168 on 16).
-inline PassChoice fill_warps(PassChoice pc, int64_t n, int32_t maxlen, int sms) {
-  if (pc.mode != kModeShared) return pc;
+// call on 1 warp, 168 on 16).  The kernel of one diagonal per thread keeps its
+// rung.
+inline PassChoice fill_warps(PassChoice pc, const Pen& pen, int64_t n, int32_t maxlen, int sms) {
+  if (pc.mode != kModeShared || pc.single || shared_single(pen, maxlen, pc.gw)) return pc;
   while (pc.gw < 16 && (n <= sms || n * pc.gw * 2 <= (int64_t)sms * 8) && pc.gw * 128 <= maxlen) pc.gw *= 2;
   return pc;
 }

@@ -181,7 +181,7 @@ __device__ __forceinline__ void cluster_sts32(smem_t a, unsigned rank, uint32_t 
 // cluster each block computes every csize-th run of words of a score, reads
 // the ring past L1, and a cluster barrier ends the score (11 pairs of 21 - 50
 // kbp: 201 ms one block each, 78 ms on clusters of 8).
-template <bool kCigar, int kModel, typename ST, bool kCluster>
+template <bool kCigar, int kModel, typename ST, bool kCluster, bool kDeep = true>
 __device__ __forceinline__ void align_wide(const AlignArgs& a, unsigned char* smem_raw) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int GW = 16, U = 4;
@@ -256,7 +256,7 @@ __device__ __forceinline__ void align_wide(const AlignArgs& a, unsigned char* sm
       const int64_t bound = score_bound(m, n, a.pen);
       const int s_max = (int)(bound < INT_MAX - 1 ? bound : INT_MAX - 1);
       const int s_lim = min(ub, kCigar ? min(s_max, a.table_cap - 1) : s_max);
-      PackedSteps<kModel> steps;
+      PackedSteps<kModel, kDeep> steps;
       steps.begin(a.pen, tables, (rows - 1) * RB);
       PackedRows r{};
       const int gem = a.pen.min_ge();
@@ -378,7 +378,7 @@ __device__ __forceinline__ void align_wide(const AlignArgs& a, unsigned char* sm
 
 // probe_packed (tsu_packed.cuh) for pairs of any length: the same window of
 // kProbeW diagonals, 32-bit cells in shared memory, sequences through L1.
-template <int kModel>
+template <int kModel, bool kDeep = true>
 __device__ __forceinline__ void probe_wide(const ProbeArgs& a, unsigned char* smem_raw) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int W = kProbeW, U = W / 32;
@@ -412,7 +412,7 @@ __device__ __forceinline__ void probe_wide(const ProbeArgs& a, unsigned char* sm
       }
       const int64_t sb = score_bound(m, n, a.pen);
       const int s_max = (int)(sb < INT_MAX - 1 ? sb : INT_MAX - 1);
-      PackedSteps<kModel> steps;
+      PackedSteps<kModel, kDeep> steps;
       steps.begin(a.pen, tables, (rows - 1) * RB);
       PackedRows r{};
       for (int s = 1; s <= s_max && found == kNoBound; ++s) {
