@@ -58,10 +58,8 @@ __device__ __forceinline__ uint32_t h2_signmask(uint32_t a) {
 }
 // trailing zero bits, 32 for 0
 __device__ __forceinline__ int h2_tz(uint32_t d) { return __clz((int)__brev(d)); }
-// acc + both halves (below 2^15 each)
-__device__ __forceinline__ uint32_t h2_sum(uint32_t a, uint32_t acc) {
-  return (uint32_t)__dp2a_lo((int)a, 0x0101, (int)acc);
-}
+// acc + both halves (unsigned: twice the bases of a match run, up to 40,926)
+__device__ __forceinline__ uint32_t h2_sum(uint32_t a, uint32_t acc) { return __dp2a_lo(a, 0x0101u, acc); }
 #endif
 __device__ __forceinline__ uint32_t h2_dup(uint32_t v) { return (v & 0xffffu) * 0x10001u; }
 
