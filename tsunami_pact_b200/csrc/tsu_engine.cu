@@ -1549,7 +1549,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     std::vector<int32_t> order;
     const size_t fixed = ctx->held() - ctx->b_scratch.cap + out_reserve();
     const size_t avail = ctx->budget > fixed ? ctx->budget - fixed : 0;
-    size_t need_bytes = 0, each = 0;
+    size_t need_bytes = 0, each = 0, plain_most = 0;
     int rc2;
     for (int c = kAll - 1, done = 0; done < kAll; ++done, c = c == kWide ? 0 : (c < kWide ? c + 1 : c - 1)) {
       // bands without a bound first (longest first), the wide kernel's, then
@@ -1575,6 +1575,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
           Pass old;
           if (plan_pass_within(ctx, r.bi, r.n, plain, r.hint, want_cigar, avail, &old) == TSU_OK)
             room = std::min(room, (size_t)old.groups * group_scratch_bytes(old.g));
+          plain_most = std::max(plain_most, room);
         }
         tsu::PassGeom g;
         if (c < kWide) {
@@ -1603,9 +1604,12 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     }
     // The launches run side by side, each in its own part of the scratch, so
     // that one class's last pairs and the next one's first share the SMs; one
-    // after the other when the budget does not hold them all at once, or the
-    // context keeps to one stream (the request server's workers).
-    const bool side = runs.size() - first > 1 && each <= avail && ctx->h2d_stream != ctx->stream;
+    // after the other when the budget (in low-memory mode: the largest of the
+    // launches without bounds, which ran one after the other) does not hold
+    // them all at once, or the context keeps to one stream (the request
+    // server's workers).
+    const bool side = runs.size() - first > 1 && each <= (low_mem ? std::min(avail, plain_most) : avail) &&
+                      ctx->h2d_stream != ctx->stream;
     if (side) need_bytes = each;
     if (need_bytes > ctx->b_scratch.cap) {
       release(ctx, ctx->b_scratch);
