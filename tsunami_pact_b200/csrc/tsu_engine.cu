@@ -47,6 +47,11 @@ struct HostBuf {
 // pairs with a score bound and the bands of pairs whose bound did not help,
 // the latter twice (pairs bounded at once, pairs bounded after a first pass).
 constexpr int kRunSlots = tsu::kBands + 2 * (tsu::kBoundClasses + 2 + tsu::kBands);
+// Counters of a call on the device, and page-locked copies of small results on
+// the host (tsu_ctx::h_scalars): the counters, then the number of runs.
+constexpr size_t kCounterBytes = 64 + 8 * kRunSlots;
+constexpr size_t kScalarRuns = 2048, kScalarBytes = 4096;
+static_assert(kCounterBytes <= kScalarRuns && kScalarRuns + 8 <= kScalarBytes, "h_scalars");
 // Streams beside the context's own for the launches of bounded classes.
 constexpr int kSideStreams = 3;
 
@@ -100,7 +105,7 @@ struct tsu_ctx {
   // statuses) go through page-locked buffers: a copy to or from pageable
   // memory blocks the calling thread inside the driver until its stream
   // reaches it, and several host threads' contexts then run one at a time.
-  HostBuf h_scalars;  // 64 bytes: retry count, arena cursor, work counters, run total
+  HostBuf h_scalars;  // kScalarBytes: counters of a call, number of runs
   HostBuf h_list;     // int32 pass order / retry list
   HostBuf h_status;   // int32 pair statuses (tsu_align_batch)
   HostBuf h_bidir;    // bidirectional mode: segments down, cuts and run counts up
@@ -1279,7 +1284,6 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   if ((rc = grow(ctx, ctx->b_order, sizeof(int32_t) * 2 * n))) return rc;
   // counters: +8 the bound probe's queue head, +16 arena cursor, +24 work (cells, steps, extension bases), +64 + 8b queue head
   // and retry count of band slot b
-  constexpr size_t kCounterBytes = 64 + 8 * kRunSlots;
   constexpr size_t kProbeQueue = 8;  // the bound probes' queue heads (wide, packed)
   if ((rc = grow(ctx, ctx->b_counters, kCounterBytes))) return rc;
   // Pairs with a bound probe (tsu::wants_bound; end to end, history of every
@@ -1657,7 +1661,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
 
   // Run offsets of the pairs (scan of their run counts into d_out_off, the
   // total to h_total), and the runs gathered into `runs` when they fit cap.
-  int64_t* const h_total = reinterpret_cast<int64_t*>(static_cast<char*>(ctx->h_scalars.p) + 2048);
+  int64_t* const h_total = reinterpret_cast<int64_t*>(static_cast<char*>(ctx->h_scalars.p) + kScalarRuns);
   auto queue_offsets = [&]() -> int {
     tsu::cig_len64_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, st>>>(
         n, P<int32_t>(ctx->b_clen), d_status, P<int64_t>(ctx->b_clen64));
@@ -2200,7 +2204,7 @@ int create(const Spec& spec, const tsu_config* cfg, bool single_stream, tsu_ctx*
     const char* gv = getenv("TSU_GRAPH");
     ctx->use_graph = !(gv && gv[0] == '0');
   }
-  if (!ctx->pool || host_grow(ctx, ctx->h_scalars, 512) != TSU_OK) {
+  if (!ctx->pool || host_grow(ctx, ctx->h_scalars, kScalarBytes) != TSU_OK) {
     tsu_destroy(ctx);
     return TSU_EDEVICE;
   }
