@@ -1380,7 +1380,11 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     double hint = 0;
     Pass ps;
     bool few = false;      // few long pairs: those that outgrow it get a bound
-    bool rebound = false;  // the pairs that outgrew it have run again with bounds
+    // the pairs that outgrew it have run again with bounds; the ones that the
+    // shared rings cannot take at all are left for the ladder
+    bool rebound = false;
+    std::vector<int32_t> left;
+    bool all_bytes = false;  // what the ladder gets are pairs with bytes outside ACGT
   };
   BandSplit split;
   if (!ctx->one_warp && h_plen) split_bands(n, h_plen, h_tlen, &split, &bi);
@@ -1731,32 +1735,43 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   }
   ctx->timing.kernel_launches += 3 + (int64_t)runs.size() + (probe.n_wide ? 1 : 0) + (n_probed > probe.n_wide ? 1 : 0);
   CU(early_ev ? cudaEventSynchronize(early_ev) : wait_stream(ctx, st));
+  const size_t first_runs = runs.size();  // the ones of pairs that were not probed
   if (n_probed) {
     if ((rc = fetch_bounds()) || (rc = bounded_runs(probed, probe_off))) return rc;
   }
   // Pairs that outgrew an unbounded shared ring get a bound, and a second
   // start with it: 20,000 pairs of 800 - 1,000 bp at 10 % took 13.2 ms through
   // the ladder.  (Few of them, whose full wavefronts fit 16 warps' ring: the
-  // ladder's 16 warps are as good.)
+  // ladder's 16 warps are as good.)  Pairs with bytes outside ACGT, which every
+  // shared ring hands back and no probe takes, go on to the ladder, and there
+  // to the global ring when they are among more than the SMs.
   bool rebound_any = false;
   if (can_bound) {
     std::vector<int32_t> again;
-    const size_t first_runs = runs.size();
+    std::vector<uint8_t> bytes;  // [2 n] once fetched: sequences with bytes outside ACGT
     for (size_t j = 0; j < first_runs; ++j) {
       BandRun& r = runs[j];
       const unsigned int c = *reinterpret_cast<const unsigned int*>(h_cnt + 64 + 8 * r.slot + 4);
-      if (!c || r.ps.g.bounded || r.ps.g.mode != tsu::kModeShared) continue;
+      if (!c || r.ps.g.mode != tsu::kModeShared || !(r.few || c > (unsigned)ctx->sms)) continue;
       if ((rc = host_grow(ctx, ctx->h_list, sizeof(int32_t) * c))) return rc;
       CU(cudaMemcpyAsync(ctx->h_list.p, P<int32_t>(ctx->b_retry) + r.off, sizeof(int32_t) * c, cudaMemcpyDeviceToHost, st));
+      if (bytes.empty()) {
+        bytes.resize(2 * (size_t)n);
+        CU(cudaMemcpyAsync(bytes.data(), ctx->b_nonacgt.p, 2 * (size_t)n, cudaMemcpyDeviceToHost, st));
+      }
       CU(wait_stream(ctx, st));
       const int32_t* l = static_cast<const int32_t*>(ctx->h_list.p);
       const size_t before = again.size();
-      for (unsigned int i = 0; i < c; ++i)
-        if (std::min(h_plen[l[i]], h_tlen[l[i]]) > 0) again.push_back(l[i]);
-      if (again.size() - before == c && (r.few || c > (unsigned)ctx->sms))
-        r.rebound = true;  // all of them
-      else
-        again.resize(before);
+      size_t n_bytes = 0;
+      for (unsigned int i = 0; i < c; ++i) {
+        const bool b = (bytes[(size_t)l[i]] | bytes[(size_t)(n + l[i])]) != 0;
+        n_bytes += b;
+        (b || std::min(h_plen[l[i]], h_tlen[l[i]]) == 0 ? r.left : again).push_back(l[i]);
+      }
+      const size_t found = again.size() - before;
+      r.rebound = r.few ? found > 0 : found > (size_t)ctx->sms;
+      r.all_bytes = n_bytes == (r.rebound ? r.left.size() : (size_t)c);
+      if (!r.rebound) again.resize(before);
     }
     ProbePlan p;
     const size_t asked = again.size();
@@ -1774,12 +1789,16 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       rebound_any = true;
       if ((rc = fetch_bounds()) || (rc = bounded_runs(again, n))) return rc;
     } else {
-      for (BandRun& r : runs) r.rebound = false;
+      for (BandRun& r : runs) {
+        r.all_bytes = r.all_bytes && !r.rebound;
+        r.rebound = false;
+      }
     }
   }
   std::vector<unsigned int> first_retry(runs.size());
   for (const BandRun& r : runs) {
-    first_retry[(size_t)r.slot] = r.rebound ? 0u : *reinterpret_cast<const unsigned int*>(h_cnt + 64 + 8 * r.slot + 4);
+    first_retry[(size_t)r.slot] = r.rebound ? (unsigned int)r.left.size()
+                                            : *reinterpret_cast<const unsigned int*>(h_cnt + 64 + 8 * r.slot + 4);
     log_pass(r.ps, r.n);
     char t[48];
     snprintf(t, sizeof t, "@%.1fms", ev_ms(ctx->bev[2 * r.slot], ctx->bev[2 * r.slot + 1]));
@@ -1811,11 +1830,16 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
                        nretry, passlog.c_str());
       // The retry list, longest pairs first, becomes the next pass's order;
       // its lengths pick the next rung.  Global passes grow the hint.
-      rlist.resize(nretry);
+      const bool first = passes == band_first_pass + 1;
       if ((rc = host_grow(ctx, ctx->h_list, sizeof(int32_t) * nretry))) return rc;
-      CU(cudaMemcpyAsync(ctx->h_list.p, d_retry, sizeof(int32_t) * nretry, cudaMemcpyDeviceToHost, st));
-      CU(wait_stream(ctx, st));
-      memcpy(rlist.data(), ctx->h_list.p, sizeof(int32_t) * nretry);
+      if (first && r.rebound) {
+        rlist = r.left;
+      } else {
+        rlist.resize(nretry);
+        CU(cudaMemcpyAsync(ctx->h_list.p, d_retry, sizeof(int32_t) * nretry, cudaMemcpyDeviceToHost, st));
+        CU(wait_stream(ctx, st));
+        memcpy(rlist.data(), ctx->h_list.p, sizeof(int32_t) * nretry);
+      }
       BatchInfo pbi;
       pbi.n = nretry;
       for (int32_t i : rlist) {
@@ -1827,8 +1851,9 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       memcpy(ctx->h_list.p, rlist.data(), sizeof(int32_t) * nretry);
       CU(cudaMemcpyAsync(d_order, ctx->h_list.p, sizeof(int32_t) * nretry, cudaMemcpyHostToDevice, st));
       hint = tsu::next_hint(hint, last_mode == tsu::kModeGlobal);
-      pc = ctx->one_warp ? tsu::PassChoice{tsu::kModeGlobal, 1}
-                         : tsu::next_pass(pc, ctx->rp, pbi.max_m, pbi.max_n, ctx->smem_optin);
+      pc = ctx->one_warp             ? tsu::PassChoice{tsu::kModeGlobal, 1}
+           : first && r.all_bytes    ? tsu::PassChoice{tsu::kModeGlobal, 16}
+                                     : tsu::next_pass(pc, ctx->rp, pbi.max_m, pbi.max_n, ctx->smem_optin);
       if (want_cigar) {
         unsigned long long* h_used = reinterpret_cast<unsigned long long*>(h_cnt + 16);
         CU(cudaMemcpyAsync(h_used, d_cursor, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
