@@ -195,8 +195,11 @@ const char* tsu_pass_log(const tsu_ctx* ctx);
  * ring in shared memory (mode 0) or in device memory (mode 1), with 1, 2, 4,
  * 8, 16 or 32 warps per pair.  A context starts from the table compiled in
  * (tsu_tuning.h, written by the autotuner tsunami_pact_b200/tune.py); these
- * calls read and change the context's copy.  Pairs that outgrow a rung are
- * retried at the next one, so a rung never changes a result.  No
+ * calls read and change the context's copy.  A context chooses for itself where
+ * a band's first pass starts when the call has no more pairs than SMs, or pairs
+ * long enough for a score bound; a band whose rung was set starts there whatever
+ * the call.  Pairs that outgrow a rung are retried at the next one, or with a
+ * bound, so a rung never changes a result.  No
  * counterpart in the reference (one fixed launch shape, wfa_gpu.cu:113-114). */
 int tsu_set_band_start(tsu_ctx* ctx, int band, int mode, int warps_per_pair);
 

@@ -101,6 +101,7 @@ struct tsu_ctx {
   bool exact_grow = false;       // grow buffers to the asked size only
   bool fit_start = false;        // start rungs by the hint's predicted width (tsu::fit_start)
   tsu::PassChoice band_start[tsu::kBands] = {};  // starting rung per length band (tsu_set_band_start)
+  bool band_set[tsu::kBands] = {};               // set by the caller: first passes start there as it says
   // The engine's own host transfers (counters, pass orders, retry lists,
   // statuses) go through page-locked buffers: a copy to or from pageable
   // memory blocks the calling thread inside the driver until its stream
@@ -1332,7 +1333,8 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     if (low_mem) limits.side = std::min(limits.side, tsu::kBoundLowMemLen);
     if (bi.max_side >= limits.side || bi.max_sum >= limits.sum)
       for (int64_t i = 0; i < n; ++i)
-        if (limits.wants(h_plen[i], h_tlen[i])) probed.push_back((int32_t)i);
+        if (limits.wants(h_plen[i], h_tlen[i]) && !ctx->band_set[tsu::length_band(std::max(h_plen[i], h_tlen[i]))])
+          probed.push_back((int32_t)i);
     if ((int64_t)probed.size() <= ctx->sms && !low_mem) {
       few_side = limits.few_side;
       probed.erase(std::remove_if(probed.begin(), probed.end(),
@@ -1396,6 +1398,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     BandRun r;
     r.n = n;
     r.bi = bi;
+    r.band = split.uniform_band;
     r.pc = tsu::PassChoice{tsu::kModeShared, 1};
     if (!ctx->one_warp && h_plen) r.pc = tsu::band_start_in(ctx->band_start, split.uniform_band, std::max(bi.max_m, bi.max_n));
     runs.push_back(r);
@@ -1430,8 +1433,9 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       if (ctx->fit_start && !ctx->one_warp)
         r.pc = tsu::fit_start(r.pc, ctx->rp, r.bi.max_m, r.bi.max_n, r.hint, ctx->smem_optin);
       r.few = r.n <= ctx->sms && std::max(r.bi.max_m, r.bi.max_n) >= few_side;
-      if (r.few) r.pc = tsu::few_start(r.pc, ctx->rp, std::max(r.bi.max_m, r.bi.max_n));
-      if (!ctx->one_warp) r.pc = tsu::fill_warps(r.pc, ctx->rp, r.n, std::max(r.bi.max_m, r.bi.max_n), ctx->sms);
+      const bool as_set = ctx->band_set[r.band];
+      if (r.few && !as_set) r.pc = tsu::few_start(r.pc, ctx->rp, std::max(r.bi.max_m, r.bi.max_n));
+      if (!ctx->one_warp && !as_set) r.pc = tsu::fill_warps(r.pc, ctx->rp, r.n, std::max(r.bi.max_m, r.bi.max_n), ctx->sms);
       if ((rc = plan_pass_within(ctx, r.bi, r.n, r.pc, r.hint, want_cigar, avail, &r.ps))) return rc;
       need = std::max(need, scratch_bytes(r.ps, want_cigar));
     }
@@ -2634,6 +2638,7 @@ int tsu_set_band_start(tsu_ctx* ctx, int band, int mode, int warps_per_pair) {
       (gw != 1 && gw != 2 && gw != 4 && gw != 8 && gw != 16 && gw != 32))
     return set_err(ctx, TSU_EINVAL, "band %d, mode %d, %d warps per pair: not a rung", band, mode, gw);
   ctx->band_start[band] = tsu::PassChoice{mode, gw};
+  ctx->band_set[band] = true;
   return TSU_OK;
 }
 

@@ -433,8 +433,10 @@ constexpr int kBoundLowMemLen = 256;
 // ring / probe at once / this: gap-affine 4/6/2 of 12 kbp at 1 % 0.97 / 0.88 /
 // 0.53 ms, at 5 % 5.2 / 3.0 / 2.4, at 15 % 23 / 9.4 / 10.4; 4/6/2/24/1 of 1.2
 // kbp at 4 % 0.83 / - / 0.39, of 2.5 kbp at 10 % 8.3 / 2.3 / 1.9, of 9 kbp at
-// 1 % 8.0 / 1.2 / 0.74, at 4 % 40 / 4.1 / 5.8.  (A rung that the caller set
-// stays.)
+// 1 % 8.0 / 1.2 / 0.74, at 4 % 40 / 4.1 / 5.8: noisy pairs of little more than
+// the ring holds lose a part of the probe's gain, since the first ring's work is
+// thrown away (100 of 16 kbp at 15 %: 181 / 13.7 / 24.6).  Bands whose rung the
+// caller set keep it, here and in fill_warps, and are not probed.
 inline PassChoice few_start(PassChoice pc, const Pen& pen, int32_t maxlen) {
   const PassChoice d = band_start_in(band_start_table(pen.dual()), length_band(maxlen), maxlen);
   if (pc.mode == kModeGlobal && pc.mode == d.mode && pc.gw == d.gw && maxlen <= kPackedBandLen) return {kModeShared, 16};
