@@ -655,9 +655,9 @@ int bidir_pack(tsu_ctx* ctx, const tsu::SeqView& sv, const BatchInfo& bi, tsu::P
   size_t tb = tmp_bytes;
   CU(cub::DeviceScan::ExclusiveSum(ctx->b_scan_tmp.p, tb, P<int64_t>(ctx->b_words_cnt), P<int64_t>(ctx->b_woff),
                                    (int)(2 * n), st));
-  const int64_t pblocks = std::min<int64_t>((2 * n + 7) / 8, (int64_t)ctx->sms * 16);
-  tsu::pack_kernel<<<(int)pblocks, 256, 0, st>>>(sv, *pk);
-  tsu::pack_kernel<true><<<(int)pblocks, 256, 0, st>>>(sv, *pkr);
+  const int32_t maxlen = std::max(bi.max_m, bi.max_n);
+  tsu::launch_pack<false>(maxlen, ctx->sms, st, sv, *pk);
+  tsu::launch_pack<true>(maxlen, ctx->sms, st, sv, *pkr);
   CU(cudaGetLastError());
   CU(cudaEventRecord(ctx->ev[3], st));
   return TSU_OK;
@@ -1702,8 +1702,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     size_t tb = tmp_bytes;
     CU(cub::DeviceScan::ExclusiveSum(ctx->b_scan_tmp.p, tb, P<int64_t>(ctx->b_words_cnt), P<int64_t>(ctx->b_woff),
                                      (int)(2 * n), st));
-    const int64_t blocks = std::min<int64_t>((2 * n + 7) / 8, (int64_t)ctx->sms * 16);
-    tsu::pack_kernel<<<(int)blocks, 256, 0, st>>>(sv, pk);
+    tsu::launch_pack<false>(std::max(bi.max_m, bi.max_n), ctx->sms, st, sv, pk);
     CU(cudaGetLastError());
     CU(record(ctx, ctx->ev[3], st));
     if (!order_all.empty())

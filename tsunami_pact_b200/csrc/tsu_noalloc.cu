@@ -191,7 +191,7 @@ extern "C" int tsu_align_scores_noalloc(const tsu_penalties* pen, const tsu_batc
                         b->text_off,
                         b->text_len};
   const tsu::PackView pk{words, woff, nonacgt};
-  tsu::pack_kernel<<<(int)std::min<int64_t>((2 * n + 7) / 8, (int64_t)sms * 16), 256, 0, st>>>(sv, pk);
+  tsu::launch_pack<false>(std::max(max_m, max_n), sms, st, sv, pk);
   NA_CU(cudaGetLastError());
 
   // align passes: shared-memory ring first, then a global ring for the pairs
