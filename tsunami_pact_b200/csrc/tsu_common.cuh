@@ -197,6 +197,17 @@ struct ProbeArgs {
   unsigned int* queue;
 };
 
+// a / b towards 0, below 2^53 (on the host in floating point, where it is exact
+// there: 64-bit integer division was a third of the planning of a batch of
+// bounded pairs).
+__host__ __device__ inline int64_t div_small(int64_t a, int64_t b) {
+#ifdef __CUDA_ARCH__
+  return a / b;
+#else
+  return (int64_t)((double)a / (double)b);
+#endif
+}
+
 // Diagonals [lo, hi] that an end-to-end path of cost at most ub can visit,
 // and two more on each side: at score s up to g(s) from 0 (gap openings and
 // extensions) and up to (ub - s) / e from n - m; the two lines cross at lo and
@@ -206,8 +217,8 @@ __host__ __device__ inline void bound_reach(const Pen& p, int m, int n, int ub, 
   auto side = [&](int64_t k_end) -> int64_t {  // furthest diagonal towards k_end's positive side
     int64_t best = k_end > 0 ? k_end : 0;
     auto piece = [&](int64_t go, int64_t ge) {
-      const int64_t s = ((k_end - 1) * ge * e + (int64_t)ub * ge + go * e) / (ge + e);
-      const int64_t v = s >= go ? 1 + (s - go) / ge : 0;
+      const int64_t s = div_small((k_end - 1) * ge * e + (int64_t)ub * ge + go * e, ge + e);
+      const int64_t v = s >= go ? 1 + div_small(s - go, ge) : 0;
       if (v > best) best = v;
     };
     piece(p.go, p.ge);

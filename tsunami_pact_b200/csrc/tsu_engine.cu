@@ -307,7 +307,7 @@ struct BatchInfo {
   int64_t n = 0;
   int32_t max_m = 0, max_n = 0;
   int64_t total_words = 0;
-  // of the pairs' longer sides and of both sides (set by add())
+  // of the pairs' longer sides and of both sides' sums (set by add())
   int32_t min_side = INT32_MAX, max_side = 0, min_sum = INT32_MAX, max_sum = 0;
   int64_t len_sum = 0;
   void add(int32_t m, int32_t t) {
@@ -1287,7 +1287,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   // and retry count of band slot b
   constexpr size_t kProbeQueue = 8;  // the bound probes' queue heads (wide, packed)
   if ((rc = grow(ctx, ctx->b_counters, kCounterBytes))) return rc;
-  // Pairs with a bound probe (tsu::wants_bound; end to end, history of every
+  // Pairs with a bound probe (tsu::bound_limits; end to end, history of every
   // score): they wait for their bounds, the others start at once.
   const bool low_mem = want_cigar && ctx->low_mem < 0;
   const bool can_bound = !ctx->one_warp && h_plen && tsu::packed_fits(ctx->rp) &&
@@ -1301,12 +1301,20 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     size_t smem = 0, wide_smem = 0;
   };
   auto plan_probes = [&](std::vector<int32_t>* list, ProbePlan* p) -> int {
-    std::stable_sort(list->begin(), list->end(), [&](int32_t u, int32_t v) {
-      const bool wu = std::max(h_plen[u], h_tlen[u]) > tsu::kPackedMaxLen;
-      const bool wv = std::max(h_plen[v], h_tlen[v]) > tsu::kPackedMaxLen;
-      if (wu != wv) return wu;
-      return (int64_t)h_plen[u] + h_tlen[u] > (int64_t)h_plen[v] + h_tlen[v];
-    });
+    // (a counting sort by the leading five bits of both lengths' sum)
+    constexpr int kKeys = 32 * 16;
+    auto key = [&](int32_t i) -> int {
+      const uint32_t s = std::max((uint32_t)h_plen[i] + (uint32_t)h_tlen[i], 16u);
+      const int b = 31 - __builtin_clz(s);
+      const bool packed = std::max(h_plen[i], h_tlen[i]) <= tsu::kPackedMaxLen;
+      return (packed ? kKeys : 0) + kKeys - 1 - (b * 16 + (int)((s >> (b - 4)) & 15));
+    };
+    int32_t start[2 * kKeys + 1] = {};
+    for (int32_t i : *list) ++start[key(i) + 1];
+    for (int k = 0; k < 2 * kKeys; ++k) start[k + 1] += start[k];
+    std::vector<int32_t> sorted(list->size());
+    for (int32_t i : *list) sorted[(size_t)start[key(i)]++] = i;
+    list->swap(sorted);
     for (int32_t i : *list) {
       if (std::max(h_plen[i], h_tlen[i]) > tsu::kPackedMaxLen)
         ++p->n_wide;
@@ -1331,7 +1339,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   if (can_bound) {
     tsu::BoundLimits limits = tsu::bound_limits(ctx->rp, ctx->smem_optin);
     if (low_mem) limits.side = std::min(limits.side, tsu::kBoundLowMemLen);
-    if (bi.max_side >= limits.side || bi.max_sum >= limits.sum)
+    if (bi.max_side >= limits.side)
       for (int64_t i = 0; i < n; ++i)
         if (limits.wants(h_plen[i], h_tlen[i]) && !ctx->band_set[tsu::length_band(std::max(h_plen[i], h_tlen[i]))])
           probed.push_back((int32_t)i);
@@ -1533,6 +1541,18 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     // classes of the shared ring, of the wide kernel (16- and 32-bit rows), bands
     constexpr int kWide = tsu::kBoundClasses, kBand0 = kWide + 2, kAll = kBand0 + tsu::kBands;
     std::vector<Class> cls((size_t)kAll);
+    // class of the shared ring by bytes / 16 (bounded_bytes); -1: not yet known,
+    // kAll: they do not fit a block
+    std::vector<int8_t> ring_class((size_t)ctx->smem_optin / 16 + 1, -1);
+    auto class_of = [&](int bytes) -> int {
+      if (bytes > ctx->smem_optin) return kAll;
+      int8_t& c = ring_class[(size_t)bytes / 16];
+      if (c < 0) {
+        int per_sm = 0;
+        c = (int8_t)(tsu::bounded_warps(bytes, INT32_MAX, ctx->sms, ctx->smem_optin, &per_sm) ? tsu::bound_class(per_sm) : kAll);
+      }
+      return c;
+    };
     for (int32_t i : list) {
       const int32_t m = h_plen[i], t = h_tlen[i], u = ub[i];
       size_t c = (size_t)(kBand0 + tsu::length_band(std::max(m, t)));
@@ -1541,10 +1561,10 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       if (u != tsu::kNoBound) {
         need = tsu::bound_need(ctx->rp, m, t, u);
         bytes = tsu::bounded_bytes(ctx->rp, need.width, need.words, 16);
-        int per_sm = 0;
-        if (std::max(m, t) <= tsu::kPackedMaxLen && tsu::packed_width(need.width) <= tsu::kPackedMaxW &&
-            tsu::bounded_warps(bytes, INT32_MAX, ctx->sms, ctx->smem_optin, &per_sm))
-          c = (size_t)tsu::bound_class(per_sm);
+        const bool ring = std::max(m, t) <= tsu::kPackedMaxLen && tsu::packed_width(need.width) <= tsu::kPackedMaxW;
+        const int rc3 = ring ? class_of(bytes) : kAll;
+        if (rc3 != kAll)
+          c = (size_t)rc3;
         else if (need.hist <= tsu::kWideMaxHist)
           c = (size_t)(t <= tsu::kWide16MaxLen ? kWide : kWide + 1);
       }

@@ -275,22 +275,27 @@ inline int64_t arena_runs(const Pen& pen, int64_t n, int32_t max_m, int32_t max_
 
 // ---- passes of pairs whose score bound is known ----------------------------
 
-// Whether a pair of a large batch is worth a bound probe: its full wavefronts
-// are expected to reach 420 diagonals at 4 % edits (gap-affine 4/6/2: from
-// 1.3 kbp), or one warp's unbounded ring takes over 14 KB (two gap pieces,
-// deep penalties), so that an SM holds few of them.  Below that a pair fits
-// one warp's ring without a bound and the probe, two words per lane and score,
-// costs about what it saves.
-constexpr int kBoundMinWidth = 420;
-constexpr int kBoundMinRing = 14 << 10;
-// (In terms of the longer side and of both: pairs from the limits up, found
-// once per call.)
+// Whether a pair of a large batch is worth a bound probe, by the width its full
+// wavefronts are expected to reach at 4 % edits: 420 diagonals and 1,024 bases
+// (gap-affine 4/6/2: from 1.2 kbp; edit distance: 4.9 kbp), 224 where the ring
+// of one warp (kSharedW1 diagonals) takes over 14 KB, so that an SM holds few of
+// them (two gap pieces 4/6/2/24/1: from 300 bp).  A probe computes 128
+// diagonals and the bookkeeping of every score once more, so it saves nothing
+// where the wavefronts are about that wide, and costs accurate pairs most.
+// Probed / not, ms a scored call on one B200 at 0.5, 2, 5 and 15 %: two pieces
+// 20,000 x 100 bp 0.93 / 0.43, 0.95 / 0.51, 1.41 / 1.05, 2.15 / 2.73; x 200 bp
+// 0.96 / 0.45, 1.33 / 0.96, 1.87 / 2.23, -; x 300 bp 0.98 / 0.56, 1.63 / 1.61,
+// 2.42 / 3.22; x 500 bp 1.24 / 0.92, 2.01 / 2.52, 3.34 /
+// 5.16; gap-affine 3/5/1 6,000 x 1 kbp 0.54 / 0.21, 0.83 / 0.38, 1.50 / 2.13; 4/6/2
+// 2,000 x 1.5 kbp 0.31 / 0.17, 0.47 / 0.26, 0.68 / 0.53, 600 of them at 15 % 1.48 /
+// 1.94, 6,000 x 2.5 kbp 0.68 / 0.54, 1.20 / 1.17, x 5 kbp 0.97 / 1.20, 2.28 / 3.24.
+// Pairs below the line that outgrow their ring get a bound then.
+constexpr int kBoundMinWidth = 420, kBoundMinWidthDeep = 224;
+constexpr int kBoundMinRing = 14 << 10, kBoundMinLen = 1024;
 struct BoundLimits {
-  int32_t side = INT32_MAX, sum = INT32_MAX;
+  int32_t side = INT32_MAX;      // the longer side from which a pair of a large batch is probed
   int32_t few_side = INT32_MAX;  // the longer side from which few pairs get a bound (below)
-  bool wants(int32_t m, int32_t n) const {
-    return std::min(m, n) > 0 && (std::max(m, n) >= side || m + n >= sum);
-  }
+  bool wants(int32_t m, int32_t n) const { return std::min(m, n) > 0 && std::max(m, n) >= side; }
 };
 // With no more such pairs than SMs each has an SM to itself, and a probe (0.35
 // us per score on one warp) costs more than the narrower search saves until a
@@ -314,9 +319,8 @@ inline BoundLimits bound_limits(const Pen& pen, int smem_optin) {
     }
     return lo;
   };
-  b.side = from(kBoundMinWidth, 0.04);
-  const int64_t d = kBoundMinRing / (2 * ((int64_t)pen.slots() + 1)) + 1;  // diagonals that take more than kBoundMinRing
-  if (d <= kSharedW1) b.sum = (int32_t)std::max<int64_t>(d - 3, 1);
+  const bool deep = 2 * ((int64_t)pen.slots() + 1) * kSharedW1 > kBoundMinRing;
+  b.side = deep ? from(kBoundMinWidthDeep, 0.04) : std::max(from(kBoundMinWidth, 0.04), kBoundMinLen);
   b.few_side = from(std::max(shared_ring_width(pen, 16, kSharedSeqWordsN, smem_optin, true), 64), 0.163);
   return b;
 }
