@@ -1443,7 +1443,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       r.few = r.n <= ctx->sms && std::max(r.bi.max_m, r.bi.max_n) >= few_side;
       const bool as_set = ctx->band_set[r.band];
       if (r.few && !as_set) r.pc = tsu::few_start(r.pc, ctx->rp, std::max(r.bi.max_m, r.bi.max_n));
-      if (!ctx->one_warp && !as_set) r.pc = tsu::fill_warps(r.pc, ctx->rp, r.n, std::max(r.bi.max_m, r.bi.max_n), ctx->sms);
+      if (!ctx->one_warp && !as_set && !(want_cigar && ctx->low_mem)) r.pc = tsu::fill_warps(r.pc, ctx->rp, r.n, std::max(r.bi.max_m, r.bi.max_n), ctx->sms);
       if ((rc = plan_pass_within(ctx, r.bi, r.n, r.pc, r.hint, want_cigar, avail, &r.ps))) return rc;
       need = std::max(need, scratch_bytes(r.ps, want_cigar));
     }
@@ -1876,7 +1876,8 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       hint = tsu::next_hint(hint, last_mode == tsu::kModeGlobal);
       pc = ctx->one_warp             ? tsu::PassChoice{tsu::kModeGlobal, 1}
            : first && r.all_bytes    ? tsu::PassChoice{tsu::kModeGlobal, 16}
-                                     : tsu::next_pass(pc, ctx->rp, pbi.max_m, pbi.max_n, ctx->smem_optin);
+                                     : tsu::next_pass(pc, ctx->rp, pbi.max_m, pbi.max_n, ctx->smem_optin, 16,
+                                                      want_cigar && ctx->low_mem);
       if (want_cigar) {
         unsigned long long* h_used = reinterpret_cast<unsigned long long*>(h_cnt + 16);
         CU(cudaMemcpyAsync(h_used, d_cursor, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));

@@ -184,16 +184,19 @@ inline PassGeom plan_geometry(const Pen& pen, int32_t max_m, int32_t max_n, int 
 // global_gw (16) warps per pair (the pairs that reach it are the longest and
 // most divergent ones; their count in flight is bounded by memory, not by
 // warps).
+// lowmem: low-memory passes, whose shared ring takes all sides up to
+// kSharedMaxLen itself.
 inline PassChoice next_pass(PassChoice prev, const Pen& pen, int32_t max_m, int32_t max_n, int smem_optin,
-                            int global_gw = 16) {
+                            int global_gw = 16, bool lowmem = false) {
   const int64_t need_w = (int64_t)max_m + max_n + 3;
   const int64_t maxlen = std::max(max_m, max_n);
   if (prev.mode == kModeShared && maxlen <= kSharedMaxLen) {
     // sides past the packed kernel's offsets, handed back by it: the kernel of
     // one diagonal per thread, from the same warps on
-    const bool single = prev.single || maxlen > kPackedPlainLen;
-    const int least = maxlen > kPackedPlainLen && !prev.single && !shared_single(pen, maxlen, prev.gw) ? prev.gw : prev.gw + 1;
-    const bool packed = !single && packed_fits(pen);
+    const bool single = !lowmem && (prev.single || maxlen > kPackedPlainLen);
+    const bool again = single && !prev.single && !shared_single(pen, maxlen, prev.gw);
+    const int least = again ? prev.gw : prev.gw + 1;
+    const bool packed = !lowmem && !single && packed_fits(pen);
     const int64_t seqw =
         std::min<int64_t>(2 * packed_words(max_m) + 2 * packed_words(max_n), kSharedSeqWordsN);
     static const int kGW[] = {2, 4, 8, 16};
@@ -454,7 +457,7 @@ inline PassChoice few_start(PassChoice pc, const Pen& pen, int32_t maxlen) {
 // fewer than 8 warps (600 pairs of 1 kbp: 0.22 ms on 1, 0.19 on 2, 0.26 on 4);
 // at most one warp per 64 bases beyond the rung (20 pairs of 115 bp: 162 us a
 // call on 1 warp, 168 on 16).  The kernel of one diagonal per thread keeps its
-// rung.
+// rung, and so do low-memory passes, whose checkpoints are as wide as the ring.
 inline PassChoice fill_warps(PassChoice pc, const Pen& pen, int64_t n, int32_t maxlen, int sms) {
   if (pc.mode != kModeShared || pc.single || shared_single(pen, maxlen, pc.gw)) return pc;
   while (pc.gw < 16 && (n <= sms || n * pc.gw * 2 <= (int64_t)sms * 8) && pc.gw * 128 <= maxlen) pc.gw *= 2;
