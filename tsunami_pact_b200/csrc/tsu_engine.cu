@@ -913,11 +913,14 @@ int run_bidir_cigar(tsu_ctx* ctx, const tsu::SeqView& sv, int32_t* d_score, int3
     const size_t fixed = ctx->held() - ctx->b_scratch.cap;
     const size_t avail = ctx->budget > fixed ? ctx->budget - fixed : 0;
     warps = std::min<int64_t>(warps, (int64_t)(avail / per_warp));
-    // The leaves of a few pairs (no more than SMs) run in the scratch that the
-    // breakpoint rings already hold, or on 32 warps: one 50 kbp pair's 130
-    // leaves would take 56 MB of history at once, three times its rings.
+    // No more leaves than SMs (of a few pairs) run in the scratch that the
+    // breakpoint rings already hold, or in 32 MB, or on 32 warps: one 50 kbp
+    // pair's 130 leaves would take 56 MB of history at once, three times its
+    // rings.  (On 32 warps 30 pairs of 3 kbp at 15 %, edit distance, took 14.7
+    // ms, all 60 leaves at once 12.4.)
+    constexpr size_t kLeafBytes = 32 << 20;
     if (c <= ctx->sms)
-      warps = std::min<int64_t>(warps, std::max<int64_t>(32, (int64_t)(ctx->b_scratch.cap / per_warp)));
+      warps = std::min<int64_t>(warps, std::max<int64_t>(32, (int64_t)(std::max(ctx->b_scratch.cap, kLeafBytes) / per_warp)));
     if (warps < 1) {
       ctx->need_bytes = fixed + per_warp;
       return set_err(ctx, TSU_ENOMEM, "bidirectional mode: base-case history of one segment exceeds the budget");
