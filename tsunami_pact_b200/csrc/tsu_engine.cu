@@ -89,6 +89,7 @@ struct tsu_ctx {
   DevBuf b_bsegs, b_boff, b_blen, b_bruns, b_bfirst;      // bidirectional CIGARs: base cases, their runs
   DevBuf b_pre;                                           // bidirectional CIGARs: the whole-pair launch's results
   DevBuf b_bound;                                         // score bounds of the pairs (bound probe)
+  DevBuf b_again;                                         // pass order, then retry list, of pairs started again with bounds
   bool one_warp = false;  // TSU_ONE_WARP of the current call
   bool bidir = false;     // TSU_BIDIRECTIONAL of the current call
   cudaEvent_t pev[2] = {};  // per-pass timing
@@ -142,7 +143,7 @@ struct tsu_ctx {
     return {&b_pat,  &b_txt,    &b_poff,     &b_toff,  &b_plen,  &b_tlen,   &b_words_cnt, &b_woff, &b_words,
             &b_nonacgt, &b_score, &b_status, &b_cpos, &b_clen, &b_clen64, &b_coff,      &b_out,  &b_order,
             &b_retry, &b_counters, &b_scratch, &b_arena, &b_scan_tmp, &b_out2, &b_rwords, &b_rnonacgt,
-            &b_segs,  &b_bout, &b_bsegs, &b_boff, &b_blen, &b_bruns, &b_bfirst, &b_pre, &b_bound};
+            &b_segs,  &b_bout, &b_bsegs, &b_boff, &b_blen, &b_bruns, &b_bfirst, &b_pre, &b_bound, &b_again};
   }
   size_t held() const {
     size_t s = 0;
@@ -1282,10 +1283,18 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   const tsu::PackView pk{P<uint64_t>(ctx->b_words), P<int64_t>(ctx->b_woff), P<uint8_t>(ctx->b_nonacgt)};
   if ((rc = grow(ctx, ctx->b_cpos, sizeof(int64_t) * n))) return rc;
   if ((rc = grow(ctx, ctx->b_clen, sizeof(int32_t) * n))) return rc;
-  // pass orders and retry lists: the first passes', then those of pairs that
-  // got a bound after outgrowing theirs
-  if ((rc = grow(ctx, ctx->b_retry, sizeof(int32_t) * 2 * n))) return rc;
-  if ((rc = grow(ctx, ctx->b_order, sizeof(int32_t) * 2 * n))) return rc;
+  if ((rc = grow(ctx, ctx->b_retry, sizeof(int32_t) * n))) return rc;
+  if ((rc = grow(ctx, ctx->b_order, sizeof(int32_t) * n))) return rc;
+  // Pass orders and retry lists: of the first passes, and (again) of pairs that
+  // got a bound after outgrowing theirs.
+  auto order_of = [&](bool again) -> int32_t* { return P<int32_t>(again ? ctx->b_again : ctx->b_order); };
+  auto retry_of = [&](bool again) -> int32_t* { return again ? P<int32_t>(ctx->b_again) + n : P<int32_t>(ctx->b_retry); };
+  // Buffers that only bounds need: without them the call does without bounds.
+  auto spare = [&](DevBuf& b, size_t bytes) -> bool {
+    if (grow(ctx, b, bytes) == TSU_OK) return true;
+    ctx->err.clear();
+    return false;
+  };
   // counters: +8 the bound probe's queue head, +16 arena cursor, +24 work (cells, steps, extension bases), +64 + 8b queue head
   // and retry count of band slot b
   constexpr size_t kProbeQueue = 8;  // the bound probes' queue heads (wide, packed)
@@ -1353,7 +1362,10 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
                    probed.end());
     }
     if ((rc = plan_probes(&probed, &probe))) return rc;
-    if (!probed.empty() && (rc = grow(ctx, ctx->b_bound, sizeof(int32_t) * n))) return rc;
+    if (!probed.empty() && !spare(ctx->b_bound, sizeof(int32_t) * n)) {
+      probed.clear();
+      probe = ProbePlan{};
+    }
   }
   const int64_t n_probed = (int64_t)probed.size();
   const int min_pen = ctx->rp.min_pen();
@@ -1388,6 +1400,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   struct BandRun {
     int band = 0, slot = 0;
     int64_t off = 0, n = 0;  // slice of the pass order / retry list
+    bool again = false;      // of b_again
     BatchInfo bi;
     tsu::PassChoice pc;
     double hint = 0;
@@ -1495,9 +1508,9 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     a.wide_cell = ps.g.wide_cell;
     return a;
   };
-  // The bound probe over `count` pairs of the order from `off` on;
+  // The bound probe over the `count` pairs at `order`;
   // fetch_bounds: their bounds to ctx->h_bound.
-  auto queue_probe = [&](const ProbePlan& p, int64_t off, int64_t count) -> int {
+  auto queue_probe = [&](const ProbePlan& p, const int32_t* order, int64_t count) -> int {
     CU(cudaMemsetAsync(ctx->b_bound.p, 0x7f, sizeof(int32_t) * n, st));  // kNoBound
     tsu::ProbeArgs b{};
     b.seq = sv;
@@ -1506,14 +1519,14 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     b.seq_cap = p.seq;
     b.bound = P<int32_t>(ctx->b_bound);
     if (p.n_wide) {
-      b.order = P<int32_t>(ctx->b_order) + off;
+      b.order = order;
       b.n_order = p.n_wide;
       b.queue = reinterpret_cast<unsigned int*>(d_cnt + kProbeQueue);
       launch_probe(ctx, true, p.wide_blocks, p.wide_smem, st, b);
       CU(cudaGetLastError());
     }
     if (count > p.n_wide) {
-      b.order = P<int32_t>(ctx->b_order) + off + p.n_wide;
+      b.order = order + p.n_wide;
       b.n_order = count - p.n_wide;
       b.queue = reinterpret_cast<unsigned int*>(d_cnt + kProbeQueue) + 1;
       launch_probe(ctx, false, p.blocks, p.smem, st, b);
@@ -1531,7 +1544,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   // bounds need, each one launch on the shared ring planned from the bounds;
   // pairs without a bound, or too wide for a block's ring, by length band as
   // the others.  Appends to runs and reads the counters back.
-  auto bounded_runs = [&](const std::vector<int32_t>& list, int64_t off) -> int {
+  auto bounded_runs = [&](const std::vector<int32_t>& list, int64_t off, bool again) -> int {
     const int32_t* ub = ctx->h_bound.data();
     struct Class {
       std::vector<int32_t> pairs;
@@ -1594,6 +1607,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
       BandRun r;
       r.slot = (int)runs.size();
       r.off = off + (int64_t)order.size();
+      r.again = again;
       r.n = (int64_t)k.pairs.size();
       r.bi = k.bi;
       r.bi.n = r.n;
@@ -1652,8 +1666,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     }
     if ((rc2 = host_grow(ctx, ctx->h_list, sizeof(int32_t) * order.size()))) return rc2;
     memcpy(ctx->h_list.p, order.data(), sizeof(int32_t) * order.size());
-    CU(cudaMemcpyAsync(P<int32_t>(ctx->b_order) + off, ctx->h_list.p, sizeof(int32_t) * order.size(),
-                       cudaMemcpyHostToDevice, st));
+    CU(cudaMemcpyAsync(order_of(again) + off, ctx->h_list.p, sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice, st));
     for (size_t j = first; j < runs.size(); ++j)
       for (int e = 0; e < 2; ++e)
         if (!ctx->bev[2 * runs[j].slot + e]) CU(cudaEventCreate(&ctx->bev[2 * runs[j].slot + e]));
@@ -1665,7 +1678,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     size_t at = 0;
     for (size_t j = first; j < runs.size(); ++j) {
       const BandRun& r = runs[j];
-      tsu::AlignArgs a = align_args(r.ps, P<int32_t>(ctx->b_order) + r.off, r.n, r.slot, P<int32_t>(ctx->b_retry) + r.off);
+      tsu::AlignArgs a = align_args(r.ps, order_of(again) + r.off, r.n, r.slot, retry_of(again) + r.off);
       const size_t lane = (j - first) % (kSideStreams + 1);
       cudaStream_t cs = side && lane ? ctx->side[lane - 1] : st;
       if (side) {
@@ -1734,7 +1747,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     CU(cudaMemsetAsync(d_cnt, 0, kCounterBytes, st));
     CU(record(ctx, ctx->ev[4], st));
     if (n_probed) {
-      if (const int prc = queue_probe(probe, probe_off, n_probed)) return prc;
+      if (const int prc = queue_probe(probe, order_of(false) + probe_off, n_probed)) return prc;
     }
     for (const BandRun& r : runs) {
       const tsu::AlignArgs a = align_args(r.ps, all_pairs ? nullptr : P<int32_t>(ctx->b_order) + r.off, r.n, r.slot,
@@ -1763,7 +1776,7 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
   CU(early_ev ? cudaEventSynchronize(early_ev) : wait_stream(ctx, st));
   const size_t first_runs = runs.size();  // the ones of pairs that were not probed
   if (n_probed) {
-    if ((rc = fetch_bounds()) || (rc = bounded_runs(probed, probe_off))) return rc;
+    if ((rc = fetch_bounds()) || (rc = bounded_runs(probed, probe_off, false))) return rc;
   }
   // Pairs that outgrew an unbounded shared ring get a bound, and a second
   // start with it: 20,000 pairs of 800 - 1,000 bp at 10 % took 13.2 ms through
@@ -1802,18 +1815,17 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     ProbePlan p;
     const size_t asked = again.size();
     if ((rc = plan_probes(&again, &p))) return rc;
-    if (asked && again.size() == asked) {
+    if (asked && again.size() == asked && spare(ctx->b_again, sizeof(int32_t) * 2 * n) &&
+        spare(ctx->b_bound, sizeof(int32_t) * n)) {
       if ((rc = host_grow(ctx, ctx->h_list, sizeof(int32_t) * again.size()))) return rc;
       memcpy(ctx->h_list.p, again.data(), sizeof(int32_t) * again.size());
-      CU(cudaMemcpyAsync(P<int32_t>(ctx->b_order) + n, ctx->h_list.p, sizeof(int32_t) * again.size(),
-                         cudaMemcpyHostToDevice, st));
-      if ((rc = grow(ctx, ctx->b_bound, sizeof(int32_t) * n))) return rc;
+      CU(cudaMemcpyAsync(order_of(true), ctx->h_list.p, sizeof(int32_t) * again.size(), cudaMemcpyHostToDevice, st));
       CU(cudaMemsetAsync(d_cnt + kProbeQueue, 0, 8, st));
-      if ((rc = queue_probe(p, n, (int64_t)again.size()))) return rc;
+      if ((rc = queue_probe(p, order_of(true), (int64_t)again.size()))) return rc;
       ctx->timing.kernel_launches += (p.n_wide ? 1 : 0) + ((int64_t)again.size() > p.n_wide ? 1 : 0);
       ctx->timing.retried_pairs += (int64_t)again.size();
       rebound_any = true;
-      if ((rc = fetch_bounds()) || (rc = bounded_runs(again, n))) return rc;
+      if ((rc = fetch_bounds()) || (rc = bounded_runs(again, 0, true))) return rc;
     } else {
       for (BandRun& r : runs) {
         r.all_bytes = r.all_bytes && !r.rebound;
@@ -1843,8 +1855,8 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     tsu::PassChoice pc = r.pc;
     double hint = r.hint;
     int last_mode = r.ps.g.mode;
-    int32_t* const d_order = P<int32_t>(ctx->b_order) + r.off;  // this band's slices
-    int32_t* const d_retry = P<int32_t>(ctx->b_retry) + r.off;
+    int32_t* const d_order = order_of(r.again) + r.off;  // this band's slices
+    int32_t* const d_retry = retry_of(r.again) + r.off;
     unsigned int* const d_slot = reinterpret_cast<unsigned int*>(d_cnt + 64 + 8 * r.slot);
     const int band_first_pass = passes - 1;
     for (;;) {
