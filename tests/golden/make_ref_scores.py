@@ -7,7 +7,7 @@ every set with the CPU model of the kernel (oracle/ref_kernel_model.c) before
 it launches anything, and records whether the GPU scores equal the model's.
 
     python tests/golden/make_ref_scores.py --out tests/golden/ref_scores.json
-    python tests/golden/make_ref_scores.py --from-dir gpurun_out --out ...  # assemble earlier harness runs
+    python tests/golden/make_ref_scores.py --from-dir DIR --out ...  # assemble earlier harness runs
 
 Sets (penalties 4/6/2, text = pattern with round(L * rate) edits, equal
 insertion and deletion counts, so every pair is L x L as the kernel needs):
@@ -52,7 +52,7 @@ def main():
     ap.add_argument("--out", default=os.path.join(ROOT, "tests", "golden", "ref_scores.json"))
     ap.add_argument("--harness", default=os.path.join(ROOT, "oracle", "_ref", "ref_harness"))
     ap.add_argument("--from-dir", default=None, help="use ref_<set>.txt / ref_<set>.json written by earlier runs")
-    ap.add_argument("--work", default=os.path.join(ROOT, "gpurun_out"))
+    ap.add_argument("--work", default=os.path.join(ROOT, "oracle", "_ref"))
     args = ap.parse_args()
     os.makedirs(args.work, exist_ok=True)
     out = {"what": "scores of the reference's own GPU kernel (wfa_dispatcher, wfa_gpu.cu:191-752), built unchanged "

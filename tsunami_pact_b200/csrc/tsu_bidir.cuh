@@ -34,10 +34,11 @@
 // up to less is not scanned: before the two passes meet, no check reads a
 // cell.
 //
-// Measured on one B200, 500 pairs of 10 kbp at 15 % with CIGARs: 142 ms a cell 121 ms with two (compute() below); 109 ms with the crossing tests
-// of a turn on the lanes of a warp and turns without a scan ended without
-// barriers.  The first level takes 45 of them at 13 warps per SM, issue slots
-// 45 % busy: latency of the ring's loads (they hit L1 to 70 %).
+// Measured on one B200, 500 pairs of 10 kbp at 15 % with CIGARs: 142 ms with one
+// cell per lane, 121 with two (compute() below), 109 with the crossing tests of a
+// turn on the lanes of a warp and turns without a scan ended without barriers.
+// The first level takes 45 of them at 13 warps per SM, issue slots 44 % busy:
+// latency of the ring's loads (they hit L1 to 70 %, 2.5 stalled warps per issue).
 //
 // One group of GW warps per segment, persistent over a work queue.  The
 // rings of both directions live in global memory (indexed by diagonal:

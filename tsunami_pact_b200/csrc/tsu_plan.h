@@ -285,13 +285,16 @@ inline int64_t arena_runs(const Pen& pen, int64_t n, int32_t max_m, int32_t max_
 // them (two gap pieces 4/6/2/24/1: from 300 bp).  A probe computes 128
 // diagonals and the bookkeeping of every score once more, so it saves nothing
 // where the wavefronts are about that wide, and costs accurate pairs most.
-// Probed / not, ms a scored call on one B200 at 0.5, 2, 5 and 15 %: two pieces
-// 20,000 x 100 bp 0.93 / 0.43, 0.95 / 0.51, 1.41 / 1.05, 2.15 / 2.73; x 200 bp
-// 0.96 / 0.45, 1.33 / 0.96, 1.87 / 2.23, -; x 300 bp 0.98 / 0.56, 1.63 / 1.61,
-// 2.42 / 3.22; x 500 bp 1.24 / 0.92, 2.01 / 2.52, 3.34 /
-// 5.16; gap-affine 3/5/1 6,000 x 1 kbp 0.54 / 0.21, 0.83 / 0.38, 1.50 / 2.13; 4/6/2
-// 2,000 x 1.5 kbp 0.31 / 0.17, 0.47 / 0.26, 0.68 / 0.53, 600 of them at 15 % 1.48 /
-// 1.94, 6,000 x 2.5 kbp 0.68 / 0.54, 1.20 / 1.17, x 5 kbp 0.97 / 1.20, 2.28 / 3.24.
+// Probed / not, ms a scored call on one B200 at 0.5, 2, 5 and 15 %:
+//   two pieces   20,000 x 100 bp  0.93 / 0.43  0.95 / 0.51  1.41 / 1.05  2.15 / 2.73
+//                20,000 x 200 bp  0.96 / 0.45  1.33 / 0.96  1.87 / 2.23
+//                20,000 x 300 bp  0.98 / 0.56  1.63 / 1.61  2.42 / 3.22
+//                20,000 x 500 bp  1.24 / 0.92  2.01 / 2.52  3.34 / 5.16
+//   affine 3/5/1  6,000 x 1 kbp   0.54 / 0.21  0.83 / 0.38  1.50 / 2.13
+//   affine 4/6/2  2,000 x 1.5 kbp 0.31 / 0.17  0.47 / 0.26  0.68 / 0.53
+//                   600 x 1.5 kbp 0.23 / 0.14  0.32 / 0.18  0.48 / 0.30  1.48 / 1.94
+//                 6,000 x 2.5 kbp 0.68 / 0.54  1.20 / 1.17
+//                 6,000 x 5 kbp   0.97 / 1.20  2.28 / 3.24
 // Pairs below the line that outgrow their ring get a bound then.
 constexpr int kBoundMinWidth = 420, kBoundMinWidthDeep = 224;
 constexpr int kBoundMinRing = 14 << 10, kBoundMinLen = 1024;
@@ -425,7 +428,8 @@ inline int wide_cluster(int64_t n, int sms) {
   while (c < 8 && n * c * 2 <= (int64_t)sms * 7 / 8) c *= 2;
   return c;
 }
-// Cells of history a wide launch may keep (32-bit words below 2^31).
+// History a wide launch may keep (32-bit words below 2^31).  Scores alone are held
+// to it too: it keeps the rows' byte offsets in the ring below 2^31.
 constexpr int64_t kWideMaxHist = INT32_MAX - 65536;
 
 // In low-memory mode (interval chosen here) every pair from this length on is

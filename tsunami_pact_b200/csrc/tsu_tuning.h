@@ -1,5 +1,6 @@
 // tsu_tuning.h -- starting rung of the pass ladder per length band.
-// Written by tsunami_pact_b200/tune.py (the autotuner); rebuild the library after changing it.
+// Written by tsunami_pact_b200/tune.py (the autotuner), bands 1 and 2 then set by hand (below); rebuild the library
+// after changing it.
 // band: max(m, n) < 1024, < 2048, < 4096, < 8192, < 16384, >= 16384
 // rung: {ring mode (0 shared, 1 global), warps per pair}
 // align time in ms per starting rung (s1 s2 s4 s8 s16 g8 g16 g32):
@@ -15,5 +16,5 @@
 //   20,000 x 1 kbp at 5 %, 100 free bases per end (band 1): 11.3r 6.2 7.9 9.1
 //   10,000 x 2 kbp at 5 %, 100 free bases per end (band 2): 21.0r 16.4r 9.3 10.1
 #pragma once
-#define TSU_TUNING_SOURCE "tune.py on NVIDIA B200, 2026-12-03, workloads c2:200000,c4:100000,c3:5000"
+#define TSU_TUNING_SOURCE "tune.py on NVIDIA B200, 2026-12-03, workloads c2:200000,c4:100000,c3:5000; bands 1 and 2 by hand, 2026-12-05"
 #define TSU_BAND_START {{0, 1}, {0, 2}, {0, 4}, {0, 8}, {0, 16}, {1, 32}}

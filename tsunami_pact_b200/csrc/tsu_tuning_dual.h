@@ -2,6 +2,8 @@
 // Written by tsunami_pact_b200/tune.py (the autotuner); rebuild the library after changing it.
 // band: max(m, n) < 1024, < 2048, < 4096, < 8192, < 16384, >= 16384
 // rung: {ring mode (0 shared, 1 global), warps per pair}
+// measured on the kernels of one diagonal per thread; pairs from 300 bp on start with a score bound instead, unless
+// ends are free or bytes outside ACGT keep them from one (on the global ring, bands 1 to 5 then start there).
 // align time in ms per starting rung (s1 s2 s4 s8 s16 s32 g8 g16 g32):
 //   band 0 (< 1024): 615.6 585.2 649.4 255.0 559.7 1404.8 293.8 609.3 1353.4
 //   band 1 (< 2048): 109.5 105.1 107.6 116.5 105.7 240.1 76.3 115.7 210.0

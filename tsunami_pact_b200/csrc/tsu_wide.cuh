@@ -5,10 +5,11 @@
 // the bound, source bits as history, one end test per score), one diagonal per
 // lane in 32-bit registers, the ring in device memory: one pair per block of
 // 16 warps, rows of h + 1 (0: absent) in 16 bits for texts of up to 65,532
-// bases and 32 bits for longer ones.  What bounds it is the ring's L2 traffic
-// (five loads and three stores per cell), so 16-bit rows halve the time of the
-// widest scores, and U = 4 cells per lane are in flight to cover its latency; few pairs are
-// spread over clusters of up to 8 blocks.
+// bases and 32 bits for longer ones.  A block's scores are bound by issue and the
+// ring's L2 traffic (five loads and three stores per cell), so 16-bit rows halve
+// the time of the widest, and U = 4 cells per lane are in flight to cover its
+// latency; few pairs are spread over clusters of up to 8 blocks, whose barrier
+// between scores is then half of what a warp waits for (issue 35 %).
 // The sequences are read through L1 (a few neighbouring words per warp).
 #pragma once
 
