@@ -1313,20 +1313,26 @@ int run_device(tsu_ctx* ctx, const tsu::SeqView& sv, bool want_cigar, int32_t* d
     size_t smem = 0, wide_smem = 0;
   };
   auto plan_probes = [&](std::vector<int32_t>* list, ProbePlan* p) -> int {
-    // (a counting sort by the leading five bits of both lengths' sum)
-    constexpr int kKeys = 32 * 16;
-    auto key = [&](int32_t i) -> int {
-      const uint32_t s = std::max((uint32_t)h_plen[i] + (uint32_t)h_tlen[i], 16u);
-      const int b = 31 - __builtin_clz(s);
-      const bool packed = std::max(h_plen[i], h_tlen[i]) <= tsu::kPackedMaxLen;
-      return (packed ? kKeys : 0) + kKeys - 1 - (b * 16 + (int)((s >> (b - 4)) & 15));
-    };
-    int32_t start[2 * kKeys + 1] = {};
-    for (int32_t i : *list) ++start[key(i) + 1];
-    for (int k = 0; k < 2 * kKeys; ++k) start[k + 1] += start[k];
-    std::vector<int32_t> sorted(list->size());
-    for (int32_t i : *list) sorted[(size_t)start[key(i)]++] = i;
-    list->swap(sorted);
+    // (many pairs: a counting sort by the leading seven bits of both lengths'
+    // sum; few, whose longest ones may be a launch's last: exactly)
+    constexpr int kSub = 64, kKeys = 32 * kSub;
+    auto sum = [&](int32_t i) -> uint32_t { return (uint32_t)h_plen[i] + (uint32_t)h_tlen[i]; };
+    auto wide = [&](int32_t i) -> bool { return std::max(h_plen[i], h_tlen[i]) > tsu::kPackedMaxLen; };
+    if (list->size() <= 1024) {
+      std::stable_sort(list->begin(), list->end(),
+                       [&](int32_t u, int32_t v) { return wide(u) != wide(v) ? wide(u) : sum(u) > sum(v); });
+    } else {
+      auto key = [&](int32_t i) -> int {
+        const uint32_t s = std::max(sum(i), (uint32_t)kSub);
+        const int b = 31 - __builtin_clz(s);
+        return (wide(i) ? 0 : kKeys) + kKeys - 1 - (b * kSub + (int)((s >> (b - 6)) & (kSub - 1)));
+      };
+      std::vector<int32_t> start(2 * kKeys + 1, 0), sorted(list->size());
+      for (int32_t i : *list) ++start[(size_t)key(i) + 1];
+      for (int k = 0; k < 2 * kKeys; ++k) start[(size_t)k + 1] += start[(size_t)k];
+      for (int32_t i : *list) sorted[(size_t)start[(size_t)key(i)]++] = i;
+      list->swap(sorted);
+    }
     for (int32_t i : *list) {
       if (std::max(h_plen[i], h_tlen[i]) > tsu::kPackedMaxLen)
         ++p->n_wide;
